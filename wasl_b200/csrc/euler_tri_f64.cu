@@ -34,159 +34,371 @@ template <> __device__ __forceinline__ const VolumeTable<1, double> &volume_tabl
 template <> __device__ __forceinline__ const VolumeTable<2, double> &volume_table<2>() { return c_vol2; }
 template <> __device__ __forceinline__ const VolumeTable<3, double> &volume_table<3>() { return c_vol3; }
 
-// Euler state of element `e` of a global SoA array at a point with basis `b`.
-template <int M>
-__device__ __forceinline__ void eval_global(const double *__restrict__ u, std::int64_t ne,
-                                            std::int64_t e, const double *b, double *s) {
+// The HLLC flux of hllc() (euler_device.cuh; cpp/include/wasl/flux/hllc.hpp:40-74)
+// with the side whose state the flux is built on chosen before its physical
+// flux and star state are evaluated, not after both sides' are: the same
+// expressions on the chosen side, so the same doubles, one evaluation of each
+// for every branch, and no divergence between the branches of a warp.
+__device__ __forceinline__ void hllc_selected(double gamma, const double (&l)[4],
+                                              const double (&r)[4], double nx, double ny,
+                                              double (&f)[4]) {
+  const Prim<double> lv = primitive(gamma, l);
+  const Prim<double> rv = primitive(gamma, r);
+  const double lu = lv.vx * nx + lv.vy * ny;
+  const double ru = rv.vx * nx + rv.vy * ny;
+  const double lc = sound_speed(gamma, lv);
+  const double rc = sound_speed(gamma, rv);
+  const double sl = smin(lu - lc, ru - rc);
+  const double sr = smax(lu + lc, ru + rc);
+  const double contact = (rv.p - lv.p + l[0] * lu * (sl - lu) - r[0] * ru * (sr - ru)) /
+                         (l[0] * (sl - lu) - r[0] * (sr - ru));
+  // The reference's tests in its order (NaN speeds fall through to the right
+  // star state, as there).
+  const bool left_flow = sl >= 0.0, right_flow = sr <= 0.0;
+  const bool left = left_flow || (!right_flow && contact >= 0.0);
+  double s[4];
 #pragma unroll
-  for (int v = 0; v < 4; ++v) {
-    double acc = 0.0;
-#pragma unroll
-    for (int m = 0; m < M; ++m)
-      acc += __ldg(u + (static_cast<std::int64_t>(v) * M + m) * ne + e) * b[m];
-    s[v] = acc;
+  for (int v = 0; v < 4; ++v)
+    s[v] = left ? l[v] : r[v];
+  const double vx = left ? lv.vx : rv.vx, vy = left ? lv.vy : rv.vy, p = left ? lv.p : rv.p;
+  const double un = left ? lu : ru, wave = left ? sl : sr;
+  const double energy = s[3] + p;
+  f[0] = nx * s[1] + ny * s[2];
+  f[1] = nx * (s[1] * vx + p) + ny * (s[1] * vy);
+  f[2] = nx * (s[2] * vx) + ny * (s[2] * vy + p);
+  f[3] = nx * (energy * vx) + ny * (energy * vy);
+  if (!left_flow && !right_flow) {
+    const double rho_star = s[0] * (wave - un) / (wave - contact);
+    const double shift = contact - un;
+    const double e_star = s[3] / s[0] + shift * (contact + p / (s[0] * (wave - un)));
+    f[0] = f[0] + wave * (rho_star - s[0]);
+    f[1] = f[1] + wave * (rho_star * (vx + shift * nx) - s[1]);
+    f[2] = f[2] + wave * (rho_star * (vy + shift * ny) - s[2]);
+    f[3] = f[3] + wave * (rho_star * e_star - s[3]);
   }
 }
 
+// The two lanes of an element (lanes i and i + 16 of a warp) hold two of its
+// four variables each, for every point; at a pair of points each lane takes
+// one point whole.  share_points: mine[k][v] are this lane's two variables at
+// points k = 0, 1; full[v] becomes all four variables at point `half`.
+__device__ __forceinline__ double across(double x) { return __shfl_xor_sync(0xffffffffu, x, 16); }
+
+__device__ __forceinline__ void share_points(int half, const double (&mine)[2][2],
+                                             double (&full)[4]) {
+#pragma unroll
+  for (int v = 0; v < 2; ++v) {
+    const double other = across(half ? mine[0][v] : mine[1][v]);
+    full[v] = half ? other : mine[0][v];
+    full[2 + v] = half ? mine[1][v] : other;
+  }
+}
+
+// And back: full[v] is a quantity of this lane's point; out[k][v] becomes this
+// lane's two variables of it at points k = 0, 1.
+__device__ __forceinline__ void return_points(int half, const double (&full)[4],
+                                              double (&out)[2][2]) {
+#pragma unroll
+  for (int v = 0; v < 2; ++v) {
+    const double other = across(half ? full[v] : full[2 + v]);
+    out[0][v] = half ? other : full[v];
+    out[1][v] = half ? full[2 + v] : other;
+  }
+}
+
+// This lane's two variables at a point with basis b: the modal sum over modes
+// 0..M-1.  (Started from the first product instead of from 0.0 plus it: a
+// zero's sign apart, which no term below keeps, the same double.)
 template <int M>
-__device__ __forceinline__ void eval_local(const double (&c)[4][M], const double *b, double *s) {
+__device__ __forceinline__ void eval_pair(const double (&c)[2][M], const double *b, double *s) {
 #pragma unroll
-  for (int v = 0; v < 4; ++v) {
-    double acc = 0.0;
+  for (int v = 0; v < 2; ++v) {
+    double acc = c[v][0] * b[0];
 #pragma unroll
-    for (int m = 0; m < M; ++m)
+    for (int m = 1; m < M; ++m)
       acc += c[v][m] * b[m];
     s[v] = acc;
   }
 }
 
+// One stage, a block of 64 consecutive elements, two lanes per element.
+//
+// Bound by the FP64 pipe (64 results a clock per SM; every product and sum is
+// its own instruction: about 7,900 per element at P2, 57 us of pipe time at
+// 131,072 elements) and by what does not overlap with it (the state's loads
+// and stores, the phases' barriers).  Against one thread per element (254
+// registers, 8 warps per SM, P3 spilling, each face's flux evaluated by both
+// its elements), per stage on a B200: P1 at 131,072 elements 54 -> 47 us, P2
+// 126 -> 94 us, P3 at 51,842 elements 150 -> 92 us.
+//   * Two lanes per element (each half the variables: half the registers, twice
+//     the warps per SM) share out the points of the volume rule, so no flux is
+//     evaluated twice for it; duplicated are only the gradients' few products.
+//   * A face between two elements of the block is evaluated once, for its left
+//     element (the doubles its right element would compute), and every face's
+//     points are shared out over the whole block.
+//   * Terms that are zero by construction are not summed: mode 0's gradient,
+//     and the xi-derivative of the modes with i = 0 (constant along xi), whose
+//     gradient is then one product per direction; the factor 0.5 of the
+//     gradients is taken into the map's columns (exact).
+// Phases: A the traces of both sides at the face points (shared memory), B the
+// listed faces' fluxes, over the evaluating side's trace, C the volume term,
+// then the lifts in slot order, so each residual is summed as before.
+template <int P> struct StageBlock {
+  static constexpr int QF = TriShape<P>::QF, E = 64;
+  FaceTable<P, double> table;
+  double own[3][QF][4][E];     // each slot's own trace, then its flux
+  double outside[3][QF][4][E]; // the trace across, where it is not in the block
+  std::int16_t partner[3][E];  // in the block: the slot across, k * E + element; else -1
+  std::int16_t local[3][E];    // the neighbour's element of the block, -1 outside, -2 boundary
+  std::uint8_t code[3][E];
+  std::uint16_t items[3 * E];  // slots to evaluate, k * E + element
+  int count;
+};
+
+// Resident blocks per SM the registers are sized for: 5 (96 registers) at P0
+// to P2, 4 (128) at P3, where the two coefficient arrays alone take 80.
+// Measured per stage: P2 94 us (4: 99, 3: 110, 6: 102), P3 92 us (3: 93, 5: 100).
+template <int P> constexpr int kStageBlocks = P < 3 ? 5 : 4;
+
 template <int P>
-__global__ void __launch_bounds__(128) euler_tri_stage_f64(const StageArgs a) {
+__global__ void __launch_bounds__(128, kStageBlocks<P>) euler_tri_stage_f64(const StageArgs a) {
   using S = TriShape<P>;
-  constexpr int M = S::M, QV = S::QV, QF = S::QF;
+  constexpr int M = S::M, QV = S::QV, QF = S::QF, E = StageBlock<P>::E;
+  extern __shared__ __align__(16) unsigned char stage_smem[];
+  StageBlock<P> &B = *reinterpret_cast<StageBlock<P> *>(stage_smem);
   const std::int64_t ne = a.mesh.ne;
-  const std::int64_t e = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (e >= ne)
-    return;
-  const double *__restrict__ in = a.in;
+  const int lane = threadIdx.x & 31, half = lane >> 4;
+  const int te = (threadIdx.x >> 5) * 16 + (lane & 15);
+  const std::int64_t first = static_cast<std::int64_t>(blockIdx.x) * E;
+  const int count = ne - first < E ? static_cast<int>(ne - first) : E;
+  const bool active = te < count;
+  const std::int64_t e = active ? first + te : ne - 1; // (every lane takes part in the exchanges)
   const VolumeTable<P, double> &T = volume_table<P>();
-  const FaceTable<P, double> *__restrict__ F = static_cast<const FaceTable<P, double> *>(a.face_table);
   const double gamma = a.gamma;
+  // This lane's rows: variables 2 half and 2 half + 1.
+  const std::int64_t rows = static_cast<std::int64_t>(2 * half) * M * ne;
+  const double *__restrict__ in = a.in + rows;
 
-  double c[4][M], r[4][M];
+  double c[2][M], r[2][M];
 #pragma unroll
-  for (int v = 0; v < 4; ++v)
+  for (int v = 0; v < 2; ++v)
 #pragma unroll
-    for (int m = 0; m < M; ++m) {
+    for (int m = 0; m < M; ++m)
       c[v][m] = in[(static_cast<std::int64_t>(v) * M + m) * ne + e];
-      r[v][m] = 0.0;
-    }
   const double *__restrict__ geo = a.mesh.geo;
-  const double ax = geo[e], ay = geo[ne + e], bx = geo[2 * ne + e], by = geo[3 * ne + e];
-
-  // Volume term: sum_q w_q (F_x . d(phi)/dx + F_y . d(phi)/dy) det(J).
-#pragma unroll 1
-  for (int q = 0; q < QV; ++q) {
-    double s[4], fx[4], fy[4];
-    eval_local<M>(c, T.phi[q], s);
-    flux_xy(gamma, s, fx, fy);
-    const double w = T.w[q];
-#pragma unroll
-    for (int m = 0; m < M; ++m) {
-      const double gxi = T.dxi[q][m], geta = T.deta[q][m];
-      const double gx = 0.5 * (by * gxi - ay * geta);
-      const double gy = 0.5 * (-bx * gxi + ax * geta);
-#pragma unroll
-      for (int v = 0; v < 4; ++v)
-        r[v][m] += w * (fx[v] * gx + fy[v] * gy);
-    }
+  {
+    const double *src = static_cast<const double *>(a.face_table);
+    double *dst = reinterpret_cast<double *>(&B.table);
+    for (int i = threadIdx.x; i < static_cast<int>(sizeof(B.table) / sizeof(double)); i += 128)
+      dst[i] = src[i];
   }
+  if (threadIdx.x == 0)
+    B.count = 0;
+  __syncthreads();
 
-  // Face terms in ascending global face index.  A neighbour's trace at the
-  // face's points is gathered once per face: each of its coefficients is
-  // loaded once and added into every point's sum (each sum still runs over
-  // the modes 0..M-1 from 0.0), and the sums wait in this thread's column of
-  // shared memory for the point loop.
-  __shared__ double outside[QF * 4][128];
-  const int t = threadIdx.x;
-  // u^n (read by the combination at the end of stages 2 and 3) into L1 while
-  // the faces run; no registers wait on it.
-  if (a.stage > 0) {
-#pragma unroll
-    for (int row = 0; row < 4 * M; ++row)
-      asm volatile("prefetch.global.L1 [%0];\n" ::"l"(a.u0 + static_cast<std::int64_t>(row) * ne + e));
-  }
+  // A. Traces at the face points, in the face's point order.
 #pragma unroll 1
   for (int k = 0; k < 3; ++k) {
     const std::int32_t raw = a.mesh.slot_nbr[k * ne + e];
     const std::int32_t nb =
         raw >= 0 ? static_cast<std::int32_t>(checked_index(raw, ne, a.error)) : raw;
     const unsigned code = a.mesh.slot_code[k * ne + e];
-    const double nx = a.mesh.slot_geo[(3 * k) * ne + e];
-    const double ny = a.mesh.slot_geo[(3 * k + 1) * ne + e];
-    const double scale = a.mesh.slot_geo[(3 * k + 2) * ne + e];
     const bool self_left = code & 1u;
     const int le = (code >> 1) & 3u, re = (code >> 3) & 3u, flip = (code >> 5) & 1u;
-    const double(*lb)[M] = F->lb[le];
-    const double(*rb)[M] = F->rb[(le * 3 + re) * 2 + flip];
-    if (nb >= 0) {
+    const double(*lb)[M] = B.table.lb[le];
+    const double(*rb)[M] = B.table.rb[(le * 3 + re) * 2 + flip];
+    const std::int64_t away = nb - first;
+    const bool inside = nb >= 0 && away >= 0 && away < count;
+    if (half == 0) {
+      B.local[k][te] = static_cast<std::int16_t>(nb < 0 ? -2 : inside ? away : -1);
+      B.code[k][te] = static_cast<std::uint8_t>(code);
+    }
+    {
+      const double(*own_basis)[M] = self_left ? lb : rb;
+#pragma unroll
+      for (int q = 0; q < QF; ++q) {
+        double s[2];
+        eval_pair<M>(c, own_basis[q], s);
+        B.own[k][q][2 * half][te] = s[0];
+        B.own[k][q][2 * half + 1][te] = s[1];
+      }
+    }
+    if (nb >= 0 && !inside) {
+      // Each of the neighbour's coefficients loaded once and added into every
+      // point's sum.
       const double(*ob)[M] = self_left ? rb : lb;
 #pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        double acc[QF];
-#pragma unroll
-        for (int q = 0; q < QF; ++q)
-          acc[q] = 0.0;
+      for (int v = 0; v < 2; ++v) {
+        double sum[QF];
 #pragma unroll
         for (int m = 0; m < M; ++m) {
           const double x = __ldg(in + (static_cast<std::int64_t>(v) * M + m) * ne + nb);
 #pragma unroll
           for (int q = 0; q < QF; ++q)
-            acc[q] += x * ob[q][m];
+            sum[q] = m == 0 ? x * ob[q][0] : sum[q] + x * ob[q][m];
         }
 #pragma unroll
         for (int q = 0; q < QF; ++q)
-          outside[q * 4 + v][t] = acc[q];
+          B.outside[k][q][2 * half + v][te] = sum[q];
+      }
+    } else if (nb < 0 && a.mesh.boundary != 3) {
+#pragma unroll
+      for (int q = 0; q < QF; ++q) {
+        const std::int64_t point = static_cast<std::int64_t>(-nb - 1) * QF + q;
+        const std::int64_t d = checked_index(a.mesh.donor[point], ne, a.error);
+        const double *b = a.mesh.donor_basis + point * M;
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+          double sum = 0.0;
+#pragma unroll
+          for (int m = 0; m < M; ++m)
+            sum += __ldg(in + (static_cast<std::int64_t>(v) * M + m) * ne + d) * b[m];
+          B.outside[k][q][2 * half + v][te] = sum;
+        }
       }
     }
+  }
+  __syncthreads();
+  // The faces to evaluate, and where each slot of the block finds its flux.
+  for (int i = threadIdx.x; i < 3 * E; i += 128) {
+    const int k = i / E, t = i % E;
+    const int other = B.local[k][t];
+    const unsigned code = B.code[k][t];
+    int partner = -1;
+    if (other >= 0) {
+#pragma unroll
+      for (int k2 = 0; k2 < 3; ++k2)
+        if (B.local[k2][other] == t && (B.code[k2][other] ^ code) == 1u)
+          partner = k2 * E + other;
+    }
+    B.partner[k][t] = static_cast<std::int16_t>(partner);
+    const bool listed = t < count && (partner < 0 || (code & 1u));
+    const unsigned ballot = __ballot_sync(0xffffffffu, listed);
+    int base = 0;
+    if (lane == 0 && ballot)
+      base = atomicAdd(&B.count, __popc(ballot));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (listed)
+      B.items[base + __popc(ballot & ((1u << lane) - 1u))] = static_cast<std::uint16_t>(i);
+  }
+  __syncthreads();
+
+  // B. The listed faces, one point per thread.
+  {
+    const int n = B.count;
 #pragma unroll 1
-    for (int q = 0; q < QF; ++q) {
+    for (int u = threadIdx.x; u < n * QF; u += 128) {
+      const int q = u / n, item = B.items[u - q * n];
+      const int k = item / E, t = item % E;
+      const double nx = a.mesh.slot_geo[(3 * k) * ne + first + t];
+      const double ny = a.mesh.slot_geo[(3 * k + 1) * ne + first + t];
+      const bool self_left = B.code[k][t] & 1u;
+      const int partner = B.partner[k][t];
+      const double *own = &B.own[k][q][0][t];
+      // A transmissive boundary's outside state is its own trace.
+      const double *other = partner >= 0 ? &B.own[partner / E][q][0][partner % E]
+                            : B.local[k][t] == -2 && a.mesh.boundary == 3 ? own
+                                                                         : &B.outside[k][q][0][t];
       double ls[4], rs[4], f[4];
-      if (self_left) {
-        eval_local<M>(c, lb[q], ls);
-        if (nb >= 0) {
-#pragma unroll
-          for (int v = 0; v < 4; ++v)
-            rs[v] = outside[q * 4 + v][t];
-        } else if (a.mesh.boundary == 3) {
-#pragma unroll
-          for (int v = 0; v < 4; ++v)
-            rs[v] = ls[v];
-        } else {
-          const std::int64_t point = static_cast<std::int64_t>(-nb - 1) * QF + q;
-          eval_global<M>(in, ne, checked_index(a.mesh.donor[point], ne, a.error),
-                         a.mesh.donor_basis + point * M, rs);
-        }
-      } else {
-#pragma unroll
-        for (int v = 0; v < 4; ++v)
-          ls[v] = outside[q * 4 + v][t];
-        eval_local<M>(c, rb[q], rs);
-      }
-      hllc(gamma, ls, rs, nx, ny, f);
-      const double weight = F->ew[le][q] * scale;
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
-        const double value = f[v] * weight;
-        if (self_left) {
+        const double o = own[v * E], x = other[v * E];
+        ls[v] = self_left ? o : x;
+        rs[v] = self_left ? x : o;
+      }
+      hllc_selected(gamma, ls, rs, nx, ny, f);
 #pragma unroll
-          for (int m = 0; m < M; ++m)
-            r[v][m] -= value * lb[q][m];
-        } else {
+      for (int v = 0; v < 4; ++v)
+        B.own[k][q][v][t] = f[v];
+    }
+  }
+  // u^n (read by the combination at the end of stages 2 and 3) into L1 while
+  // the volume term runs; no registers wait on it.
+  if (a.stage > 0) {
 #pragma unroll
-          for (int m = 0; m < M; ++m)
-            r[v][m] += value * rb[q][m];
+    for (int row = 0; row < 2 * M; ++row)
+      asm volatile("prefetch.global.L1 [%0];\n" ::"l"(a.u0 + rows + static_cast<std::int64_t>(row) * ne + e));
+  }
+
+  // C. Volume term: sum_q w_q (F_x . d(phi)/dx + F_y . d(phi)/dy) det(J).
+#pragma unroll
+  for (int v = 0; v < 2; ++v)
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+      r[v][m] = 0.0;
+  {
+    const double hax = 0.5 * geo[e], nhay = -0.5 * geo[ne + e], nhbx = -0.5 * geo[2 * ne + e],
+                 hby = 0.5 * geo[3 * ne + e];
+    auto accumulate = [&](int q, const double *fx, const double *fy) {
+      const double w = T.w[q];
+#pragma unroll
+      for (int n = 0; n <= P; ++n)
+#pragma unroll
+        for (int i = 0; i <= n; ++i) {
+          const int m = n * (n + 1) / 2 + i;
+          if (m == 0)
+            continue;
+          const double geta = T.deta[q][m];
+          double gx, gy;
+          if (i == 0) {
+            gx = nhay * geta;
+            gy = hax * geta;
+          } else {
+            const double gxi = T.dxi[q][m];
+            gx = hby * gxi + nhay * geta;
+            gy = nhbx * gxi + hax * geta;
+          }
+#pragma unroll
+          for (int v = 0; v < 2; ++v)
+            r[v][m] += w * (fx[v] * gx + fy[v] * gy);
         }
+    };
+#pragma unroll 1
+    for (int q = 0; q < QV; q += 2) {
+      const bool two = q + 1 < QV;
+      const int q1 = two ? q + 1 : q;
+      double s[2][2], full[4], fx[4], fy[4], px[2][2], py[2][2];
+      eval_pair<M>(c, T.phi[q], s[0]);
+      eval_pair<M>(c, T.phi[q1], s[1]);
+      share_points(half, s, full);
+      flux_xy(gamma, full, fx, fy);
+      return_points(half, fx, px);
+      return_points(half, fy, py);
+      accumulate(q, px[0], py[0]);
+      if (two)
+        accumulate(q1, px[1], py[1]);
+    }
+    // Mode 0's volume terms are zero, or NaN where a flux is not finite (which
+    // mode 1's sum then is not either).
+    if constexpr (M > 1) {
+#pragma unroll
+      for (int v = 0; v < 2; ++v)
+        r[v][0] = 0.0 * r[v][1];
+    }
+  }
+  __syncthreads(); // the fluxes are in place
+
+  // Face terms in ascending global face index.
+#pragma unroll 1
+  for (int k = 0; k < 3; ++k) {
+    const unsigned code = B.code[k][te];
+    const double scale = a.mesh.slot_geo[(3 * k + 2) * ne + e];
+    const bool self_left = code & 1u;
+    const int le = (code >> 1) & 3u, re = (code >> 3) & 3u, flip = (code >> 5) & 1u;
+    const double(*own_basis)[M] = self_left ? B.table.lb[le] : B.table.rb[(le * 3 + re) * 2 + flip];
+    const int partner = self_left ? -1 : B.partner[k][te];
+    const double *flux = partner >= 0 ? &B.own[partner / E][0][2 * half][partner % E]
+                                      : &B.own[k][0][2 * half][te];
+#pragma unroll
+    for (int q = 0; q < QF; ++q) {
+      const double weight = B.table.ew[le][q] * scale;
+#pragma unroll
+      for (int v = 0; v < 2; ++v) {
+        const double f = flux[(q * 4 + v) * E];
+        const double value = self_left ? -(f * weight) : f * weight;
+#pragma unroll
+        for (int m = 0; m < M; ++m)
+          r[v][m] += value * own_basis[q][m];
       }
     }
   }
@@ -194,9 +406,11 @@ __global__ void __launch_bounds__(128) euler_tri_stage_f64(const StageArgs a) {
   // Mass inverse and the Shu-Osher combination.
   const double inv = geo[4 * ne + e];
   const double dt = a.dt ? *a.dt : a.dt_value;
+  const double *__restrict__ u0 = a.u0 + rows;
+  double *__restrict__ out = a.out + rows;
   double rho[M];
 #pragma unroll
-  for (int v = 0; v < 4; ++v)
+  for (int v = 0; v < 2; ++v)
 #pragma unroll
     for (int m = 0; m < M; ++m) {
       const std::int64_t idx = (static_cast<std::int64_t>(v) * M + m) * ne + e;
@@ -205,17 +419,18 @@ __global__ void __launch_bounds__(128) euler_tri_stage_f64(const StageArgs a) {
       if (a.stage == 0)
         o = c[v][m] + dt * rr;
       else if (a.stage == 1)
-        o = 0.75 * a.u0[idx] + 0.25 * (c[v][m] + dt * rr);
+        o = 0.75 * u0[idx] + 0.25 * (c[v][m] + dt * rr);
       else
-        o = (1.0 / 3.0) * a.u0[idx] + (2.0 / 3.0) * (c[v][m] + dt * rr);
-      a.out[idx] = o;
+        o = (1.0 / 3.0) * u0[idx] + (2.0 / 3.0) * (c[v][m] + dt * rr);
+      if (active)
+        out[idx] = o;
       if (v == 0)
         rho[m] = o;
     }
 
-  // Modal-decay sensor on the density modes of the new stage
+  // Modal-decay sensor on the density modes (lanes of half 0) of the new stage
   // (limiting/troubled_cell/modal_decay.hpp:23-33, euler_modal_limiter.cpp:18-24).
-  if (a.sense) {
+  if (a.sense && half == 0 && active) {
     double total = 0.0, high = 0.0;
 #pragma unroll
     for (int m = 0; m < M; ++m) {
@@ -225,20 +440,20 @@ __global__ void __launch_bounds__(128) euler_tri_stage_f64(const StageArgs a) {
     }
     const bool troubled = !(total == 0.0 || high / total <= a.threshold);
     a.flags[e] = troubled ? 1 : 0;
-    const unsigned active = __activemask();
-    const unsigned ballot = __ballot_sync(active, troubled);
+    const unsigned voting = __activemask();
+    const unsigned ballot = __ballot_sync(voting, troubled);
     if (ballot) {
-      const int lane = threadIdx.x & 31;
       const int leader = __ffs(ballot) - 1;
       int base = 0;
       if (lane == leader)
         base = atomicAdd(a.troubled_count, __popc(ballot));
-      base = __shfl_sync(active, base, leader);
+      base = __shfl_sync(voting, base, leader);
       if (troubled)
         a.troubled[base + __popc(ballot & ((1u << lane) - 1u))] = static_cast<std::int32_t>(e);
     }
   }
 }
+
 
 // ---- limiter ------------------------------------------------------------------
 
@@ -829,8 +1044,23 @@ template <int P> void upload_volume(const void *symbol) {
 }
 
 template <int P> void stage(const StageArgs &a, cudaStream_t s) {
-  const unsigned blocks = static_cast<unsigned>((a.mesh.ne + 127) / 128);
-  euler_tri_stage_f64<P><<<blocks, 128, 0, s>>>(a);
+  constexpr int bytes = sizeof(StageBlock<P>);
+  // Above 48 KiB (P3) the attribute opts in, once per device.
+  if constexpr (bytes > 48 * 1024) {
+    static bool opted_in[64] = {};
+    int device = 0;
+    check(cudaGetDevice(&device), "cudaGetDevice");
+    if (device >= 64 || !opted_in[device]) {
+      check(cudaFuncSetAttribute(euler_tri_stage_f64<P>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, bytes),
+            "stage kernel shared memory");
+      if (device < 64)
+        opted_in[device] = true;
+    }
+  }
+  constexpr int E = StageBlock<P>::E;
+  const unsigned blocks = static_cast<unsigned>((a.mesh.ne + E - 1) / E);
+  euler_tri_stage_f64<P><<<blocks, 128, bytes, s>>>(a);
 }
 
 } // namespace
