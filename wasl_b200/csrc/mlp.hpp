@@ -15,7 +15,7 @@ namespace wasl_b200 {
 constexpr int kMlpHidden = 64;
 constexpr int kMlpMaxFeatures = 48;
 constexpr int kMlpMaxModes = 10; // P3 triangles
-constexpr int kMlpBatch = 64; // samples per training block
+constexpr int kMlpBatch = 64; // a mini-batch is a multiple of this
 
 // Offsets of each parameter block in the flat FP32 vector:
 // W1 [64][F], b1 [64], W2 [64][64], b2 [64], w3 [64], b3.
@@ -58,13 +58,25 @@ void launch_mlp_features(const double *state, std::int64_t ne, int M,
                          const std::int32_t *neighbors, int F, double threshold,
                          int highest_degree_begin, float *features, std::uint8_t *labels,
                          cudaStream_t stream);
+// Training scratch: one gradient row and one loss per block of the pass.
+struct MlpWorkspace {
+  float *rows = nullptr;    // [mlp_train_rows][shape.count]
+  double *losses = nullptr; // [mlp_train_rows]
+};
+// Rows the pass over `samples` samples (a multiple of kMlpBatch) writes.
+int mlp_train_rows(std::int64_t samples);
 void launch_mlp_train(const MlpShape &shape, const float *params, const float *features,
                       const std::uint8_t *labels, std::int64_t n, std::int64_t first,
-                      std::int64_t blocks, float pos_weight, float *grad, double *loss,
+                      std::int64_t samples, float pos_weight, const MlpWorkspace &workspace,
                       cudaStream_t stream);
-void launch_mlp_adam(std::int64_t count, float *params, float *grad, float *m1, float *m2,
-                     float lr, float beta1, float beta2, float eps, std::int64_t step, float scale,
-                     cudaStream_t stream);
+// After the pass: the gradient of the summed loss, and that loss.
+void launch_mlp_gradient(const MlpShape &shape, std::int64_t samples,
+                         const MlpWorkspace &workspace, float *grad, double *loss,
+                         cudaStream_t stream);
+// After the pass: one Adam step with the mean gradient, and the summed loss.
+void launch_mlp_adam(const MlpShape &shape, std::int64_t samples, const MlpWorkspace &workspace,
+                     double *loss, float *params, float *m1, float *m2, float lr, float beta1,
+                     float beta2, float eps, std::int64_t step, cudaStream_t stream);
 void launch_mlp_predict(const MlpShape &shape, const float *params, const float *features,
                         std::int64_t n, float *logits, cudaStream_t stream);
 void launch_mlp_indicator(const MlpIndicatorArgs &args, cudaStream_t stream);
@@ -92,11 +104,14 @@ public:
   cudaStream_t stream() const { return stream_; }
 
 private:
+  // The training scratch for `samples` samples (grown when needed, kept).
+  MlpWorkspace workspace(std::int64_t samples);
+
   MlpShape shape_;
   cudaStream_t stream_ = nullptr;
-  DeviceArray<float> params_, grad_, m1_, m2_, data_;
+  DeviceArray<float> params_, rows_, m1_, m2_, data_;
   DeviceArray<std::uint8_t> labels_;
-  DeviceArray<double> loss_;
+  DeviceArray<double> loss_, losses_;
   std::int64_t n_ = 0, cursor_ = 0, step_ = 0;
 };
 

@@ -25,7 +25,6 @@ MlpTrainer::MlpTrainer(int features, std::uint64_t seed, int device) : shape_(ml
   fill(shape_.w3, kMlpHidden, kMlpHidden);
   params_.upload(p, stream_);
   std::vector<float> zero(shape_.count, 0.0f);
-  grad_.upload(zero, stream_);
   m1_.upload(zero, stream_);
   m2_.upload(zero, stream_);
   loss_.resize(1);
@@ -52,23 +51,32 @@ void MlpTrainer::set_data(const float *features, const std::uint8_t *labels, std
   cursor_ = 0;
 }
 
+MlpWorkspace MlpTrainer::workspace(std::int64_t samples) {
+  const std::size_t rows = static_cast<std::size_t>(mlp_train_rows(samples));
+  if (losses_.size() < rows) {
+    // (The stream may still use the old scratch.)
+    cuda_check(cudaStreamSynchronize(stream_), "indicator workspace");
+    rows_.resize(rows * static_cast<std::size_t>(shape_.count));
+    losses_.resize(rows);
+  }
+  return {rows_.get(), losses_.get()};
+}
+
 double MlpTrainer::train(std::int64_t steps, std::int64_t batch, double lr, double pos_weight) {
   if (n_ == 0)
     throw SolverError(WASL_ERR_ARGUMENT, "indicator training: no data set");
   if (batch <= 0 || batch % kMlpBatch != 0)
     throw SolverError(WASL_ERR_ARGUMENT, "indicator training: batch must be a positive multiple"
                                          " of 64");
-  const std::int64_t blocks = batch / kMlpBatch;
+  const MlpWorkspace w = workspace(batch);
   double loss = 0.0;
   for (std::int64_t s = 0; s < steps; ++s) {
-    cuda_check(cudaMemsetAsync(loss_.get(), 0, sizeof(double), stream_), "loss reset");
-    launch_mlp_train(shape_, params_.get(), data_.get(), labels_.get(), n_, cursor_, blocks,
-                     static_cast<float>(pos_weight), grad_.get(), loss_.get(), stream_);
+    launch_mlp_train(shape_, params_.get(), data_.get(), labels_.get(), n_, cursor_, batch,
+                     static_cast<float>(pos_weight), w, stream_);
     cursor_ = (cursor_ + batch) % n_;
     ++step_;
-    launch_mlp_adam(shape_.count, params_.get(), grad_.get(), m1_.get(), m2_.get(),
-                    static_cast<float>(lr), 0.9f, 0.999f, 1e-8f, step_,
-                    1.0f / static_cast<float>(batch), stream_);
+    launch_mlp_adam(shape_, batch, w, loss_.get(), params_.get(), m1_.get(), m2_.get(),
+                    static_cast<float>(lr), 0.9f, 0.999f, 1e-8f, step_, stream_);
   }
   cuda_check(cudaMemcpyAsync(&loss, loss_.get(), sizeof(double), cudaMemcpyDeviceToHost, stream_),
              "loss");
@@ -87,10 +95,10 @@ double MlpTrainer::gradient(const float *features, const std::uint8_t *labels, s
                              cudaMemcpyHostToDevice, stream_),
              "gradient data");
   cuda_check(cudaMemcpyAsync(y.get(), labels, n, cudaMemcpyHostToDevice, stream_), "labels");
-  cuda_check(cudaMemsetAsync(g.get(), 0, sizeof(float) * shape_.count, stream_), "grad reset");
-  cuda_check(cudaMemsetAsync(loss_.get(), 0, sizeof(double), stream_), "loss reset");
-  launch_mlp_train(shape_, params_.get(), f.get(), y.get(), n, 0, n / kMlpBatch,
-                   static_cast<float>(pos_weight), g.get(), loss_.get(), stream_);
+  const MlpWorkspace w = workspace(n);
+  launch_mlp_train(shape_, params_.get(), f.get(), y.get(), n, 0, n,
+                   static_cast<float>(pos_weight), w, stream_);
+  launch_mlp_gradient(shape_, n, w, g.get(), loss_.get(), stream_);
   double loss = 0.0;
   cuda_check(cudaMemcpyAsync(grad_out, g.get(), sizeof(float) * shape_.count,
                              cudaMemcpyDeviceToHost, stream_),
