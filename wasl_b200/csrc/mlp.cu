@@ -92,15 +92,16 @@ __global__ void mlp_features_kernel(const double *state, std::int64_t ne, int M,
 // mini-batch, each block leaving the gradient of its samples' summed loss in
 // its own row of a workspace, then the rows' sum and the update.
 //
-// The pass, per tile of 32 samples (256 threads): the tile and the network
-// (weights rounded to BF16, held as FP32) in shared memory, every product from
-// there with 8 or 16 results per thread in registers.  Bound by shared-memory
-// reads (one 16-byte and one 8-byte read per 8 multiply-adds), about 5 us; 32
-// samples, not 64, so that a batch of 4,096 fills 128 of 148 SMs.  Against
-// blocks of 64 samples whose threads read each weight from global memory per
-// product and added their gradients atomically: 240 -> 13 us per step of 4,096
-// samples and 48 features.  The rows make the sum's order fixed: the same data
-// gives the same weights, bit for bit.
+// The pass, per tile of 32 samples (256 threads): the tile and the network in
+// shared memory, every product from there with 8 or 16 results per thread in
+// registers.  Bound by the latency of its dozen barriers with 8 warps per SM
+// and by shared-memory reads (one 16-byte and one 8-byte read per 8
+// multiply-adds); 32 samples, not 64, so that a batch of 4,096 fills 128 of 148
+// SMs.  Per step of 4,096 samples and 48 features: 22 us (the pass 12, the
+// update 6), against 240 us for blocks of 64 samples whose threads read each
+// weight from global memory per product and added their gradients atomically.
+// The rows make the sum's order fixed: the same data gives the same weights,
+// bit for bit.
 namespace {
 
 constexpr int kTrainTile = 32;   // samples per tile
@@ -108,12 +109,41 @@ constexpr int kTrainRow = 36;    // floats per row of 32 samples (16-byte aligne
 constexpr int kWeightRow = 66;   // floats per row of 64 outputs (8-byte aligned)
 constexpr int kTrainBlocks = 296; // at most: two resident blocks on each of 148 SMs
 
-template <int KF> struct TrainSmem {
+// The network as the pass reads it (weights rounded to BF16, held as FP32),
+// laid out in global memory by the update so that a block copies it as it is.
+template <int KF> struct alignas(16) TrainNet {
   static constexpr int F = KF * 16, Hd = kMlpHidden;
-  float w1[F][kWeightRow];  // W1 transposed: [feature][unit]
-  float w2[Hd][kWeightRow]; // W2 transposed: [input][output]
+  float w2[Hd][kWeightRow];  // W2 transposed: [input][output]
   float w2n[Hd][kWeightRow]; // W2: [output][input]
   float b1[Hd], b2[Hd], w3[Hd];
+  float b3, unused[3];
+  float w1[F][kWeightRow];   // W1 transposed: [feature][unit]
+};
+
+// Parameter i of the flat vector (value v) to its places in the packed network.
+__device__ __forceinline__ void pack_parameter(const MlpShape &sh, std::int64_t i, float v,
+                                               float *packed) {
+  TrainNet<1> &net = *reinterpret_cast<TrainNet<1> *>(packed); // (w1, whose length varies, is last)
+  constexpr int Hd = kMlpHidden;
+  if (i < sh.b1) {
+    net.w1[0][i % sh.features * kWeightRow + i / sh.features] = bf16_round(v);
+  } else if (i < sh.w2) {
+    net.b1[i - sh.b1] = v;
+  } else if (i < sh.b2) {
+    const int r = static_cast<int>(i - sh.w2) / Hd, c = static_cast<int>(i - sh.w2) % Hd;
+    net.w2[c][r] = net.w2n[r][c] = bf16_round(v);
+  } else if (i < sh.w3) {
+    net.b2[i - sh.b2] = v;
+  } else if (i < sh.b3) {
+    net.w3[i - sh.w3] = bf16_round(v);
+  } else {
+    net.b3 = v;
+  }
+}
+
+template <int KF> struct TrainSmem {
+  static constexpr int F = KF * 16, Hd = kMlpHidden;
+  TrainNet<KF> net;
   alignas(16) float x[F][kTrainRow]; // the tile: [feature][sample], and so on
   float h1[Hd][kTrainRow], h2[Hd][kTrainRow], d2[Hd][kTrainRow], d1[Hd][kTrainRow];
   alignas(16) float d3[kTrainTile];
@@ -170,7 +200,7 @@ __device__ __forceinline__ void tile_outer(const float (*a)[kTrainRow], const fl
 // logit (positives weighted pos_weight), backward; block b's gradient of its
 // samples' summed loss to rows[b][count], that loss to losses[b].
 template <int KF>
-__global__ void __launch_bounds__(256, 2) mlp_train_kernel(const MlpShape sh, const float *params,
+__global__ void __launch_bounds__(256, 2) mlp_train_kernel(const MlpShape sh, const float *packed,
                                                            const float *features,
                                                            const std::uint8_t *labels,
                                                            std::int64_t n, std::int64_t first,
@@ -198,20 +228,20 @@ __global__ void __launch_bounds__(256, 2) mlp_train_kernel(const MlpShape sh, co
   load_tile(blockIdx.x);
   // The data is constant; the weights are the launch before's.
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
-  for (int i = t; i < Hd * F; i += 256)
-    S.w1[i % F][i / F] = bf16_round(params[sh.w1 + i]);
-  for (int i = t; i < Hd * Hd; i += 256) {
-    const float w = bf16_round(params[sh.w2 + i]);
-    S.w2[i % Hd][i / Hd] = w;
-    S.w2n[i / Hd][i % Hd] = w;
+  {
+    static_assert(sizeof(TrainNet<KF>) % 16 == 0, "copied in 16-byte pieces");
+    constexpr int pieces = sizeof(TrainNet<KF>) / 16;
+    const float4 *src = reinterpret_cast<const float4 *>(packed);
+    float4 *dst = reinterpret_cast<float4 *>(&S.net);
+#pragma unroll
+    for (int i = 0; i < pieces / 256; ++i)
+      dst[i * 256 + t] = src[i * 256 + t];
+    if (t < pieces % 256)
+      dst[pieces / 256 * 256 + t] = src[pieces / 256 * 256 + t];
   }
-  if (t < Hd) {
-    S.b1[t] = params[sh.b1 + t];
-    S.b2[t] = params[sh.b2 + t];
-    S.w3[t] = bf16_round(params[sh.w3 + t]);
-  }
-  const float b3 = params[sh.b3];
   __syncthreads();
+  const TrainNet<KF> &N = S.net;
+  const float b3 = N.b3;
 
   const int sx = t & 7, jx = t >> 3; // products: samples 4 sx .. 4 sx + 3, units 2 jx, 2 jx + 1
   const int tx = t & 15, ty = t >> 4; // weight gradients: rows ty + 16 i, columns tx + 16 j
@@ -228,8 +258,8 @@ __global__ void __launch_bounds__(256, 2) mlp_train_kernel(const MlpShape sh, co
     for (int u = 0; u < 2; ++u)
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        acc[u][i] = S.b1[2 * jx + u];
-    tile_product<F>(S.x, S.w1, sx, jx, acc);
+        acc[u][i] = N.b1[2 * jx + u];
+    tile_product<F>(S.x, N.w1, sx, jx, acc);
 #pragma unroll
     for (int u = 0; u < 2; ++u)
 #pragma unroll
@@ -240,8 +270,8 @@ __global__ void __launch_bounds__(256, 2) mlp_train_kernel(const MlpShape sh, co
     for (int u = 0; u < 2; ++u)
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        acc[u][i] = S.b2[2 * jx + u];
-    tile_product<Hd>(S.h1, S.w2, sx, jx, acc);
+        acc[u][i] = N.b2[2 * jx + u];
+    tile_product<Hd>(S.h1, N.w2, sx, jx, acc);
 #pragma unroll
     for (int u = 0; u < 2; ++u)
 #pragma unroll
@@ -254,7 +284,7 @@ __global__ void __launch_bounds__(256, 2) mlp_train_kernel(const MlpShape sh, co
       float z = 0.0f;
 #pragma unroll
       for (int i = 0; i < Hd / 8; ++i)
-        z = fmaf(S.w3[part + 8 * i], S.h2[part + 8 * i][s], z);
+        z = fmaf(N.w3[part + 8 * i], S.h2[part + 8 * i][s], z);
 #pragma unroll
       for (int off = 1; off < 8; off <<= 1)
         z += __shfl_xor_sync(0xffffffffu, z, off);
@@ -273,11 +303,11 @@ __global__ void __launch_bounds__(256, 2) mlp_train_kernel(const MlpShape sh, co
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int k = 2 * jx + u, s = 4 * sx + i;
-        S.d2[k][s] = S.h2[k][s] > 0.0f ? S.d3[s] * S.w3[k] : 0.0f;
+        S.d2[k][s] = S.h2[k][s] > 0.0f ? S.d3[s] * N.w3[k] : 0.0f;
         acc[u][i] = 0.0f;
       }
     __syncthreads();
-    tile_product<Hd>(S.d2, S.w2n, sx, jx, acc);
+    tile_product<Hd>(S.d2, N.w2n, sx, jx, acc);
 #pragma unroll
     for (int u = 0; u < 2; ++u)
 #pragma unroll
@@ -332,7 +362,7 @@ __global__ void __launch_bounds__(256, 2) mlp_train_kernel(const MlpShape sh, co
   }
 }
 
-// The rows' sum, 32 parameters per block (each warp every eighth row), and
+// The rows' sum, 32 parameters per block (each warp every sixteenth row), and
 // with it either Adam on the FP32 master weights, the gradient scaled by
 // `scale` (1 / samples), or (params null) the gradient itself to grad; the
 // losses' sum to loss.
@@ -343,20 +373,29 @@ struct MlpUpdateArgs {
   const double *losses = nullptr;
   float *grad = nullptr;
   double *loss = nullptr;
-  float *params = nullptr, *m1 = nullptr, *m2 = nullptr;
+  MlpShape shape;
+  float *params = nullptr, *packed = nullptr, *m1 = nullptr, *m2 = nullptr;
   float lr = 0.0f, beta1 = 0.0f, beta2 = 0.0f, eps = 0.0f, bias1 = 1.0f, bias2 = 1.0f, scale = 1.0f;
 };
 
-__global__ void __launch_bounds__(256) mlp_update_kernel(const MlpUpdateArgs a) {
-  __shared__ float part[8][32];
+__global__ void mlp_pack_kernel(const MlpShape sh, const float *params, float *packed) {
+  const std::int64_t i = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i < sh.count)
+    pack_parameter(sh, i, params[i], packed);
+}
+
+constexpr int kUpdateWarps = 16;
+
+__global__ void __launch_bounds__(32 * kUpdateWarps) mlp_update_kernel(const MlpUpdateArgs a) {
+  __shared__ float part[kUpdateWarps][32];
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const std::int64_t i = static_cast<std::int64_t>(blockIdx.x) * 32 + lane;
   float sum = 0.0f;
   if (i < a.count) {
-#pragma unroll 4
-    for (int r = warp; r < a.row_count; r += 8)
+#pragma unroll 8
+    for (int r = warp; r < a.row_count; r += kUpdateWarps)
       sum += a.rows[static_cast<std::int64_t>(r) * a.count + i];
   }
   part[warp][lane] = sum;
@@ -372,7 +411,8 @@ __global__ void __launch_bounds__(256) mlp_update_kernel(const MlpUpdateArgs a) 
   }
   if (warp != 0 || i >= a.count)
     return;
-  for (int w = 1; w < 8; ++w)
+#pragma unroll
+  for (int w = 1; w < kUpdateWarps; ++w)
     sum += part[w][lane];
   if (!a.params) {
     a.grad[i] = sum;
@@ -383,7 +423,9 @@ __global__ void __launch_bounds__(256) mlp_update_kernel(const MlpUpdateArgs a) 
   const float m2 = a.beta2 * a.m2[i] + (1.0f - a.beta2) * g * g;
   a.m1[i] = m1;
   a.m2[i] = m2;
-  a.params[i] -= a.lr * (m1 / a.bias1) / (sqrtf(m2 / a.bias2) + a.eps);
+  const float p = a.params[i] - a.lr * (m1 / a.bias1) / (sqrtf(m2 / a.bias2) + a.eps);
+  a.params[i] = p;
+  pack_parameter(a.shape, i, p, a.packed);
 }
 
 // Logits of samples with the training forward pass (FP32 SIMT, BF16 rounding).
@@ -957,11 +999,11 @@ void check_launch(cudaError_t rc) {
 // A launch that may start while the launch before it on the stream drains
 // (the kernel waits where it needs that launch's results).
 template <typename... P, typename... A>
-void launch_after(void (*kernel)(P...), unsigned blocks, std::size_t smem, cudaStream_t s,
-                  const A &...args) {
+void launch_after(void (*kernel)(P...), unsigned blocks, unsigned threads, std::size_t smem,
+                  cudaStream_t s, const A &...args) {
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(blocks);
-  config.blockDim = dim3(256);
+  config.blockDim = dim3(threads);
   config.dynamicSmemBytes = smem;
   config.stream = s;
   cudaLaunchAttribute attribute[1];
@@ -973,7 +1015,7 @@ void launch_after(void (*kernel)(P...), unsigned blocks, std::size_t smem, cudaS
 }
 
 template <int KF>
-void train_blocks(const MlpShape &sh, const float *params, const float *features,
+void train_blocks(const MlpShape &sh, const float *features,
                   const std::uint8_t *labels, std::int64_t n, std::int64_t first,
                   std::int64_t tiles, float pos_weight, const MlpWorkspace &w, unsigned blocks,
                   cudaStream_t s) {
@@ -987,12 +1029,14 @@ void train_blocks(const MlpShape &sh, const float *params, const float *features
     if (device < 64)
       opted_in[device] = true;
   }
-  launch_after(mlp_train_kernel<KF>, blocks, sizeof(TrainSmem<KF>), s, sh, params, features, labels,
-               n, first, tiles, pos_weight, w.rows, w.losses);
+  launch_after(mlp_train_kernel<KF>, blocks, 256, sizeof(TrainSmem<KF>), s, sh,
+               static_cast<const float *>(w.packed), features, labels, n, first, tiles, pos_weight,
+               w.rows, w.losses);
 }
 
 void launch_update(const MlpUpdateArgs &a, cudaStream_t s) {
-  launch_after(mlp_update_kernel, static_cast<unsigned>((a.count + 31) / 32), 0, s, a);
+  launch_after(mlp_update_kernel, static_cast<unsigned>((a.count + 31) / 32), 32 * kUpdateWarps, 0,
+               s, a);
 }
 
 } // namespace
@@ -1001,7 +1045,18 @@ int mlp_train_rows(std::int64_t samples) {
   return static_cast<int>(std::min<std::int64_t>(samples / kTrainTile, kTrainBlocks));
 }
 
-void launch_mlp_train(const MlpShape &sh, const float *params, const float *features,
+std::size_t mlp_packed_floats(const MlpShape &sh) {
+  return sizeof(TrainNet<3>) / sizeof(float) -
+         static_cast<std::size_t>(kMlpMaxFeatures - sh.features) * kWeightRow;
+}
+
+void launch_mlp_pack(const MlpShape &sh, const float *params, const MlpWorkspace &w,
+                     cudaStream_t s) {
+  mlp_pack_kernel<<<static_cast<unsigned>((sh.count + 255) / 256), 256, 0, s>>>(sh, params,
+                                                                                w.packed);
+}
+
+void launch_mlp_train(const MlpShape &sh, const float *features,
                       const std::uint8_t *labels, std::int64_t n, std::int64_t first,
                       std::int64_t samples, float pos_weight, const MlpWorkspace &w,
                       cudaStream_t s) {
@@ -1010,9 +1065,9 @@ void launch_mlp_train(const MlpShape &sh, const float *params, const float *feat
     return;
   const std::int64_t tiles = samples / kTrainTile;
   switch (sh.features / 16) {
-  case 1: train_blocks<1>(sh, params, features, labels, n, first, tiles, pos_weight, w, blocks, s); break;
-  case 2: train_blocks<2>(sh, params, features, labels, n, first, tiles, pos_weight, w, blocks, s); break;
-  case 3: train_blocks<3>(sh, params, features, labels, n, first, tiles, pos_weight, w, blocks, s); break;
+  case 1: train_blocks<1>(sh, features, labels, n, first, tiles, pos_weight, w, blocks, s); break;
+  case 2: train_blocks<2>(sh, features, labels, n, first, tiles, pos_weight, w, blocks, s); break;
+  case 3: train_blocks<3>(sh, features, labels, n, first, tiles, pos_weight, w, blocks, s); break;
   default: throw std::invalid_argument("indicator network: unsupported feature count");
   }
 }
@@ -1038,7 +1093,9 @@ void launch_mlp_adam(const MlpShape &sh, std::int64_t samples, const MlpWorkspac
   a.rows = w.rows;
   a.losses = w.losses;
   a.loss = loss;
+  a.shape = sh;
   a.params = params;
+  a.packed = w.packed;
   a.m1 = m1;
   a.m2 = m2;
   a.lr = lr;

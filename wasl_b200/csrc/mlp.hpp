@@ -58,14 +58,21 @@ void launch_mlp_features(const double *state, std::int64_t ne, int M,
                          const std::int32_t *neighbors, int F, double threshold,
                          int highest_degree_begin, float *features, std::uint8_t *labels,
                          cudaStream_t stream);
-// Training scratch: one gradient row and one loss per block of the pass.
+// Training scratch: the network packed for the pass, and one gradient row and
+// one loss per block of it.
 struct MlpWorkspace {
+  float *packed = nullptr;  // [mlp_packed_floats]
   float *rows = nullptr;    // [mlp_train_rows][shape.count]
   double *losses = nullptr; // [mlp_train_rows]
 };
 // Rows the pass over `samples` samples (a multiple of kMlpBatch) writes.
 int mlp_train_rows(std::int64_t samples);
-void launch_mlp_train(const MlpShape &shape, const float *params, const float *features,
+std::size_t mlp_packed_floats(const MlpShape &shape);
+// Packs the parameters (before the first pass with them; the Adam step keeps
+// the packed network in step).
+void launch_mlp_pack(const MlpShape &shape, const float *params, const MlpWorkspace &workspace,
+                     cudaStream_t stream);
+void launch_mlp_train(const MlpShape &shape, const float *features,
                       const std::uint8_t *labels, std::int64_t n, std::int64_t first,
                       std::int64_t samples, float pos_weight, const MlpWorkspace &workspace,
                       cudaStream_t stream);
@@ -109,7 +116,7 @@ private:
 
   MlpShape shape_;
   cudaStream_t stream_ = nullptr;
-  DeviceArray<float> params_, rows_, m1_, m2_, data_;
+  DeviceArray<float> params_, packed_, rows_, m1_, m2_, data_;
   DeviceArray<std::uint8_t> labels_;
   DeviceArray<double> loss_, losses_;
   std::int64_t n_ = 0, cursor_ = 0, step_ = 0;

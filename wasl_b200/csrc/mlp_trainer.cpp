@@ -28,6 +28,8 @@ MlpTrainer::MlpTrainer(int features, std::uint64_t seed, int device) : shape_(ml
   m1_.upload(zero, stream_);
   m2_.upload(zero, stream_);
   loss_.resize(1);
+  packed_.resize(mlp_packed_floats(shape_));
+  cuda_check(cudaMemsetAsync(packed_.get(), 0, packed_.size() * sizeof(float), stream_), "pack");
   cuda_check(cudaStreamSynchronize(stream_), "indicator network setup");
 }
 
@@ -59,7 +61,7 @@ MlpWorkspace MlpTrainer::workspace(std::int64_t samples) {
     rows_.resize(rows * static_cast<std::size_t>(shape_.count));
     losses_.resize(rows);
   }
-  return {rows_.get(), losses_.get()};
+  return {packed_.get(), rows_.get(), losses_.get()};
 }
 
 double MlpTrainer::train(std::int64_t steps, std::int64_t batch, double lr, double pos_weight) {
@@ -69,9 +71,10 @@ double MlpTrainer::train(std::int64_t steps, std::int64_t batch, double lr, doub
     throw SolverError(WASL_ERR_ARGUMENT, "indicator training: batch must be a positive multiple"
                                          " of 64");
   const MlpWorkspace w = workspace(batch);
+  launch_mlp_pack(shape_, params_.get(), w, stream_);
   double loss = 0.0;
   for (std::int64_t s = 0; s < steps; ++s) {
-    launch_mlp_train(shape_, params_.get(), data_.get(), labels_.get(), n_, cursor_, batch,
+    launch_mlp_train(shape_, data_.get(), labels_.get(), n_, cursor_, batch,
                      static_cast<float>(pos_weight), w, stream_);
     cursor_ = (cursor_ + batch) % n_;
     ++step_;
@@ -96,7 +99,8 @@ double MlpTrainer::gradient(const float *features, const std::uint8_t *labels, s
              "gradient data");
   cuda_check(cudaMemcpyAsync(y.get(), labels, n, cudaMemcpyHostToDevice, stream_), "labels");
   const MlpWorkspace w = workspace(n);
-  launch_mlp_train(shape_, params_.get(), f.get(), y.get(), n, 0, n,
+  launch_mlp_pack(shape_, params_.get(), w, stream_);
+  launch_mlp_train(shape_, f.get(), y.get(), n, 0, n,
                    static_cast<float>(pos_weight), w, stream_);
   launch_mlp_gradient(shape_, n, w, g.get(), loss_.get(), stream_);
   double loss = 0.0;
