@@ -251,6 +251,8 @@ struct LineStageArgs {
   std::uint8_t *flags = nullptr;
   std::int32_t *troubled = nullptr;
   std::int32_t *troubled_count = nullptr;
+  unsigned long long *speed_max = nullptr; // Euler: the result's largest CFL speed (or null)
+  unsigned long long *error = nullptr;     // with speed_max
   LineTable table;
 };
 

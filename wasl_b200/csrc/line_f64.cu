@@ -18,6 +18,7 @@
 
 #include "basis.hpp"
 #include "euler_device.cuh"
+#include "hllc_selected.cuh"
 #include "kernels.hpp"
 
 namespace wasl_b200 {
@@ -196,45 +197,236 @@ __device__ __forceinline__ void line_element_stage(const LineStageArgs &a, std::
     }
 }
 
-template <int V, int P>
-__global__ void __launch_bounds__(128) line_stage_f64(const LineStageArgs a) {
+// Modal-decay sensor on the density modes (modal_decay.hpp:23-33).
+template <int M>
+__device__ __forceinline__ void line_sensor(const LineStageArgs &a, std::int64_t e,
+                                            const double (&rho)[M]) {
+  if (!a.sense)
+    return;
+  double total = 0.0, high = 0.0;
+#pragma unroll
+  for (int m = 0; m < M; ++m) {
+    total += rho[m] * rho[m];
+    if (m >= a.highest_degree_begin)
+      high += rho[m] * rho[m];
+  }
+  const bool troubled = !(total == 0.0 || high / total <= a.threshold);
+  a.flags[e] = troubled ? 1 : 0;
+  const unsigned active = __activemask();
+  const unsigned ballot = __ballot_sync(active, troubled);
+  if (ballot) {
+    const int lane = threadIdx.x & 31;
+    const int leader = __ffs(ballot) - 1;
+    int base = 0;
+    if (lane == leader)
+      base = atomicAdd(a.troubled_count, __popc(ballot));
+    base = __shfl_sync(active, base, leader);
+    if (troubled)
+      a.troubled[base + __popc(ballot & ((1u << lane) - 1u))] = static_cast<std::int32_t>(e);
+  }
+}
+
+// Trace of a thread's element at an endpoint, the modes summed from the first
+// product (a zero's sign apart, which no flux keeps, the sum from 0.0).
+template <int M> __device__ __forceinline__ double trace_of(const double (&c)[M], const double *b) {
+  double s = c[0] * b[0];
+#pragma unroll
+  for (int m = 1; m < M; ++m)
+    s += c[m] * b[m];
+  return s;
+}
+
+// Volume term of the Euler residual into r: sum_q w_q F(u_q) dphi/dxi
+// (cpp/include/wasl/dg/euler/line_residual.hpp:34-45).  Mode 0's derivative is
+// zero: its term is zero, or NaN where a flux is not finite (which mode 1's sum
+// then is not either).
+template <int M>
+__device__ __forceinline__ void euler_volume(const LineTable &T, double gamma,
+                                             const double (&c)[4][M], double (&r)[4][M]) {
+#pragma unroll
+  for (int v = 0; v < 4; ++v)
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+      r[v][m] = 0.0;
+  if constexpr (M > 1) {
+#pragma unroll
+    for (int q = 0; q < M; ++q) {
+      double s[4], fx[4], fy[4];
+#pragma unroll
+      for (int v = 0; v < 4; ++v)
+        s[v] = trace_of(c[v], T.phi[q]);
+      flux_xy(gamma, s, fx, fy);
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        const double wf = T.w[q] * fx[v];
+#pragma unroll
+        for (int m = 1; m < M; ++m)
+          r[v][m] += wf * T.dphi[q][m];
+      }
+    }
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+      r[v][0] = 0.0 + 0.0 * r[v][1];
+  } else {
+    // (P0: the same rule, for the NaN of a flux that is not finite.)
+    double s[4], fx[4], fy[4];
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+      s[v] = trace_of(c[v], T.phi[0]);
+    flux_xy(gamma, s, fx, fy);
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+      r[v][0] += T.w[0] * fx[v] * T.dphi[0][0];
+  }
+}
+
+// The Shu-Osher combination of one coefficient (time/ssp_rk3.hpp:44-60).
+__device__ __forceinline__ double combine(int stage, double u0, double c, double dt, double rr) {
+  if (stage == 0)
+    return c + dt * rr;
+  if (stage == 1)
+    return 0.75 * u0 + 0.25 * (c + dt * rr);
+  return (1.0 / 3.0) * u0 + (2.0 / 3.0) * (c + dt * rr);
+}
+
+// One Euler stage with each face's flux evaluated once: a block of 128 threads
+// computes the 128 faces first .. first + 127 (thread t: face first + t, the
+// left face of element first + t) and updates the 127 elements between them;
+// right traces and fluxes pass between neighbouring threads through shared
+// memory.  Bound by the FP64 pipe (two HLLC fluxes of 190 operations per
+// element were more than half of its work) and by the 96 M bytes per element
+// that stages 2 and 3 move.  Four steps at 1,000,003 cells, P2: 1978 -> 843 us
+// (with one thread per element evaluating both its faces: 150 us a stage).
+constexpr int kLineBlock = 128;
+
+// Resident blocks per SM the registers are sized for.  Measured, four steps:
+// P1 (700,001 cells) 486 us (7: 510, 9: 505, no bound: 595); P2 (1,000,003)
+// 843 us (6: 883, 8: 888, no bound: 977); P3 (700,001) 868 us (5: 885, 7:
+// 1002); from P4 on a bound spills (100,001 cells: 272 us without, 312 at 6).
+template <int P> constexpr int kLineBlocks = P <= 1 ? 8 : P == 2 ? 7 : P == 3 ? 6 : 1;
+
+template <int P>
+__global__ void __launch_bounds__(kLineBlock, kLineBlocks<P>) line_euler_stage_f64(const LineStageArgs a) {
+  constexpr int M = P + 1;
+  __shared__ double right[4][kLineBlock], flux[4][kLineBlock];
+  const int t = threadIdx.x;
+  const std::int64_t ne = a.ne;
+  const std::int64_t e = static_cast<std::int64_t>(blockIdx.x) * (kLineBlock - 1) + t;
+  const bool present = e < ne;
+  const LineTable &T = a.table;
+  const double *lb = T.lb, *rb = T.rb;
+  double c[4][M];
+  if (present) {
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+#pragma unroll
+      for (int m = 0; m < M; ++m)
+        c[v][m] = a.in[(static_cast<std::int64_t>(v) * M + m) * ne + e];
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+      right[v][t] = trace_of(c[v], rb);
+  }
+  const bool updates = present && t < kLineBlock - 1;
+  if (a.stage > 0 && updates) {
+    // u^n (read by the combination) into L1 meanwhile.
+#pragma unroll
+    for (int row = 0; row < 4 * M; ++row)
+      asm volatile("prefetch.global.L1 [%0];\n" ::"l"(a.u0 + static_cast<std::int64_t>(row) * ne + e));
+  }
+  __syncthreads();
+  double f[4] = {0.0, 0.0, 0.0, 0.0};
+  if (e <= ne) {
+    // Left and right states of face e: the ends take the periodic image or the
+    // end element's own trace (outflow).
+    double ls[4], rs[4];
+    if (e > 0 && t > 0) {
+#pragma unroll
+      for (int v = 0; v < 4; ++v)
+        ls[v] = right[v][t - 1];
+    } else if (e > 0 || a.left_kind == 0) {
+      trace_global<4, M>(a.in, ne, e > 0 ? e - 1 : ne - 1, rb, ls);
+    } else {
+#pragma unroll
+      for (int v = 0; v < 4; ++v)
+        ls[v] = trace_of(c[v], lb);
+    }
+    if (present) {
+#pragma unroll
+      for (int v = 0; v < 4; ++v)
+        rs[v] = trace_of(c[v], lb);
+    } else if (a.right_kind == 0) {
+      trace_global<4, M>(a.in, ne, 0, lb, rs);
+    } else {
+#pragma unroll
+      for (int v = 0; v < 4; ++v)
+        rs[v] = ls[v];
+    }
+    hllc_selected(a.gamma, ls, rs, 1.0, 0.0, f);
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+      flux[v][t] = f[v];
+  }
+  __syncthreads();
+  if (!updates)
+    return;
+  double r[4][M], rho[M], mean[4];
+  euler_volume(T, a.gamma, c, r);
+  const double inv = a.inv_jacobian[e];
+  const double dt = a.dt ? *a.dt : a.dt_value;
+#pragma unroll
+  for (int v = 0; v < 4; ++v) {
+    const double after = flux[v][t + 1];
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      r[v][m] += lb[m] * f[v];
+      r[v][m] += -rb[m] * after;
+      const std::int64_t idx = (static_cast<std::int64_t>(v) * M + m) * ne + e;
+      const double o = combine(a.stage, a.stage > 0 ? a.u0[idx] : 0.0, c[v][m], dt, r[v][m] * inv);
+      a.out[idx] = o;
+      if (v == 0)
+        rho[m] = o;
+      if (m == 0)
+        mean[v] = o;
+    }
+  }
+  if (a.speed_max) {
+    // The next step's CFL speed from this stage's cell averages (the CFL
+    // kernels' formula), the warp's largest to the word.
+    const double scale = 1.0 / sqrt(2.0);
+    const double sa[4] = {scale * mean[0], scale * mean[1], scale * mean[2], scale * mean[3]};
+    bool physical = true;
+    const double speed = cfl_speed(a.gamma, sa, 1, physical);
+    unsigned long long best = 0;
+    if (physical)
+      best = __double_as_longlong(speed);
+    else
+      raise_error(a.error, kNonPhysicalAverage, e);
+    const unsigned mask = __activemask();
+    const unsigned hi = __reduce_max_sync(mask, static_cast<unsigned>(best >> 32));
+    const unsigned lo = __reduce_max_sync(
+        mask, static_cast<unsigned>(best >> 32) == hi ? static_cast<unsigned>(best) : 0u);
+    if ((t & 31) == __ffs(mask) - 1)
+      atomicMax(a.speed_max, (static_cast<unsigned long long>(hi) << 32) | lo);
+  }
+  line_sensor<M>(a, e, rho);
+}
+
+// One scalar advection stage, one thread per element (bound by the state's
+// bytes: 90% of the HBM rate).
+template <int P>
+__global__ void __launch_bounds__(128) line_scalar_stage_f64(const LineStageArgs a) {
   constexpr int M = P + 1;
   const std::int64_t e = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (e >= a.ne)
     return;
   double rho[M];
-  line_element_stage<V, P>(a, e, a.in, a.u0, a.out, a.stage, a.dt ? *a.dt : a.dt_value, rho);
-
-  // Modal-decay sensor on the density modes (modal_decay.hpp:23-33).
-  if (V == 4 && a.sense) {
-    double total = 0.0, high = 0.0;
-#pragma unroll
-    for (int m = 0; m < M; ++m) {
-      total += rho[m] * rho[m];
-      if (m >= a.highest_degree_begin)
-        high += rho[m] * rho[m];
-    }
-    const bool troubled = !(total == 0.0 || high / total <= a.threshold);
-    a.flags[e] = troubled ? 1 : 0;
-    const unsigned active = __activemask();
-    const unsigned ballot = __ballot_sync(active, troubled);
-    if (ballot) {
-      const int lane = threadIdx.x & 31;
-      const int leader = __ffs(ballot) - 1;
-      int base = 0;
-      if (lane == leader)
-        base = atomicAdd(a.troubled_count, __popc(ballot));
-      base = __shfl_sync(active, base, leader);
-      if (troubled)
-        a.troubled[base + __popc(ballot & ((1u << lane) - 1u))] = static_cast<std::int32_t>(e);
-    }
-  }
+  line_element_stage<1, P>(a, e, a.in, a.u0, a.out, a.stage, a.dt ? *a.dt : a.dt_value, rho);
 }
 
 // A whole run in one launch of one CTA (meshes whose three state buffers fit
 // in its shared memory): the serial run loop of cpp/src/case/serial_case_runner.cpp:107-142
 // (dt clipped to land on end_time; "timestep cannot advance time" ends the
-// run) around the SSP-RK3 stages of line_stage_f64, with a block barrier
+// run) around the SSP-RK3 stages of the stage kernels, with a block barrier
 // between stages instead of a kernel boundary.  The CFL step is fixed
 // (fixed_dt > 0: scalar advection, cfl_timestep.cpp:55-60) or taken from the
 // state each step (Euler: the largest |u| + c of the cell averages,
@@ -314,9 +506,228 @@ template <int V, int P> __global__ void __launch_bounds__(512) line_run_f64(Line
   }
 }
 
+// The same run with one element per thread, for meshes of at most
+// kLineRunThreads - 1 elements (the 400-cell advection run, for one): the
+// stage's coefficients stay in registers over the whole run (and u^n too, for
+// scalar advection; in the thread's column of shared memory for Euler), and
+// only what a neighbour needs passes through shared memory: the one trace an
+// upwind flux reads, or Euler's right traces and face fluxes.  Bound by the
+// FP64 pipe of one SM and the barriers (one per advection stage, two per Euler
+// stage).  400 cells at P2: 0.67 -> 0.34 us per stage against the kernel above,
+// which keeps the three state buffers in shared memory, evaluates every trace
+// twice and reads each coefficient it needs.
+template <int V, int P> struct LineRunLimit {
+  static constexpr int threads = V == 1 ? (P <= 2 ? 1024 : 512) : (P <= 3 ? 512 : 0);
+};
+
+template <int V, int P>
+__global__ void __launch_bounds__(LineRunLimit<V, P>::threads) line_run_registers_f64(LineRunArgs r) {
+  constexpr int M = P + 1;
+  extern __shared__ double run_smem[];
+  const int n = static_cast<int>(r.stage.ne), e = threadIdx.x, T = blockDim.x;
+  const bool active = e < n;
+  const LineTable &table = r.stage.table;
+  const double *lb = table.lb, *rb = table.rb;
+  __shared__ unsigned long long speed_bits[32];
+  __shared__ double first_left[4]; // element 0's left trace (Euler)
+  __shared__ int status;
+  if (e == 0)
+    status = 0;
+  double c[V][M];
+  double un[V == 1 ? M : 1]; // u^n (scalar)
+  double *held = run_smem;   // u^n (Euler): [V M][T]
+#pragma unroll
+  for (int v = 0; v < V; ++v)
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+      c[v][m] = active ? r.state[(v * M + m) * n + e] : 0.0;
+  const double inv = active ? r.stage.inv_jacobian[e] : 0.0;
+  __syncthreads();
+  double time = r.start_time;
+  unsigned long long steps = 0;
+  int buffer = 0;
+  while (time < r.end_time && steps < r.max_steps) {
+    double stable = r.fixed_dt;
+    if constexpr (V == 4) {
+      // Largest cell-average speed, with the CFL kernels' physical-state check.
+      unsigned long long best = 0;
+      if (active) {
+        const double scale = 1.0 / sqrt(2.0);
+        const double sa[4] = {scale * c[0][0], scale * c[1][0], scale * c[2][0], scale * c[3][0]};
+        bool physical = true;
+        const double speed = cfl_speed(r.stage.gamma, sa, 1, physical);
+        if (!physical) {
+          raise_error(r.error, kNonPhysicalAverage, e);
+          status = 2;
+        } else {
+          best = __double_as_longlong(speed);
+        }
+      }
+      for (int off = 16; off > 0; off >>= 1) {
+        const unsigned long long o = __shfl_down_sync(0xffffffffu, best, off);
+        best = o > best ? o : best;
+      }
+      if ((e & 31) == 0)
+        speed_bits[e >> 5] = best;
+      __syncthreads();
+      best = 0;
+      for (int w = 0; w < (T >> 5); ++w)
+        best = speed_bits[w] > best ? speed_bits[w] : best;
+      __syncthreads();
+      if (status)
+        break;
+      const double speed = __longlong_as_double(static_cast<long long>(best));
+      stable = speed > 0.0 ? r.cfl * r.length / (speed * (2 * P + 1)) : 0.0;
+    }
+    const double remaining = r.end_time - time;
+    const double dt = stable > 0.0 ? (remaining < stable ? remaining : stable) : remaining;
+    if (dt <= 0.0 || time + dt == time) {
+      status = 1; // every thread finds the same dt: the same value, one break
+      break;
+    }
+    if constexpr (V == 1) {
+#pragma unroll
+      for (int m = 0; m < M; ++m)
+        un[m] = c[0][m];
+    } else {
+#pragma unroll
+      for (int v = 0; v < V; ++v)
+#pragma unroll
+        for (int m = 0; m < M; ++m)
+          held[(v * M + m) * T + e] = c[v][m];
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      if constexpr (V == 1) {
+        // The upwind flux reads the left state's trace for a speed >= 0 and
+        // the right state's otherwise (scalar_advection.hpp:36-42); two
+        // buffers, so one barrier per stage keeps readers and writers apart.
+        const double speed = r.stage.speed;
+        const bool forward = speed >= 0.0;
+        double *traces = run_smem + buffer * T;
+        buffer ^= 1;
+        const double own = trace_of(c[0], forward ? rb : lb);
+        traces[e] = own;
+        double rhs[M];
+#pragma unroll
+        for (int m = 0; m < M; ++m)
+          rhs[m] = 0.0;
+        if constexpr (P > 0) {
+#pragma unroll
+          for (int q = 0; q < P; ++q) {
+            const double wf = table.w[q] * (speed * trace_of(c[0], table.phi[q]));
+#pragma unroll
+            for (int m = 1; m < M; ++m)
+              rhs[m] += wf * table.dphi[q][m];
+          }
+          rhs[0] = 0.0 + 0.0 * rhs[1]; // (mode 0's derivative is zero)
+        } else {
+          rhs[0] += table.w[0] * (speed * trace_of(c[0], table.phi[0])) * table.dphi[0][0];
+        }
+        __syncthreads();
+        double before, after;
+        if (forward) {
+          double left;
+          if (e > 0)
+            left = traces[e - 1];
+          else if (r.stage.left_kind == 1)
+            left = r.stage.left_value;
+          else if (r.stage.left_kind == 2)
+            left = trace_of(c[0], lb);
+          else
+            left = traces[n - 1];
+          before = speed * left;
+          after = speed * own;
+        } else {
+          double right;
+          if (e + 1 < n)
+            right = traces[e + 1];
+          else if (r.stage.right_kind == 1)
+            right = r.stage.right_value;
+          else if (r.stage.right_kind == 2)
+            right = trace_of(c[0], rb);
+          else
+            right = traces[0];
+          before = speed * own;
+          after = speed * right;
+        }
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+          rhs[m] += lb[m] * before;
+          rhs[m] -= rb[m] * after;
+          c[0][m] = combine(k, un[m], c[0][m], dt, rhs[m] * inv);
+        }
+      } else {
+        double(*right)[LineRunLimit<V, P>::threads] = reinterpret_cast<
+            double(*)[LineRunLimit<V, P>::threads]>(run_smem + V * M * T);
+        double(*flux)[LineRunLimit<V, P>::threads] = right + 4;
+        double own[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          right[v][e] = trace_of(c[v], rb);
+          own[v] = trace_of(c[v], lb);
+          if (e == 0)
+            first_left[v] = own[v];
+        }
+        __syncthreads();
+        double f[4] = {0.0, 0.0, 0.0, 0.0};
+        if (e <= n) {
+          // Face e, between element e - 1 and this thread's.
+          double ls[4];
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            ls[v] = e > 0 ? right[v][e - 1] : r.stage.left_kind == 0 ? right[v][n - 1] : own[v];
+            if (e == n)
+              own[v] = r.stage.right_kind == 0 ? first_left[v] : ls[v];
+          }
+          hllc_selected(r.stage.gamma, ls, own, 1.0, 0.0, f);
+#pragma unroll
+          for (int v = 0; v < 4; ++v)
+            flux[v][e] = f[v];
+        }
+        double rhs[4][M];
+        euler_volume(table, r.stage.gamma, c, rhs);
+        __syncthreads();
+        if (active) {
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            const double after = flux[v][e + 1];
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+              rhs[v][m] += lb[m] * f[v];
+              rhs[v][m] += -rb[m] * after;
+              c[v][m] = combine(k, held[(v * M + m) * T + e], c[v][m], dt, rhs[v][m] * inv);
+            }
+          }
+        }
+      }
+    }
+    time += dt;
+    ++steps;
+  }
+  __syncthreads();
+  if (active) {
+#pragma unroll
+    for (int v = 0; v < V; ++v)
+#pragma unroll
+      for (int m = 0; m < M; ++m)
+        r.state[(v * M + m) * n + e] = c[v][m];
+  }
+  if (e == 0) {
+    r.result[0] = steps;
+    r.result[1] = static_cast<unsigned long long>(__double_as_longlong(time));
+    r.result[2] = static_cast<unsigned long long>(status);
+  }
+}
+
 template <int V, int P> void launch(const LineStageArgs &a, cudaStream_t s) {
-  const unsigned blocks = static_cast<unsigned>((a.ne + 127) / 128);
-  line_stage_f64<V, P><<<blocks, 128, 0, s>>>(a);
+  if constexpr (V == 4) {
+    constexpr int E = kLineBlock - 1;
+    // (ne + 1 faces; the last one may fall on a block's last thread)
+    line_euler_stage_f64<P><<<static_cast<unsigned>((a.ne + E - 1) / E), kLineBlock, 0, s>>>(a);
+  } else {
+    line_scalar_stage_f64<P><<<static_cast<unsigned>((a.ne + 127) / 128), 128, 0, s>>>(a);
+  }
 }
 
 template <int V> void launch_order(int p, const LineStageArgs &a, cudaStream_t s) {
@@ -332,18 +743,38 @@ template <int V> void launch_order(int p, const LineStageArgs &a, cudaStream_t s
   }
 }
 
-template <int V, int P> void launch_run(const LineRunArgs &r, cudaStream_t s) {
-  const std::size_t bytes = line_run_bytes(V, P, r.stage.ne);
-  static bool opted_in[64] = {};
+// Shared memory above the default needs the opt-in attribute, once per device.
+template <typename Kernel> void run_opt_in(Kernel kernel, std::size_t bytes, bool (&opted_in)[64]) {
   int device = 0;
   if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64)
     throw std::runtime_error("resident run: no usable CUDA device");
-  if (!opted_in[device]) {
-    if (cudaFuncSetAttribute(line_run_f64<V, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(kLineRunMaxBytes)) != cudaSuccess)
-      throw std::runtime_error("resident run: shared memory opt-in failed");
-    opted_in[device] = true;
+  if (opted_in[device])
+    return;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           static_cast<int>(bytes)) != cudaSuccess)
+    throw std::runtime_error("resident run: shared memory opt-in failed");
+  opted_in[device] = true;
+}
+
+// One element (and, for Euler, one face) per thread where the block has the
+// threads and the registers for it; else the elements of a thread in turn.
+template <int V, int P> void launch_run(const LineRunArgs &r, cudaStream_t s) {
+  constexpr int limit = LineRunLimit<V, P>::threads;
+  if constexpr (limit > 0) {
+    if (r.stage.ne < limit) {
+      static bool opted_in[64] = {};
+      constexpr std::size_t most = sizeof(double) * limit * (V == 1 ? 2 : V * (P + 1) + 8);
+      run_opt_in(line_run_registers_f64<V, P>, most, opted_in);
+      const unsigned threads = static_cast<unsigned>((r.stage.ne + 1 + 31) / 32 * 32);
+      const std::size_t bytes =
+          sizeof(double) * (V == 1 ? 2 * threads : V * (P + 1) * threads + 8 * limit);
+      line_run_registers_f64<V, P><<<1, threads, bytes, s>>>(r);
+      return;
+    }
   }
+  const std::size_t bytes = line_run_bytes(V, P, r.stage.ne);
+  static bool opted_in[64] = {};
+  run_opt_in(line_run_f64<V, P>, kLineRunMaxBytes, opted_in);
   const std::int64_t threads = std::min<std::int64_t>(512, (r.stage.ne + 31) / 32 * 32);
   line_run_f64<V, P><<<1, static_cast<unsigned>(threads), bytes, s>>>(r);
 }
