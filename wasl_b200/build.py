@@ -31,14 +31,16 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 NVCC = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++20", "-lineinfo", f"-I{INCLUDE}", f"-I{CSRC}",
-          "-Xcompiler", "-fPIC,-ffp-contract=off", "--expt-relaxed-constexpr"]
+          "-Xcompiler", "-fPIC,-ffp-contract=off", "--expt-relaxed-constexpr",
+          "-Xfatbin", "-compress-all"]
 
 # file -> extra flags
 SOURCES = {
     "euler_tri_f64.cu": ["--fmad=false"],
     # FP32 here carries only perturbations around FP64 means: approximate
     # division/square root and flushed denormals cost nothing in accuracy.
-    "euler_tri_mixed.cu": ["-ftz=true", "-prec-div=false", "-prec-sqrt=false"],
+    "euler_tri_mixed_kernels.cu": ["-ftz=true", "-prec-div=false", "-prec-sqrt=false"],
+    "euler_tri_mixed.cu": [],
     "euler_tri_solver.cu": [],
     "line_f64.cu": ["--fmad=false"],
     "scalar_tri_f64.cu": ["--fmad=false"],
@@ -58,6 +60,13 @@ SOURCES = {
     "setup_device.cu": ["--fmad=false"],
     "halo.cu": [],
 }
+# file -> its objects, each with extra flags (one per polynomial order and volume
+# rule: an object takes up to a minute, all of them in one took seven)
+VARIANTS = {
+    "euler_tri_mixed_kernels.cu": {
+        f"p{p}r{r}": [f"-DWASL_P={p}", f"-DWASL_R={r}"]
+        for p, rules in ((3, (5, 4, 3, 0)), (2, (4, 3, 2, 0)), (1, (3, 2, 1, 0))) for r in rules},
+}
 HEADERS = [f for f in os.listdir(CSRC) if f.endswith((".hpp", ".cuh", ".h"))]
 
 
@@ -66,8 +75,8 @@ def _newest_header() -> float:
     return max(os.path.getmtime(p) for p in paths)
 
 
-def _compile(src: str, flags: list[str], build_dir: str = BUILD) -> str:
-    obj = os.path.join(build_dir, src + ".o")
+def _compile(src: str, flags: list[str], build_dir: str = BUILD, variant: str = "") -> str:
+    obj = os.path.join(build_dir, src + (f".{variant}" if variant else "") + ".o")
     path = os.path.join(CSRC, src)
     if (os.path.exists(obj) and os.path.getmtime(obj) >= os.path.getmtime(path)
             and os.path.getmtime(obj) >= _newest_header()):
@@ -86,7 +95,10 @@ def build(clean: bool = False, verbose: bool = False, checked: bool = False) -> 
         shutil.rmtree(build_dir)
     os.makedirs(build_dir, exist_ok=True)
     with cf.ThreadPoolExecutor(max_workers=os.cpu_count() or 4) as pool:
-        futures = [pool.submit(_compile, s, f + extra, build_dir) for s, f in SOURCES.items()]
+        variants = [(s, f + extra + more, v) for s, f in SOURCES.items()
+                    for v, more in VARIANTS.get(s, {"": []}).items()]
+        variants.sort(key=lambda x: not x[2])  # the long ones first
+        futures = [pool.submit(_compile, s, f, build_dir, v) for s, f, v in variants]
         objs = [f.result() for f in futures]
     if (not os.path.exists(lib) or
             max(os.path.getmtime(o) for o in objs) > os.path.getmtime(lib)):
