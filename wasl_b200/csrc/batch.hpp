@@ -55,10 +55,11 @@ private:
     TuneResult tuning;
     int highest_degree_begin = 0, check_points = 0;
     DeviceArray<double> u, e, s, geo, slot_geo, transforms, normal_x, normal_y, check, limited,
-        basis64, check_bound;
-    DeviceArray<std::int32_t> tile_nbr, tile_aux, neighbors, troubled, count, element_case, rough;
+        basis64;
+    DeviceArray<std::int32_t> tile_nbr, tile_aux, neighbors, troubled, count, element_case, rough, suspects;
     DeviceArray<std::uint8_t> tile_code, flags;
     DeviceArray<float> basis32;
+    PositivityFloors floors;
     DeviceArray<unsigned char> face_table, face_table64;
     std::array<DeviceArray<TileWork>, kTileShapeCount> work;
     std::array<std::int64_t, kTileShapeCount> work_count{};

@@ -216,16 +216,19 @@ BatchSolver::BatchSolver(const wasl_batch_config &cfg, std::int64_t case_count, 
       g->normal_x.upload(nx, stream_);
       g->normal_y.upload(ny, stream_);
       g->check.upload(first.check_basis, stream_);
-      g->check_bound.upload(positivity_check_bound(first.check_basis, M), stream_);
+      g->floors = positivity_floors(cfg.density_floor, cfg.pressure_floor, kMixedRelativeFloor,
+                                    first.check_basis, M);
+      if (cfg.positivity_all)
+        g->suspects.resize(ne);
       g->limited.resize(static_cast<std::size_t>(ne) * 4 * M);
       g->troubled.resize(ne);
-      g->count.resize(1);
+      g->count.resize(3); // troubled, rough and suspect elements
       g->flags.resize(ne);
     }
     for (auto *b : {&g->u, &g->e, &g->s})
       b->resize(static_cast<std::size_t>(4) * M * ne);
     if (cfg.limiting)
-      g->rough.resize(ne + 1); // rough list, then its count
+      g->rough.resize(ne);
     cuda_check(cudaMemsetAsync(g->u.get(), 0, g->u.size() * sizeof(double), stream_), "memset");
     // Work lists, one per tile size of the launch shapes.
     for (int shape = 0; shape < euler_tri_tile_shapes(); ++shape) {
@@ -336,7 +339,12 @@ StageArgs BatchSolver::stage_args(const Group &g, int stage) const {
   a.tile.aux = g.tile_aux.get();
   // FP64 face islands at discontinuities (the rough pass), with the limiter.
   a.rough = cfg_.limiting ? g.rough.get() : nullptr;
-  a.rough_count = a.rough ? g.rough.get() + g.ne : nullptr;
+  a.rough_count = a.rough ? g.count.get() + 1 : nullptr;
+  if (g.suspects.size() > 0) {
+    a.suspects = g.suspects.get();
+    a.suspect_count = g.count.get() + 2;
+    a.floors = g.floors;
+  }
   a.element_case = g.element_case.get();
   a.work = g.work[g.shape].get();
   a.work_count = g.work_count[g.shape];
@@ -371,15 +379,12 @@ LimitArgs BatchSolver::limit_args(const Group &g, double *state) const {
   l.check_basis = g.check.get();
   l.check_points = g.check_points;
   l.gamma = cfg_.heat_capacity_ratio;
-  l.density_floor = cfg_.density_floor;
-  l.pressure_floor = cfg_.pressure_floor;
   l.limited = g.limited.get();
   l.error = d_error_.get();
   l.positivity_all = cfg_.positivity_all ? 1 : 0;
   l.flags = g.flags.get();
-  l.relative_floor = kMixedRelativeFloor;
+  l.floors = g.floors;
   l.case_status = d_status_.get();
-  l.check_bound = g.check_bound.get();
   l.element_case = g.element_case.get();
   return l;
 }
@@ -405,6 +410,9 @@ void BatchSolver::tune() {
       g.shape = shapes[i];
       StageArgs a = stage_args(g, 0);
       a.sense = 0;
+      a.suspects = nullptr;
+      if (a.rough)
+        cuda_check(cudaMemsetAsync(a.rough_count, 0, sizeof(std::int32_t), stream_), "rough count");
       launch_euler_tri_stage_tile(g.p, g.rule, shapes[i], a, stream_);
     }, stream_);
     // By shape (0 for the shapes not timed).
@@ -429,13 +437,16 @@ void BatchSolver::enqueue_step(double cfl) {
     for (auto &gp : groups_) {
       Group &g = *gp;
       if (cfg_.limiting)
-        cuda_check(cudaMemsetAsync(g.count.get(), 0, sizeof(std::int32_t), stream_), "count");
+        cuda_check(cudaMemsetAsync(g.count.get(), 0, 3 * sizeof(std::int32_t), stream_), "count");
       const StageArgs a = stage_args(g, k);
       launch_euler_tri_stage_tile(g.p, g.rule, g.shape, a, stream_);
       launches_per_step_ += a.rough ? 2 : 1;
       if (cfg_.limiting) {
-        launch_limit_f64(g.M, 3, limit_args(g, a.out), stream_);
-        launches_per_step_ += cfg_.positivity_all ? 3 : 2;
+        LimitArgs l = limit_args(g, a.out);
+        l.suspects = a.suspects;
+        l.suspect_count = a.suspect_count;
+        launch_limit_f64(g.M, 3, l, stream_);
+        launches_per_step_ += 2;
       }
     }
 }

@@ -20,6 +20,7 @@
 #include "euler_device.cuh"
 #include "hllc_selected.cuh"
 #include "kernels.hpp"
+#include "positivity_device.cuh"
 #include "tri_tables.hpp"
 
 namespace wasl_b200 {
@@ -473,7 +474,7 @@ __device__ __forceinline__ void positivity_limit(const LimitArgs &a, double *lim
   const double inv_root2 = 1.0 / sqrt(2.0);
   const double pavg[4] = {lim[0] * inv_root2, lim[M] * inv_root2, lim[2 * M] * inv_root2,
                           lim[3 * M] * inv_root2};
-  if (!(pavg[0] > a.density_floor && primitive(a.gamma, pavg).p > a.pressure_floor)) {
+  if (!(pavg[0] > a.floors.density && primitive(a.gamma, pavg).p > a.floors.pressure)) {
     // (a NaN mean fails too) - recorded against its case when cases are tracked
     if (a.case_status)
       atomicCAS(a.case_status + a.element_case[e], 0, static_cast<int>(kBelowFloor));
@@ -484,10 +485,10 @@ __device__ __forceinline__ void positivity_limit(const LimitArgs &a, double *lim
   // Check-point floors: the absolute floors, raised to a fraction of the mean
   // density and energy when relative_floor > 0 (forms whose fluxes evaluate
   // point states in FP32, which resolves them only to ~1e-7 of the mean).
-  const double rf = a.relative_floor > 0.0 ? fmax(a.density_floor, a.relative_floor * pavg[0])
-                                           : a.density_floor;
-  const double pf = a.relative_floor > 0.0 ? fmax(a.pressure_floor, a.relative_floor * pavg[3])
-                                           : a.pressure_floor;
+  const double rf = a.floors.relative > 0.0 ? fmax(a.floors.density, a.floors.relative * pavg[0])
+                                           : a.floors.density;
+  const double pf = a.floors.relative > 0.0 ? fmax(a.floors.pressure, a.floors.relative * pavg[3])
+                                           : a.floors.pressure;
   double dscale = 1.0;
   for (int pt = 0; pt < a.check_points; ++pt) {
     const double *b = a.check_basis + pt * M;
@@ -530,48 +531,12 @@ __device__ __forceinline__ void positivity_limit(const LimitArgs &a, double *lim
       lim[v * M + m] *= pscale;
 }
 
-// Whether an element provably keeps density and pressure at or above the
-// check-point floors of positivity_limit at every check point, from bounds
-// on the point values: |sum_{m>=1} c_m phi_m| <= sum_{m>=1} |c_m| max|phi_m|
-// (max over the check points, check_bound), then the pressure's lower bound
-// from the bounds on density, momentum and energy.  Where it holds the limiter
-// would scale by exactly 1, so skipping it gives the same bits.  Small
-// margins cover the rounding of the point sums.
-template <int M> __device__ __forceinline__ bool positivity_clear(const LimitArgs &a,
-                                                                  const double *lim) {
-  const double inv_root2 = 1.0 / sqrt(2.0);
-  const double avg[4] = {lim[0] * inv_root2, lim[M] * inv_root2, lim[2 * M] * inv_root2,
-                         lim[3 * M] * inv_root2};
-  if (!(avg[0] > a.density_floor && primitive(a.gamma, avg).p > a.pressure_floor))
-    return false; // positivity_limit reports it
-  const double rf = a.relative_floor > 0.0 ? fmax(a.density_floor, a.relative_floor * avg[0])
-                                           : a.density_floor;
-  const double pf = a.relative_floor > 0.0 ? fmax(a.pressure_floor, a.relative_floor * avg[3])
-                                           : a.pressure_floor;
-  double b[4];
-#pragma unroll
-  for (int v = 0; v < 4; ++v) {
-    double sum = 0.0;
-#pragma unroll
-    for (int m = 1; m < M; ++m)
-      sum += fabs(lim[v * M + m]) * a.check_bound[m];
-    b[v] = sum;
-  }
-  const double rho_lo = avg[0] - b[0] - 1e-12 * (avg[0] + b[0]);
-  if (!(rho_lo >= rf))
-    return false;
-  const double mx = fabs(avg[1]) + b[1], my = fabs(avg[2]) + b[2];
-  const double energy_lo = avg[3] - b[3];
-  const double p_lo = (a.gamma - 1.0) * (energy_lo - 0.5 * (mx * mx + my * my) / rho_lo) -
-                      1e-12 * (a.gamma - 1.0) * (fabs(avg[3]) + b[3] + 0.5 * (mx * mx + my * my) / rho_lo);
-  return p_lo >= pf;
-}
-
 // The positivity limiter on every element the sensor did not flag (flags[e]
 // == 0), in place: the always-on positivity of the non-reference forms (the
 // reference limits positivity in troubled cells only,
 // cpp/src/limiting/euler_modal_limiter.cpp:81-96).  Elements that provably
-// need no scaling (positivity_clear) are skipped.
+// need no scaling (positivity_clear) are skipped.  For states no stage kernel
+// listed the suspects of (the initial one, the face-centric kernels').
 template <int M> __global__ void positivity_rest(const LimitArgs a) {
   for (std::int64_t e = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < a.ne;
        e += static_cast<std::int64_t>(gridDim.x) * blockDim.x) {
@@ -581,7 +546,16 @@ template <int M> __global__ void positivity_rest(const LimitArgs a) {
 #pragma unroll
     for (int i = 0; i < 4 * M; ++i)
       lim[i] = a.state[i * a.ne + e];
-    if (a.check_bound && positivity_clear<M>(a, lim))
+    double mode0[4], reach[4];
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      mode0[v] = lim[v * M];
+      reach[v] = 0.0;
+#pragma unroll
+      for (int m = 1; m < M; ++m)
+        reach[v] += fabs(lim[v * M + m]) * a.floors.bound[m];
+    }
+    if (positivity_clear(a.gamma, a.floors, mode0, reach))
       continue;
     positivity_limit<M>(a, lim, e);
 #pragma unroll
@@ -599,6 +573,78 @@ __device__ __forceinline__ double warp_min(double x) {
   return x;
 }
 
+// The positivity limiter (euler_positivity.hpp:63-102) on one element's modes
+// lim[4 M] in shared memory, one check point per lane; a mean below a floor
+// sets the error word (or the case's status) instead.
+template <int M>
+__device__ __forceinline__ void warp_positivity(const LimitArgs &a, double *lim, std::int64_t e,
+                                                int lane) {
+  constexpr int W = 4 * M;
+  const double inv_root2 = 1.0 / sqrt(2.0);
+  const double pavg[4] = {lim[0] * inv_root2, lim[M] * inv_root2,
+                          lim[2 * M] * inv_root2, lim[3 * M] * inv_root2};
+  if (!(pavg[0] > a.floors.density && primitive(a.gamma, pavg).p > a.floors.pressure)) {
+    if (lane == 0) {
+      if (a.case_status)
+        atomicCAS(a.case_status + a.element_case[e], 0, static_cast<int>(kBelowFloor));
+      else
+        raise_error(a.error, kBelowFloor, e);
+    }
+  } else {
+    const double rf = a.floors.relative > 0.0
+                          ? fmax(a.floors.density, a.floors.relative * pavg[0])
+                          : a.floors.density;
+    const double pf = a.floors.relative > 0.0
+                          ? fmax(a.floors.pressure, a.floors.relative * pavg[3])
+                          : a.floors.pressure;
+    double dscale = 1.0;
+    for (int pt = lane; pt < a.check_points; pt += 32) {
+      const double *b = a.check_basis + pt * M;
+      double rho = 0.0;
+      for (int m = 0; m < M; ++m)
+        rho += lim[m] * b[m];
+      if (rho < rf)
+        dscale = smin(dscale, (pavg[0] - rf) / (pavg[0] - rho));
+    }
+    dscale = warp_min(dscale);
+    __syncwarp();
+    for (int i = lane; i < W; i += 32)
+      if (i % M != 0)
+        lim[i] *= dscale;
+    __syncwarp();
+    double pscale = 1.0;
+    for (int pt = lane; pt < a.check_points; pt += 32) {
+      const double *b = a.check_basis + pt * M;
+      double st[4];
+      for (int v = 0; v < 4; ++v) {
+        double acc = 0.0;
+        for (int m = 0; m < M; ++m)
+          acc += lim[v * M + m] * b[m];
+        st[v] = acc;
+      }
+      if (primitive(a.gamma, st).p >= pf)
+        continue;
+      double lower = 0.0, upper = 1.0;
+      for (int it = 0; it < 64; ++it) {
+        const double middle = 0.5 * (lower + upper);
+        double x[4];
+        for (int v = 0; v < 4; ++v)
+          x[v] = pavg[v] + middle * (st[v] - pavg[v]);
+        if (primitive(a.gamma, x).p >= pf)
+          lower = middle;
+        else
+          upper = middle;
+      }
+      pscale = smin(pscale, lower);
+    }
+    pscale = warp_min(pscale);
+    __syncwarp();
+    for (int i = lane; i < W; i += 32)
+      if (i % M != 0)
+        lim[i] *= pscale;
+  }
+}
+
 // The stage limiter (cpp/src/limiting/euler_modal_limiter.cpp:70-98) with one
 // warp per troubled element of the compacted list: the lanes share out the
 // candidates (one output mode each), the characteristic projections (one mode
@@ -607,7 +653,7 @@ __device__ __forceinline__ double warp_min(double x) {
 // 64-step pressure bisections then run side by side instead of one after
 // another.  Every value is still one lane's serial sum in the reference's
 // order, so the result is the reference's bit for bit.  Limited modes go to
-// scratch by list position; scatter_limited writes them back.
+// scratch by list position; finish_limited writes them back.
 template <int M, int NB>
 __global__ void __launch_bounds__(128) limit_f64(const LimitArgs a) {
   constexpr int W = 4 * M;  // one element's values
@@ -725,70 +771,7 @@ __global__ void __launch_bounds__(128) limit_f64(const LimitArgs a) {
           cell.lim[v * M + m] = m == 0 ? cell.target[v * M] : back[4 * r + v];
     }
     __syncwarp();
-    // Positivity (euler_positivity.hpp:63-102), one check point per lane.
-    const double inv_root2 = 1.0 / sqrt(2.0);
-    const double pavg[4] = {cell.lim[0] * inv_root2, cell.lim[M] * inv_root2,
-                            cell.lim[2 * M] * inv_root2, cell.lim[3 * M] * inv_root2};
-    if (!(pavg[0] > a.density_floor && primitive(a.gamma, pavg).p > a.pressure_floor)) {
-      if (lane == 0) {
-        if (a.case_status)
-          atomicCAS(a.case_status + a.element_case[e], 0, static_cast<int>(kBelowFloor));
-        else
-          raise_error(a.error, kBelowFloor, e);
-      }
-    } else {
-      const double rf = a.relative_floor > 0.0
-                            ? fmax(a.density_floor, a.relative_floor * pavg[0])
-                            : a.density_floor;
-      const double pf = a.relative_floor > 0.0
-                            ? fmax(a.pressure_floor, a.relative_floor * pavg[3])
-                            : a.pressure_floor;
-      double dscale = 1.0;
-      for (int pt = lane; pt < a.check_points; pt += 32) {
-        const double *b = a.check_basis + pt * M;
-        double rho = 0.0;
-        for (int m = 0; m < M; ++m)
-          rho += cell.lim[m] * b[m];
-        if (rho < rf)
-          dscale = smin(dscale, (pavg[0] - rf) / (pavg[0] - rho));
-      }
-      dscale = warp_min(dscale);
-      __syncwarp();
-      for (int i = lane; i < W; i += 32)
-        if (i % M != 0)
-          cell.lim[i] *= dscale;
-      __syncwarp();
-      double pscale = 1.0;
-      for (int pt = lane; pt < a.check_points; pt += 32) {
-        const double *b = a.check_basis + pt * M;
-        double st[4];
-        for (int v = 0; v < 4; ++v) {
-          double acc = 0.0;
-          for (int m = 0; m < M; ++m)
-            acc += cell.lim[v * M + m] * b[m];
-          st[v] = acc;
-        }
-        if (primitive(a.gamma, st).p >= pf)
-          continue;
-        double lower = 0.0, upper = 1.0;
-        for (int it = 0; it < 64; ++it) {
-          const double middle = 0.5 * (lower + upper);
-          double x[4];
-          for (int v = 0; v < 4; ++v)
-            x[v] = pavg[v] + middle * (st[v] - pavg[v]);
-          if (primitive(a.gamma, x).p >= pf)
-            lower = middle;
-          else
-            upper = middle;
-        }
-        pscale = smin(pscale, lower);
-      }
-      pscale = warp_min(pscale);
-      __syncwarp();
-      for (int i = lane; i < W; i += 32)
-        if (i % M != 0)
-          cell.lim[i] *= pscale;
-    }
+    warp_positivity<M>(a, cell.lim, e, lane);
     __syncwarp();
     double *dst = a.limited + static_cast<std::int64_t>(k) * W;
     for (int i = lane; i < W; i += 32)
@@ -797,15 +780,35 @@ __global__ void __launch_bounds__(128) limit_f64(const LimitArgs a) {
   }
 }
 
-template <int M>
-__global__ void scatter_limited(double *state, std::int64_t ne, const std::int32_t *troubled,
-                                const std::int32_t *count, const double *limited) {
-  const int n = *count;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    const std::int64_t e = troubled[k];
-#pragma unroll
-    for (int i = 0; i < 4 * M; ++i)
-      state[i * ne + e] = limited[static_cast<std::int64_t>(k) * 4 * M + i];
+// The limiter's finish: the limited modes back into the state, and the
+// positivity limiter on the suspects (elements the stage kernel could not
+// prove to keep the floors) that were not limited, one warp each.  Testing in
+// the stage kernel, where the new modes are at hand, saves the pass over the
+// state that positivity_rest makes: 44 us of a 515 us stage at 500,000
+// triangles, P3.
+template <int M> __global__ void __launch_bounds__(128) finish_limited(const LimitArgs a) {
+  constexpr int W = 4 * M;
+  __shared__ double modes[4][W];
+  const std::int64_t ne = a.ne, total = static_cast<std::int64_t>(*a.troubled_count) * W;
+  const std::int64_t thread = static_cast<std::int64_t>(blockIdx.x) * 128 + threadIdx.x;
+  for (std::int64_t j = thread; j < total; j += static_cast<std::int64_t>(gridDim.x) * 128)
+    a.state[j % W * ne + a.troubled[j / W]] = a.limited[j];
+  if (!a.suspects)
+    return;
+  const int lane = threadIdx.x & 31, count = *a.suspect_count;
+  double *lim = modes[threadIdx.x >> 5];
+  for (int k = static_cast<int>(thread >> 5); k < count; k += static_cast<int>(gridDim.x) * 4) {
+    const std::int64_t e = a.suspects[k];
+    if (a.flags[e])
+      continue;
+    for (int i = lane; i < W; i += 32)
+      lim[i] = a.state[i * ne + e];
+    __syncwarp();
+    warp_positivity<M>(a, lim, e, lane);
+    __syncwarp();
+    for (int i = lane; i < W; i += 32)
+      a.state[i * ne + e] = lim[i];
+    __syncwarp();
   }
 }
 
@@ -1047,14 +1050,13 @@ void launch_euler_tri_stage_f64(int p, const StageArgs &a, cudaStream_t s) {
 void launch_limit_f64(int M, int NB, const LimitArgs &a, cudaStream_t s) {
   // Four warps (troubled elements) per block.
   const unsigned blocks = static_cast<unsigned>(std::min<std::int64_t>((a.ne + 3) / 4, 148 * 16));
-  const unsigned sblocks = static_cast<unsigned>(std::min<std::int64_t>((a.ne + 255) / 256, 148 * 8));
+  const unsigned sblocks = static_cast<unsigned>(std::min<std::int64_t>((a.ne + 3) / 4, 148 * 8));
   const unsigned pblocks = static_cast<unsigned>(std::min<std::int64_t>((a.ne + 127) / 128, 148 * 16));
 #define WASL_LIMIT(MM, NN)                                                                     \
   if (M == MM && NB == NN) {                                                                   \
     limit_f64<MM, NN><<<blocks, 128, 0, s>>>(a);                                               \
-    scatter_limited<MM><<<sblocks, 256, 0, s>>>(a.state, a.ne, a.troubled, a.troubled_count,   \
-                                                 a.limited);                                   \
-    if (a.positivity_all)                                                                      \
+    finish_limited<MM><<<sblocks, 128, 0, s>>>(a);                                             \
+    if (a.positivity_all && !a.suspects)                                                       \
       positivity_rest<MM><<<pblocks, 128, 0, s>>>(a);                                          \
     return;                                                                                    \
   }
@@ -1086,11 +1088,15 @@ void launch_sense_f64(int M, const SenseArgs &a, cudaStream_t s) {
   }
 }
 
-std::vector<double> positivity_check_bound(const std::vector<double> &check_basis, int M) {
-  std::vector<double> bound(M, 0.0);
+PositivityFloors positivity_floors(double density, double pressure, double relative,
+                                   const std::vector<double> &check_basis, int M) {
+  PositivityFloors f;
+  f.density = density;
+  f.pressure = pressure;
+  f.relative = relative;
   for (std::size_t i = 0; i < check_basis.size(); ++i)
-    bound[i % M] = std::max(bound[i % M], std::fabs(check_basis[i]));
-  return bound;
+    f.bound[i % M] = std::max(f.bound[i % M], std::fabs(check_basis[i]));
+  return f;
 }
 
 void launch_dt_from_speed(std::int64_t cases, unsigned long long *speed, double cfl,

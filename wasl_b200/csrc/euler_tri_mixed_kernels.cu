@@ -27,6 +27,7 @@
 
 #include "euler_device.cuh"
 #include "kernels.hpp"
+#include "positivity_device.cuh"
 #include "euler_tri_mixed.hpp"
 #include "tri_tables.hpp"
 
@@ -703,7 +704,7 @@ __device__ __forceinline__ void tile_finish(const StageArgs &a, std::int64_t e, 
   const double *__restrict__ geo = a.mesh.geo;
   const double inv = geo[4 * ne + e];
   const double dt = a.case_dt ? a.case_dt[case_id] : (a.dt ? *a.dt : a.dt_value);
-  double rho[M], avg[4];
+  double rho[M], avg[4], reach[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
   for (int v = 0; v < 4; ++v)
 #pragma unroll
@@ -723,6 +724,8 @@ __device__ __forceinline__ void tile_finish(const StageArgs &a, std::int64_t e, 
         rho[m] = o;
       if (m == 0)
         avg[v] = o;
+      else if (a.suspects)
+        reach[v] += fabs(o) * a.floors.bound[m];
     }
 
   if (a.speed_max) {
@@ -757,6 +760,8 @@ __device__ __forceinline__ void tile_finish(const StageArgs &a, std::int64_t e, 
     }
   }
 
+  if (a.suspects)
+    append_listed(!positivity_clear(a.gamma, a.floors, avg, reach), e, a.suspects, a.suspect_count);
   if (a.sense) {
     double total = 0.0, high = 0.0;
 #pragma unroll
@@ -1356,6 +1361,19 @@ __global__ void __launch_bounds__(kRoughThreads) euler_tri_rough(const StageArgs
                     static_cast<unsigned long long>(__double_as_longlong(speed)));
         else
           raise_error(a.error, kNonPhysicalAverage, e);
+      }
+      if (a.suspects) {
+        double mode0[4], reach[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          mode0[v] = E.next[v * M];
+          reach[v] = 0.0;
+#pragma unroll
+          for (int m = 1; m < M; ++m)
+            reach[v] += fabs(E.next[v * M + m]) * a.floors.bound[m];
+        }
+        if (!positivity_clear(gamma, a.floors, mode0, reach))
+          a.suspects[atomicAdd(a.suspect_count, 1)] = static_cast<std::int32_t>(e);
       }
       if (a.sense) {
         double total = 0.0, high = 0.0;
@@ -2209,7 +2227,7 @@ __device__ __forceinline__ void patch_outside_trace(const double *__restrict__ i
 // FP64 Shu-Osher combination (cpp/include/wasl/time/ssp_rk3.hpp:44-60) and the
 // optional next-step CFL speed and sensor (as tile_finish, with the stage
 // input read from global memory).
-template <int P>
+template <int P, bool LIMITED>
 __device__ __forceinline__ void patch_finish(const StageArgs &a, std::int64_t e, int case_id,
                                              const double (&r0)[4],
                                              const float (&racc)[4][TriShape<P>::M - 1]) {
@@ -2217,7 +2235,7 @@ __device__ __forceinline__ void patch_finish(const StageArgs &a, std::int64_t e,
   const std::int64_t ne = a.mesh.ne;
   const double inv = a.mesh.geo[4 * ne + e];
   const double dt = a.case_dt ? a.case_dt[case_id] : (a.dt ? *a.dt : a.dt_value);
-  double rho[M], avg[4];
+  double rho[M], avg[4], reach[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
   for (int v = 0; v < 4; ++v)
 #pragma unroll
@@ -2237,6 +2255,8 @@ __device__ __forceinline__ void patch_finish(const StageArgs &a, std::int64_t e,
         rho[m] = o;
       if (m == 0)
         avg[v] = o;
+      else if (LIMITED && a.suspects)
+        reach[v] += fabs(o) * a.floors.bound[m];
     }
   if (a.speed_max) {
     const double scale = 1.0 / sqrt(2.0);
@@ -2261,6 +2281,8 @@ __device__ __forceinline__ void patch_finish(const StageArgs &a, std::int64_t e,
       atomicMax(a.speed_max + case_id, best);
     }
   }
+  if (LIMITED && a.suspects)
+    append_listed(!positivity_clear(a.gamma, a.floors, avg, reach), e, a.suspects, a.suspect_count);
   if (a.sense) {
     double total = 0.0, high = 0.0;
 #pragma unroll
@@ -2741,7 +2763,7 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_patch(const StageArgs a)
       }
     }
   }
-  patch_finish<P>(a, e, case_id, r0, racc);
+  patch_finish<P, ISLANDS>(a, e, case_id, r0, racc);
 }
 
 void check(cudaError_t rc, const char *what) {
@@ -2880,8 +2902,6 @@ void stage_tile(const StageArgs &a, cudaStream_t s) {
   const std::int64_t blocks = a.work ? a.work_count : (a.mesh.ne + TILE - 1) / TILE;
   if (blocks <= 0)
     return;
-  if (a.rough)
-    check(cudaMemsetAsync(a.rough_count, 0, sizeof(std::int32_t), s), "rough count");
   if constexpr (SHARED)
     euler_tri_tile_shared<P, R, TILE, MINB>
         <<<static_cast<unsigned>(blocks), TILE, SharedFaceSmem<P, TILE>::bytes, s>>>(a);
@@ -2923,8 +2943,6 @@ void stage_tile_persistent(const StageArgs &a, cudaStream_t s) {
   const std::int64_t tiles = a.work ? a.work_count : (a.mesh.ne + TILE - 1) / TILE;
   if (tiles <= 0)
     return;
-  if (a.rough)
-    check(cudaMemsetAsync(a.rough_count, 0, sizeof(std::int32_t), s), "rough count");
   const std::int64_t blocks = tiles < resident ? tiles : resident;
   euler_tri_tile_persistent<P, R, TILE, MINB>
       <<<static_cast<unsigned>(blocks), TILE, tile_smem<P, TILE>(), s>>>(a);

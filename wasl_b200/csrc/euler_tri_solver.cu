@@ -170,7 +170,7 @@ public:
                                              " transmissive or paired periodic boundaries");
       if (tile_ok_) {
         if (cfg.limiting)
-          d_rough_.resize(ne_ + 1); // rough list, then its count
+          d_rough_.resize(ne_);
         const TileSlotArrays ts = build_tile_slots(mesh_, t, boundary_, QF);
         d_tile_nbr_.upload(columns(ids(ts.nbr), 3), stream_);
         d_tile_code_.upload(columns(ts.code, 3), stream_);
@@ -229,7 +229,11 @@ public:
       d_normal_x_.upload(columns(stencil_.normal_x, 1), stream_);
       d_normal_y_.upload(columns(stencil_.normal_y, 1), stream_);
       d_check_.upload(stencil_.check_basis, stream_);
-      d_check_bound_.upload(positivity_check_bound(stencil_.check_basis, M_), stream_);
+      floors_ = positivity_floors(cfg.density_floor, cfg.pressure_floor,
+                                  cfg.precision == WASL_MIXED ? kMixedRelativeFloor : 0.0,
+                                  stencil_.check_basis, M_);
+      if (tile_ok_ && cfg.positivity_all)
+        d_suspects_.resize(ne_);
       d_limited_.resize(static_cast<std::size_t>(ne_) * 4 * M_);
       d_troubled_.resize(ne_);
     }
@@ -635,7 +639,7 @@ private:
     a.patch.geo = d_patch_geo_.get();
     // FP64 face islands at discontinuities (the rough pass), with the limiter.
     a.rough = limiting_ ? d_rough_.get() : nullptr;
-    a.rough_count = a.rough ? d_rough_.get() + ne_ : nullptr;
+    a.rough_count = a.rough ? d_count_.get() + 1 : nullptr;
     a.dt = dt_device;
     a.dt_value = dt_value;
     a.gamma = cfg_.heat_capacity_ratio;
@@ -647,6 +651,12 @@ private:
     a.troubled_count = d_count_.get();
     if (mixed_ && kernel_ < 0)
       tune_mixed(a);
+    // The tile and patch kernels list the elements for the always-on positivity.
+    if (limiting_ && d_suspects_.size() > 0 && kernel_ >= 1) {
+      a.suspects = d_suspects_.get();
+      a.suspect_count = d_count_.get() + 2;
+      a.floors = floors_;
+    }
     double *ins[3] = {d_u_.get(), d_e_.get(), d_s_.get()};
     double *outs[3] = {d_e_.get(), d_s_.get(), d_u_.get()};
     for (int k = 0; k < 3; ++k) {
@@ -655,8 +665,8 @@ private:
       a.u0 = d_u_.get();
       a.out = outs[k];
       a.flags = d_flags_.get() + k * ne_;
-      if (limiting_)
-        cuda_check(cudaMemsetAsync(d_count_.get(), 0, sizeof(std::int32_t), stream_), "count");
+      if (limiting_) // troubled, rough and suspect elements
+        cuda_check(cudaMemsetAsync(d_count_.get(), 0, 3 * sizeof(std::int32_t), stream_), "count");
       a.speed_max = fused_speed_ && k == 2 && kernel_ >= 1 ? d_speed_.get() : nullptr;
       a.error = d_error_.get();
       stage_begin();
@@ -690,8 +700,11 @@ private:
         count_launches(2);
       }
       if (limiting_) {
-        launch_limit_f64(M_, 3, limit_args(outs[k], d_flags_.get() + k * ne_), stream_);
-        count_launches(cfg_.positivity_all ? 3 : 2);
+        LimitArgs l = limit_args(outs[k], d_flags_.get() + k * ne_);
+        l.suspects = a.suspects;
+        l.suspect_count = a.suspect_count;
+        launch_limit_f64(M_, 3, l, stream_);
+        count_launches(cfg_.positivity_all && !a.suspects ? 3 : 2);
       }
     }
     cuda_check(cudaGetLastError(), "stage launch");
@@ -744,6 +757,8 @@ private:
         a.stage = k;
         a.in = ins[k];
         a.out = outs[k];
+        if (a.rough)
+          cuda_check(cudaMemsetAsync(a.rough_count, 0, sizeof(std::int32_t), stream_), "rough count");
         launch_mixed(a);
       }
     }, stream_);
@@ -788,8 +803,7 @@ private:
     LimitArgs l;
     l.positivity_all = cfg_.positivity_all ? 1 : 0;
     l.flags = flags;
-    l.relative_floor = mixed_ ? kMixedRelativeFloor : 0.0;
-    l.check_bound = d_check_bound_.get();
+    l.floors = floors_;
     l.ne = ne_;
     l.state = state;
     l.troubled = d_troubled_.get();
@@ -801,8 +815,6 @@ private:
     l.check_basis = d_check_.get();
     l.check_points = stencil_.check_point_count();
     l.gamma = cfg_.heat_capacity_ratio;
-    l.density_floor = cfg_.density_floor;
-    l.pressure_floor = cfg_.pressure_floor;
     l.limited = d_limited_.get();
     l.error = d_error_.get();
     return l;
@@ -847,7 +859,8 @@ private:
   TuneResult tuning_;
   DeviceArray<std::int32_t> d_tile_nbr_, d_tile_aux_, d_rough_;
   DeviceArray<float> d_mlp_; // learned indicator weights (empty: the reference sensor)
-  DeviceArray<double> d_check_bound_;
+  PositivityFloors floors_;
+  DeviceArray<std::int32_t> d_suspects_; // always-on positivity: not proven to keep the floors
   DeviceArray<unsigned long long> d_mlp_stats_;
   DeviceArray<unsigned char> d_mlp_records_; // per-element inference records
   double mlp_lo_ = 0.1, mlp_hi_ = 0.9;

@@ -99,6 +99,16 @@ struct TileWork {
 //   stage 2: out = (1/3) u0 + (2/3) (in + dt r)
 // (cpp/include/wasl/time/ssp_rk3.hpp:44-60).  With sense != 0 the kernel also
 // evaluates the modal-decay sensor on `out` and appends troubled elements.
+// What the positivity test needs: the floors, and per mode the largest |basis
+// value| over the check points.
+struct PositivityFloors {
+  double density = 1e-10, pressure = 1e-10;
+  // > 0: the check-point floors become max(floor, relative x mean density) and
+  // max(floor, relative x mean energy) (the mixed form).
+  double relative = 0.0;
+  double bound[10] = {};
+};
+
 struct StageArgs {
   TriMeshView mesh;
   BoundaryView boundary;
@@ -138,6 +148,12 @@ struct StageArgs {
   std::int32_t *rough = nullptr;
   std::int32_t *rough_count = nullptr;
   const std::int32_t *element_case = nullptr;
+  // Always-on positivity: elements of `out` not proven to keep the floors are
+  // appended to suspects [ne] (count suspect_count), for the limiter's finish;
+  // null: not tested.  The tile and patch kernels only.
+  std::int32_t *suspects = nullptr;
+  std::int32_t *suspect_count = nullptr;
+  PositivityFloors floors;
 };
 
 // Limiter over the compacted troubled list (cpp/src/limiting/euler_modal_limiter.cpp:70-98).
@@ -151,28 +167,27 @@ struct LimitArgs {
   const double *normal_x = nullptr, *normal_y = nullptr;
   const double *check_basis = nullptr;       // [points][M]
   int check_points = 0;
-  double gamma = 1.4, density_floor = 1e-10, pressure_floor = 1e-10;
+  double gamma = 1.4;
+  PositivityFloors floors;
   double *limited = nullptr;                 // [ne][4][M] scratch, by list position
   unsigned long long *error = nullptr;
   // Always-on positivity (not the reference's behaviour): after the troubled
   // cells, the positivity limiter also runs on every element with flags[e]
-  // == 0.  The launch then counts three kernels instead of two.
+  // == 0: on the suspects the stage kernel listed (not proven to keep the
+  // floors), or, without a list, on all of them (a third kernel).
   int positivity_all = 0;
+  const std::int32_t *suspects = nullptr;
+  const std::int32_t *suspect_count = nullptr;
   const std::uint8_t *flags = nullptr;
-  // > 0: the check-point floors become max(floor, relative_floor x mean
-  // density) and max(floor, relative_floor x mean energy) (the mixed form).
-  double relative_floor = 0.0;
   // Batched solves: a mean below a floor is recorded as case_status[case of
   // e] (first error only) instead of in the error word.
   int *case_status = nullptr;
   const std::int32_t *element_case = nullptr;
-  // [M] largest |basis value| of each mode over the check points: lets the
-  // always-on pass skip elements whose bounds clear the floors (null: none).
-  const double *check_bound = nullptr;
 };
 
-// check_bound[m] = max over points |check_basis[point][m]| (host).
-std::vector<double> positivity_check_bound(const std::vector<double> &check_basis, int M);
+// The floors with bound[m] = max over the points of |check_basis[point][m]| (host).
+PositivityFloors positivity_floors(double density, double pressure, double relative,
+                                   const std::vector<double> &check_basis, int M);
 
 // The mixed form's positivity check-point floors relative to the mean: FP32
 // resolves a point state to ~6e-8 of the mean, so point densities and

@@ -398,8 +398,8 @@ private:
     l.check_basis = d_check_.get();
     l.check_points = stencil_.check_point_count();
     l.gamma = cfg_.heat_capacity_ratio;
-    l.density_floor = cfg_.density_floor;
-    l.pressure_floor = cfg_.pressure_floor;
+    l.floors.density = cfg_.density_floor;
+    l.floors.pressure = cfg_.pressure_floor;
     l.limited = d_limited_.get();
     l.error = d_error_.get();
     return l;
