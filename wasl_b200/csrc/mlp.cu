@@ -648,45 +648,57 @@ __device__ __forceinline__ bool indicator_row(const MlpIndicatorArgs &a, std::in
 }
 
 // The decision for element e from its logit: troubled when sigmoid(logit) >=
-// hi, smooth when <= lo, else the reference decision; the flag, the
-// compacted troubled list (one atomic per warp) and the CTA's counters.
+// hi, smooth when <= lo, else the reference decision; the flag and the
+// compacted troubled list (one atomic per warp).  Every lane of the warp
+// calls it, `active` or not, and keeps the warp's counts in its registers
+// (counters in shared memory, added to per element, serialised the warp's 32
+// lanes up to three times over).
+struct IndicatorCounts {
+  unsigned n[6] = {};
+};
+
 __device__ __forceinline__ void indicator_decide(const MlpIndicatorArgs &a, std::int64_t e,
-                                                 float logit, bool reference,
-                                                 unsigned long long *counts, int lane) {
+                                                 bool active, float logit, bool reference,
+                                                 IndicatorCounts &counts, int lane) {
   const float p = 1.0f / (1.0f + expf(-logit));
-  bool troubled;
-  int kind;
-  if (p >= a.hi) {
-    troubled = true;
-    kind = 0;
-  } else if (p <= a.lo) {
-    troubled = false;
-    kind = 1;
-  } else {
-    troubled = reference;
-    kind = 2;
+  const bool high = p >= a.hi, low = !high && p <= a.lo;
+  const bool troubled = active && (high || (!low && reference));
+  reference = reference && active;
+  if (active) {
+    if (a.logits)
+      a.logits[e] = logit;
+    a.flags[e] = troubled ? 1 : 0;
   }
-  if (a.logits)
-    a.logits[e] = logit;
-  a.flags[e] = troubled ? 1 : 0;
-  atomicAdd(&counts[kind], 1ULL);
-  if (reference)
-    atomicAdd(&counts[3], 1ULL);
-  if (reference && !troubled)
-    atomicAdd(&counts[4], 1ULL);
-  if (!reference && troubled)
-    atomicAdd(&counts[5], 1ULL);
-  const unsigned mask = __activemask();
-  const unsigned ballot = __ballot_sync(mask, troubled);
+  const unsigned all = 0xffffffffu;
+  const unsigned ballot = __ballot_sync(all, troubled);
+  counts.n[0] += __popc(__ballot_sync(all, active && high));
+  counts.n[1] += __popc(__ballot_sync(all, active && low));
+  counts.n[2] += __popc(__ballot_sync(all, active && !high && !low));
+  counts.n[3] += __popc(__ballot_sync(all, reference));
+  counts.n[4] += __popc(__ballot_sync(all, reference && !troubled));
+  counts.n[5] += __popc(__ballot_sync(all, troubled && !reference));
   if (ballot) {
-    const int leader = __ffs(ballot) - 1;
     int base = 0;
-    if (lane == leader)
+    if (lane == 0)
       base = atomicAdd(a.troubled_count, __popc(ballot));
-    base = __shfl_sync(mask, base, leader);
+    base = __shfl_sync(all, base, 0);
     if (troubled)
       a.troubled[base + __popc(ballot & ((1u << lane) - 1u))] = static_cast<std::int32_t>(e);
   }
+}
+
+// The warps' counts to the CTA's, then to the handle's (all threads; counts
+// in shared memory, zero before).
+__device__ __forceinline__ void indicator_count(const MlpIndicatorArgs &a,
+                                                const IndicatorCounts &warp,
+                                                unsigned long long *counts, int t) {
+  if ((t & 31) == 0)
+    for (int k = 0; k < 6; ++k)
+      if (warp.n[k])
+        atomicAdd(&counts[k], static_cast<unsigned long long>(warp.n[k]));
+  __syncthreads();
+  if (t < 6 && a.stats && counts[t])
+    atomicAdd(a.stats + t, counts[t]);
 }
 
 // A persistent kernel: each CTA of 128 threads loads the network once (BF16
@@ -724,6 +736,7 @@ __global__ void __launch_bounds__(128) mlp_indicator_kernel(const MlpIndicatorAr
     counts[t] = 0;
   const float b3 = P[a.shape.b3];
   const int warp = t >> 5, lane = t & 31, g = lane >> 2, q = lane & 3;
+  IndicatorCounts tally;
   const std::int64_t tiles = (a.ne + 127) / 128;
   for (std::int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const std::int64_t e = tile * 128 + t;
@@ -804,14 +817,11 @@ __global__ void __launch_bounds__(128) mlp_indicator_kernel(const MlpIndicatorAr
     }
     __syncthreads(); // logits written; the next tile's rows may overwrite X
 
-    if (active)
-      indicator_decide(a, e, logit[t], reference, counts, lane);
+    indicator_decide(a, e, active, logit[t], reference, tally, lane);
     // The logits of this tile are read above before the next tile's MMAs
     // write them: those come after the next tile's first barrier.
   }
-  __syncthreads();
-  if (t < 6 && a.stats && counts[t])
-    atomicAdd(a.stats + t, counts[t]);
+  indicator_count(a, tally, counts, t);
 }
 
 // The inference on the fifth-generation tensor cores: the persistent kernel's
@@ -877,6 +887,7 @@ __global__ void __launch_bounds__(128) mlp_indicator_tc_kernel(const MlpIndicato
   const unsigned w2_addr = static_cast<unsigned>(__cvta_generic_to_shared(W2));
   const float b3 = P[a.shape.b3];
   constexpr long long kWaitCycles = 1LL << 31;
+  IndicatorCounts tally;
   const std::int64_t tiles = (a.ne + 127) / 128;
   for (std::int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const std::int64_t e = tile * 128 + t;
@@ -938,8 +949,7 @@ __global__ void __launch_bounds__(128) mlp_indicator_tc_kernel(const MlpIndicato
 #pragma unroll
     for (int c = 0; c < Hd; ++c)
       z = fmaf(w3[c], fmaxf(v[c] + b2[c], 0.0f), z);
-    if (active)
-      indicator_decide(a, e, z + b3, reference, counts, lane);
+    indicator_decide(a, e, active, z + b3, reference, tally, lane);
   }
   __syncthreads();
   if (failed && t == 0) {
@@ -953,8 +963,7 @@ __global__ void __launch_bounds__(128) mlp_indicator_tc_kernel(const MlpIndicato
     tmem_fence_after_sync();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 64;" ::"r"(tmem) : "memory");
   }
-  if (t < 6 && a.stats && counts[t])
-    atomicAdd(a.stats + t, counts[t]);
+  indicator_count(a, tally, counts, t);
 }
 
 // ---- host launchers -------------------------------------------------------------
