@@ -48,6 +48,8 @@ private:
   struct Group {
     Group();
     ~Group();
+    cudaStream_t stream = nullptr; // groups after the first: a step's work beside the first's
+    cudaEvent_t done = nullptr;
     int p = 0, M = 0, rule = 0;
     std::int64_t ne = 0;
     std::vector<std::int64_t> cases;
@@ -56,7 +58,8 @@ private:
     int highest_degree_begin = 0, check_points = 0;
     DeviceArray<double> u, e, s, geo, slot_geo, transforms, normal_x, normal_y, check, limited,
         basis64;
-    DeviceArray<std::int32_t> tile_nbr, tile_aux, neighbors, troubled, count, element_case, rough, suspects;
+    DeviceArray<std::int32_t> tile_nbr, tile_aux, neighbors, troubled, count, element_case, rough,
+        suspects;
     DeviceArray<std::uint8_t> tile_code, flags;
     DeviceArray<float> basis32;
     PositivityFloors floors;
@@ -71,11 +74,16 @@ private:
   LimitArgs limit_args(const Group &g, double *state) const;
   void tune();
   void enqueue_step(double cfl);
+  // The groups' streams wait for the handle's, and the handle's for them.
+  void fork();
+  void join();
+  cudaStream_t group_stream(const Group &g) const { return g.stream ? g.stream : stream_; }
   void check_error();
 
   wasl_batch_config cfg_;
   std::int64_t cases_ = 0;
   cudaStream_t stream_ = nullptr;
+  cudaEvent_t forked_ = nullptr;
   std::vector<std::unique_ptr<Group>> groups_;
   std::vector<int> case_group_;
   std::vector<std::int64_t> case_offset_;
