@@ -59,17 +59,39 @@ __device__ __forceinline__ double modal_sum_global(const double *__restrict__ u,
   return value;
 }
 
+// One stage, one thread per element.  Bound by the FP64 pipe (every product and
+// sum is its own instruction) and the loads' latency.  Only what the upwind flux
+// uses is evaluated: one trace per face, of the upwind element (the element
+// itself, whose coefficients are in L1, or the one across), instead of both;
+// gradient terms that are zero by construction are not summed (mode 0's, and the
+// xi-derivative of the modes with i = 0), and the gradients' factor 0.5 is taken
+// into the map's columns (exact).  About 900 FP64 operations per element at P2
+// instead of 1,270; four steps at 518,162 elements 834 -> 599 us.
+//
+// Resident blocks per SM the registers are sized for (without a bound the
+// tables' constants are kept in registers).  Measured, four steps: P1 (5,000
+// elements) 87 us without, 93 at 8; P2 (518,162) 599 us (5: 678, 7: 608, 10: 684,
+// none: 919); P3 (80,000) 309 us (6: 337, 8: 401, none: 390).
+template <int P> constexpr int kScalarBlocks = P <= 1 ? 1 : P == 2 ? 8 : 5;
+
 template <int P>
-__global__ void __launch_bounds__(128) scalar_tri_stage_f64(const StageArgs a) {
+__global__ void __launch_bounds__(128, kScalarBlocks<P>) scalar_tri_stage_f64(const StageArgs a) {
   using S = TriShape<P>;
   constexpr int M = S::M, QF = S::QF, QV = ScalarTriVolume<P>::QV;
+  __shared__ FaceTable<P, double> F;
+  {
+    const double *src = static_cast<const double *>(a.face_table);
+    double *dst = reinterpret_cast<double *>(&F);
+    for (int i = threadIdx.x; i < static_cast<int>(sizeof(F) / sizeof(double)); i += 128)
+      dst[i] = src[i];
+  }
+  __syncthreads();
   const std::int64_t ne = a.mesh.ne;
   const std::int64_t e = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (e >= ne)
     return;
   const double *__restrict__ in = a.in;
   const ScalarTriVolume<P> &T = svol<P>();
-  const FaceTable<P, double> *__restrict__ F = static_cast<const FaceTable<P, double> *>(a.face_table);
   const double vx = a.velocity_x, vy = a.velocity_y;
 
   double c[M], r[M];
@@ -79,26 +101,53 @@ __global__ void __launch_bounds__(128) scalar_tri_stage_f64(const StageArgs a) {
     r[m] = 0.0;
   }
   const double *__restrict__ geo = a.mesh.geo;
-  const double ax = geo[e], ay = geo[ne + e], bx = geo[2 * ne + e], by = geo[3 * ne + e];
-
-#pragma unroll 1
-  for (int q = 0; q < QV; ++q) {
-    const double state = modal_sum<M>(c, T.phi[q]);
-    const double ws = T.w[q] * state;
-#pragma unroll
-    for (int m = 0; m < M; ++m) {
-      const double gx = 0.5 * (by * T.dxi[q][m] - ay * T.deta[q][m]);
-      const double gy = 0.5 * (-bx * T.dxi[q][m] + ax * T.deta[q][m]);
-      r[m] += ws * (vx * gx + vy * gy);
-    }
-  }
-
   // u^n (read by the combination at the end of stages 2 and 3) into L1 while
-  // the faces run.
+  // the element is computed.
   if (a.stage > 0) {
 #pragma unroll
     for (int m = 0; m < M; ++m)
       asm volatile("prefetch.global.L1 [%0];\n" ::"l"(a.u0 + static_cast<std::int64_t>(m) * ne + e));
+  }
+
+  if constexpr (M > 1) {
+    const double hax = 0.5 * geo[e], nhay = -0.5 * geo[ne + e], nhbx = -0.5 * geo[2 * ne + e],
+                 hby = 0.5 * geo[3 * ne + e];
+#pragma unroll 1
+    for (int q = 0; q < QV; ++q) {
+      double state = c[0] * T.phi[q][0];
+#pragma unroll
+      for (int m = 1; m < M; ++m)
+        state += c[m] * T.phi[q][m];
+      const double ws = T.w[q] * state;
+#pragma unroll
+      for (int n = 1; n <= P; ++n)
+#pragma unroll
+        for (int i = 0; i <= n; ++i) {
+          const int m = n * (n + 1) / 2 + i;
+          const double geta = T.deta[q][m];
+          double gx, gy;
+          if (i == 0) {
+            gx = nhay * geta;
+            gy = hax * geta;
+          } else {
+            const double gxi = T.dxi[q][m];
+            gx = hby * gxi + nhay * geta;
+            gy = nhbx * gxi + hax * geta;
+          }
+          r[m] += ws * (vx * gx + vy * gy);
+        }
+    }
+    // Mode 0's terms are zero, or NaN where the state is not finite (which mode
+    // 1's sum then is not either).
+    r[0] = 0.0 + 0.0 * r[1];
+  } else {
+    const double ax = geo[e], ay = geo[ne + e], bx = geo[2 * ne + e], by = geo[3 * ne + e];
+#pragma unroll
+    for (int q = 0; q < QV; ++q) {
+      const double gx = 0.5 * (by * T.dxi[q][0] - ay * T.deta[q][0]);
+      const double gy = 0.5 * (-bx * T.dxi[q][0] + ax * T.deta[q][0]);
+      r[0] += T.w[q] * (c[0] * T.phi[q][0]) * (vx * gx + vy * gy);
+    }
   }
 
 #pragma unroll 1
@@ -110,52 +159,38 @@ __global__ void __launch_bounds__(128) scalar_tri_stage_f64(const StageArgs a) {
     const double scale = a.mesh.slot_geo[(3 * k + 2) * ne + e];
     const bool self_left = code & 1u;
     const int le = (code >> 1) & 3u, re = (code >> 3) & 3u, flip = (code >> 5) & 1u;
-    const double(*lb)[M] = F->lb[le];
-    const double(*rb)[M] = F->rb[(le * 3 + re) * 2 + flip];
+    const double(*lb)[M] = F.lb[le];
+    const double(*rb)[M] = F.rb[(le * 3 + re) * 2 + flip];
+    const double(*own_basis)[M] = self_left ? lb : rb;
     const double normal_speed = vx * nx + vy * ny;
-    // The neighbour's trace at every point of the face from one load of each
-    // of its coefficients (each sum over the modes 0..M-1 from 0.0, as
-    // modal_sum_global).
-    double outside[QF];
-    if (nb >= 0) {
-      const double(*ob)[M] = self_left ? rb : lb;
-#pragma unroll
-      for (int q = 0; q < QF; ++q)
-        outside[q] = 0.0;
+    // The upwind element's trace at every point of the face, each of its
+    // coefficients loaded once (each sum over the modes 0..M-1).
+    const bool from_left = normal_speed >= 0.0, from_self = from_left == self_left;
+    double upwind[QF];
+    if (from_self || nb >= 0) {
+      const std::int64_t source = from_self ? e : nb;
+      const double(*basis)[M] = from_left ? lb : rb;
 #pragma unroll
       for (int m = 0; m < M; ++m) {
-        const double x = in[static_cast<std::int64_t>(m) * ne + nb];
+        const double x = in[static_cast<std::int64_t>(m) * ne + source];
 #pragma unroll
         for (int q = 0; q < QF; ++q)
-          outside[q] += x * ob[q][m];
+          upwind[q] = m == 0 ? x * basis[q][0] : upwind[q] + x * basis[q][m];
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < QF; ++q) {
+        const std::int64_t point = static_cast<std::int64_t>(-nb - 1) * QF + q;
+        upwind[q] = modal_sum_global<M>(in, ne, a.mesh.donor[point], a.mesh.donor_basis + point * M);
       }
     }
 #pragma unroll
     for (int q = 0; q < QF; ++q) {
-      double ls, rs;
-      if (self_left) {
-        ls = modal_sum<M>(c, lb[q]);
-        if (nb >= 0) {
-          rs = outside[q];
-        } else {
-          const std::int64_t point = static_cast<std::int64_t>(-nb - 1) * QF + q;
-          rs = modal_sum_global<M>(in, ne, a.mesh.donor[point], a.mesh.donor_basis + point * M);
-        }
-      } else {
-        ls = outside[q];
-        rs = modal_sum<M>(c, rb[q]);
-      }
-      const double flux = normal_speed * (normal_speed >= 0.0 ? ls : rs);
-      const double weight = F->ew[le][q] * scale;
-      if (self_left) {
+      const double flux = normal_speed * upwind[q];
+      const double weight = self_left ? -(F.ew[le][q] * scale) : F.ew[le][q] * scale;
 #pragma unroll
-        for (int m = 0; m < M; ++m)
-          r[m] -= weight * lb[q][m] * flux;
-      } else {
-#pragma unroll
-        for (int m = 0; m < M; ++m)
-          r[m] += weight * rb[q][m] * flux;
-      }
+      for (int m = 0; m < M; ++m)
+        r[m] += weight * own_basis[q][m] * flux;
     }
   }
 
