@@ -378,10 +378,13 @@ int wasl_gpu_run(wasl_gpu *h, double cfl, double start_time, double end_time, ui
       const double dt = std::min(stable > 0.0 ? stable : remaining, remaining);
       if (dt <= 0.0 || t + dt == t)
         throw std::runtime_error("simulation: timestep cannot advance time");
-      h->solver->step(dt);
+      // (A device error of this step is reported by the next stable_dt, which
+      // waits for the device anyway, or below: one wait per step.)
+      h->solver->enqueue(dt);
       t += dt;
       ++n;
     }
+    h->solver->check();
     if (steps)
       *steps = n;
     if (time)

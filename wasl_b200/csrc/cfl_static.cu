@@ -107,9 +107,11 @@ extern "C" int wasl_cfl_dt_static(const double *state, int64_t element_count, in
   a.result = scratch;
   a.dt = nullptr; // the host forms dt, as the handles do
   a.error = scratch + kCflResultWords;
-  // The error word must start at zero; launch_cfl clears its own counters
-  // and the pairs are fully overwritten.
+  // The error word and the block counter must start at zero (calls that raced
+  // may have left them otherwise); the rest is fully overwritten.
   rc = cudaMemsetAsync(a.error, 0, sizeof(unsigned long long), s);
+  if (rc == cudaSuccess)
+    rc = cudaMemsetAsync(scratch, 0, 16 * sizeof(unsigned long long), s);
   if (rc == cudaSuccess) {
     try {
       launch_cfl(a, s);

@@ -137,13 +137,11 @@ __global__ void __launch_bounds__(128, kStageBlocks<P>) euler_tri_stage_f64(cons
   const std::int64_t rows = static_cast<std::int64_t>(2 * half) * M * ne;
   const double *__restrict__ in = a.in + rows;
 
-  double c[2][M], r[2][M];
-#pragma unroll
-  for (int v = 0; v < 2; ++v)
-#pragma unroll
-    for (int m = 0; m < M; ++m)
-      c[v][m] = in[(static_cast<std::int64_t>(v) * M + m) * ne + e];
-  const double *__restrict__ geo = a.mesh.geo;
+  // Launched as a programmatic dependent of the launch before it, the block may
+  // be here while that one drains: the face table is constant, and the state is
+  // not touched before that launch has completed.  (Launched plainly, both
+  // instructions are no-ops.)
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   {
     const double *src = static_cast<const double *>(a.face_table);
     double *dst = reinterpret_cast<double *>(&B.table);
@@ -152,7 +150,16 @@ __global__ void __launch_bounds__(128, kStageBlocks<P>) euler_tri_stage_f64(cons
   }
   if (threadIdx.x == 0)
     B.count = 0;
-  __syncthreads();
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+
+  double c[2][M], r[2][M];
+#pragma unroll
+  for (int v = 0; v < 2; ++v)
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+      c[v][m] = in[(static_cast<std::int64_t>(v) * M + m) * ne + e];
+  const double *__restrict__ geo = a.mesh.geo;
+  __syncthreads(); // the table and the counter
 
   // A. Traces at the face points, in the face's point order.
 #pragma unroll 1
@@ -666,6 +673,8 @@ __global__ void __launch_bounds__(128) limit_f64(const LimitArgs a) {
   __shared__ Cell cells[WARPS];
   Cell &cell = cells[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
   const int count = *a.troubled_count;
   const std::int64_t ne = a.ne;
   const double *u = a.state;
@@ -789,6 +798,8 @@ __global__ void __launch_bounds__(128) limit_f64(const LimitArgs a) {
 template <int M> __global__ void __launch_bounds__(128) finish_limited(const LimitArgs a) {
   constexpr int W = 4 * M;
   __shared__ double modes[4][W];
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
   const std::int64_t ne = a.ne, total = static_cast<std::int64_t>(*a.troubled_count) * W;
   const std::int64_t thread = static_cast<std::int64_t>(blockIdx.x) * 128 + threadIdx.x;
   for (std::int64_t j = thread; j < total; j += static_cast<std::int64_t>(gridDim.x) * 128)
@@ -910,8 +921,9 @@ __device__ __forceinline__ void block_pair(unsigned long long &best, long long &
 // The whole CFL reduction in one pass over the cell averages: each block
 // reduces its elements to (largest speed, smallest element reaching it) and
 // stores the pair; the last block to finish reduces the pairs, records the
-// winner's mode-0 coefficients and forms dt (cfl_timestep.cpp:70-84), then
-// re-arms the block counter.
+// winner's mode-0 coefficients and forms dt (cfl_timestep.cpp:70-84), copies the
+// error word beside them (one read brings the host everything), then re-arms
+// the block counter (zero before the first launch).
 __global__ void __launch_bounds__(256) cfl_reduce(const CflArgs a) {
   unsigned long long best = 0;
   long long arg = LLONG_MAX;
@@ -957,6 +969,7 @@ __global__ void __launch_bounds__(256) cfl_reduce(const CflArgs a) {
       a.result[2 + v] = static_cast<unsigned long long>(__double_as_longlong(a.state[v * plane + e]));
     const double dt = speed > 0.0 ? a.cfl * a.length / (speed * (2 * a.p + 1)) : 0.0;
     a.result[6] = static_cast<unsigned long long>(__double_as_longlong(dt));
+    a.result[7] = __ldcg(a.error); // (every block's, and any earlier kernel's)
     if (a.dt)
       *a.dt = dt;
     a.result[8] = 0;
@@ -997,6 +1010,24 @@ void check(cudaError_t rc, const char *what) {
     throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(rc));
 }
 
+// Launches a kernel, as a programmatic dependent of the launch before it on the
+// stream if asked to (the kernel waits before it touches what that one writes).
+template <typename... P, typename... A>
+void launch_kernel(bool dependent, void (*kernel)(P...), unsigned blocks, unsigned threads,
+                   std::size_t smem, cudaStream_t s, const A &...args) {
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(blocks);
+  config.blockDim = dim3(threads);
+  config.dynamicSmemBytes = smem;
+  config.stream = s;
+  cudaLaunchAttribute attribute[1];
+  attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute[0].val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = attribute;
+  config.numAttrs = dependent ? 1 : 0;
+  check(cudaLaunchKernelEx(&config, kernel, args...), "kernel launch");
+}
+
 template <int P> void upload_volume(const void *symbol) {
   static VolumeTable<P, double> table;
   fill_volume_table<P, double>(table);
@@ -1020,7 +1051,7 @@ template <int P> void stage(const StageArgs &a, cudaStream_t s) {
   }
   constexpr int E = StageBlock<P>::E;
   const unsigned blocks = static_cast<unsigned>((a.mesh.ne + E - 1) / E);
-  euler_tri_stage_f64<P><<<blocks, 128, bytes, s>>>(a);
+  launch_kernel(true, euler_tri_stage_f64<P>, blocks, 128, bytes, s, a);
 }
 
 } // namespace
@@ -1054,8 +1085,8 @@ void launch_limit_f64(int M, int NB, const LimitArgs &a, cudaStream_t s) {
   const unsigned pblocks = static_cast<unsigned>(std::min<std::int64_t>((a.ne + 127) / 128, 148 * 16));
 #define WASL_LIMIT(MM, NN)                                                                     \
   if (M == MM && NB == NN) {                                                                   \
-    limit_f64<MM, NN><<<blocks, 128, 0, s>>>(a);                                               \
-    finish_limited<MM><<<sblocks, 128, 0, s>>>(a);                                             \
+    launch_kernel(a.dependent != 0, limit_f64<MM, NN>, blocks, 128, 0, s, a);                  \
+    launch_kernel(a.dependent != 0, finish_limited<MM>, sblocks, 128, 0, s, a);                \
     if (a.positivity_all && !a.suspects)                                                       \
       positivity_rest<MM><<<pblocks, 128, 0, s>>>(a);                                          \
     return;                                                                                    \
@@ -1103,23 +1134,8 @@ void launch_dt_from_speed(std::int64_t cases, unsigned long long *speed, double 
                           const double *length, const int *p, double length_all, int p_all,
                           double *dt, double *elapsed, const int *status, cudaStream_t s,
                           bool dependent) {
-  if (!dependent) {
-    dt_from_speed<<<static_cast<unsigned>((cases + 255) / 256), 256, 0, s>>>(
-        cases, speed, cfl, length, p, length_all, p_all, dt, elapsed, status);
-    return;
-  }
-  cudaLaunchConfig_t config = {};
-  config.gridDim = dim3(static_cast<unsigned>((cases + 255) / 256));
-  config.blockDim = dim3(256);
-  config.stream = s;
-  cudaLaunchAttribute attribute[1];
-  attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attribute[0].val.programmaticStreamSerializationAllowed = 1;
-  config.attrs = attribute;
-  config.numAttrs = 1;
-  check(cudaLaunchKernelEx(&config, dt_from_speed, cases, speed, cfl, length, p, length_all, p_all,
-                           dt, elapsed, status),
-        "dt launch");
+  launch_kernel(dependent, dt_from_speed, static_cast<unsigned>((cases + 255) / 256), 256, 0, s,
+                cases, speed, cfl, length, p, length_all, p_all, dt, elapsed, status);
 }
 
 void launch_cfl_speed(const CflArgs &a, cudaStream_t s) {
@@ -1129,7 +1145,6 @@ void launch_cfl_speed(const CflArgs &a, cudaStream_t s) {
 }
 
 void launch_cfl(const CflArgs &a, cudaStream_t s) {
-  check(cudaMemsetAsync(a.result, 0, 16 * sizeof(unsigned long long), s), "cfl reset");
   const unsigned blocks =
       static_cast<unsigned>(std::min<std::int64_t>((a.ne + 255) / 256, kCflBlocks));
   cfl_reduce<<<blocks, 256, 0, s>>>(a);

@@ -240,13 +240,15 @@ public:
     setup_.lap(WASL_SETUP_STENCIL);
     d_flags_.resize(3 * ne_);
     cuda_check(cudaMemsetAsync(d_flags_.get(), 0, 3 * ne_, stream_), "memset");
-    d_count_.resize(4);
+    d_count_.resize(12); // per stage: troubled, rough and suspect elements
     for (auto *b : {&d_u_, &d_e_, &d_s_})
       b->resize(static_cast<std::size_t>(4) * M_ * ne_);
     cuda_check(cudaMemsetAsync(d_u_.get(), 0, d_u_.size() * sizeof(double), stream_), "memset");
     d_error_.resize(1);
     d_speed_.resize(1);
     d_cfl_.resize(kCflResultWords);
+    cuda_check(cudaMemsetAsync(d_cfl_.get(), 0, kCflResultWords * sizeof(unsigned long long), stream_),
+               "memset");
     d_dt_.resize(1);
     cuda_check(cudaMemsetAsync(d_error_.get(), 0, sizeof(unsigned long long), stream_), "memset");
     length_ = minimum_altitude(mesh_);
@@ -394,11 +396,8 @@ public:
     cuda_check(cudaMemcpyAsync(scratch_.words, d_cfl_.get(), 8 * sizeof(unsigned long long),
                                cudaMemcpyDeviceToHost, stream_),
                "cfl result");
-    cuda_check(cudaMemcpyAsync(scratch_.words + 8, d_error_.get(), sizeof(unsigned long long),
-                               cudaMemcpyDeviceToHost, stream_),
-               "cfl error");
     cuda_check(cudaStreamSynchronize(stream_), "cfl");
-    raise_device_error(scratch_.words[8]);
+    raise_device_error(scratch_.words[7]);
     double mode0[4];
     for (int v = 0; v < 4; ++v)
       mode0[v] = bits_to_double(scratch_.words[2 + v]);
@@ -408,7 +407,16 @@ public:
 
   void step(double dt) override {
     speed_ready_ = false;
+    enqueue(dt);
+    check();
+  }
+
+  void enqueue(double dt) override {
+    speed_ready_ = false;
     enqueue_step(nullptr, dt);
+  }
+
+  void check() override {
     if (limiting_)
       check_error();
   }
@@ -654,9 +662,10 @@ private:
     // The tile and patch kernels list the elements for the always-on positivity.
     if (limiting_ && d_suspects_.size() > 0 && kernel_ >= 1) {
       a.suspects = d_suspects_.get();
-      a.suspect_count = d_count_.get() + 2;
       a.floors = floors_;
     }
+    if (limiting_) // the three stages' counts
+      cuda_check(cudaMemsetAsync(d_count_.get(), 0, 12 * sizeof(std::int32_t), stream_), "count");
     double *ins[3] = {d_u_.get(), d_e_.get(), d_s_.get()};
     double *outs[3] = {d_e_.get(), d_s_.get(), d_u_.get()};
     for (int k = 0; k < 3; ++k) {
@@ -665,8 +674,11 @@ private:
       a.u0 = d_u_.get();
       a.out = outs[k];
       a.flags = d_flags_.get() + k * ne_;
-      if (limiting_) // troubled, rough and suspect elements
-        cuda_check(cudaMemsetAsync(d_count_.get(), 0, 3 * sizeof(std::int32_t), stream_), "count");
+      if (limiting_) {
+        a.troubled_count = d_count_.get() + 4 * k;
+        a.rough_count = a.troubled_count + 1;
+        a.suspect_count = a.troubled_count + 2;
+      }
       a.speed_max = fused_speed_ && k == 2 && kernel_ >= 1 ? d_speed_.get() : nullptr;
       a.error = d_error_.get();
       stage_begin();
@@ -691,7 +703,7 @@ private:
         m.highest_degree_begin = stencil_.highest_degree_begin;
         m.flags = d_flags_.get() + k * ne_;
         m.troubled = d_troubled_.get();
-        m.troubled_count = d_count_.get();
+        m.troubled_count = a.troubled_count;
         m.stats = d_mlp_stats_.get();
         m.records = d_mlp_records_.get();
         m.error = d_error_.get();
@@ -701,6 +713,8 @@ private:
       }
       if (limiting_) {
         LimitArgs l = limit_args(outs[k], d_flags_.get() + k * ne_);
+        l.troubled_count = a.troubled_count;
+        l.dependent = 1;
         l.suspects = a.suspects;
         l.suspect_count = a.suspect_count;
         launch_limit_f64(M_, 3, l, stream_);

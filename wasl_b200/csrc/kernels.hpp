@@ -176,6 +176,9 @@ struct LimitArgs {
   // == 0: on the suspects the stage kernel listed (not proven to keep the
   // floors), or, without a list, on all of them (a third kernel).
   int positivity_all = 0;
+  // 1: each kernel a programmatic dependent of the launch before it (not while
+  // a stream is captured).
+  int dependent = 0;
   const std::int32_t *suspects = nullptr;
   const std::int32_t *suspect_count = nullptr;
   const std::uint8_t *flags = nullptr;

@@ -65,6 +65,8 @@ public:
     cuda_check(cudaMemsetAsync(d_u_.get(), 0, d_u_.size() * sizeof(double), stream_), "memset");
     d_error_.resize(1);
     d_cfl_.resize(kCflResultWords);
+    cuda_check(cudaMemsetAsync(d_cfl_.get(), 0, kCflResultWords * sizeof(unsigned long long), stream_),
+               "memset");
     d_speed_.resize(1);
     d_dt_.resize(1);
     cuda_check(cudaMemsetAsync(d_error_.get(), 0, sizeof(unsigned long long), stream_), "memset");
@@ -171,11 +173,8 @@ public:
     cuda_check(cudaMemcpyAsync(scratch_.words, d_cfl_.get(), 8 * sizeof(unsigned long long),
                                cudaMemcpyDeviceToHost, stream_),
                "cfl result");
-    cuda_check(cudaMemcpyAsync(scratch_.words + 8, d_error_.get(), sizeof(unsigned long long),
-                               cudaMemcpyDeviceToHost, stream_),
-               "cfl error");
     cuda_check(cudaStreamSynchronize(stream_), "cfl");
-    raise_device_error(scratch_.words[8]);
+    raise_device_error(scratch_.words[7]);
     double mode0[4];
     for (int v = 0; v < 4; ++v)
       mode0[v] = bits_to_double(scratch_.words[2 + v]);
@@ -184,7 +183,13 @@ public:
   }
 
   void step(double dt) override {
-    enqueue_step(nullptr, dt);
+    enqueue(dt);
+    check();
+  }
+
+  void enqueue(double dt) override { enqueue_step(nullptr, dt); }
+
+  void check() override {
     if (limiting_)
       check_error();
   }
@@ -378,7 +383,9 @@ private:
       stage_end();
       count_launches(1);
       if (limiting_) {
-        launch_limit_f64(M_, 2, limit_args(outs[k]), stream_);
+        LimitArgs l = limit_args(outs[k]);
+        l.dependent = 1;
+        launch_limit_f64(M_, 2, l, stream_);
         count_launches(2);
       }
     }

@@ -130,6 +130,11 @@ public:
     throw SolverError(WASL_ERR_ARGUMENT, "cfl parts: only for 2D Euler");
   }
   virtual void step(double dt) = 0;
+  // step() without its wait for the device: an error it raises is the next
+  // stable_dt's to report, or check()'s.
+  virtual void enqueue(double dt) { step(dt); }
+  // Reports a device error of the steps enqueued so far, if they can raise one.
+  virtual void check() {}
   virtual void limit() = 0; // the stage limiter applied to the current state
   // Enqueues `steps` device-resident steps; returns without waiting for
   // them (device errors stay in the error word until sync()).
