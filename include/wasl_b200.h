@@ -232,9 +232,9 @@ int wasl_gpu_sync(wasl_gpu *handle);
  * 4-7: the shared-face tile kernel, which evaluates a face between two
  * elements of one tile once: 4: 64 elements per CTA sized for 7 CTAs per SM;
  * 5: 96 for 5; 6: 128 for 4; 7: 128 for 3; 8-11: the patch kernel, which
- * evaluates each element's traces once and each face inside a patch once,
- * without the limiter only: 8: 128 elements per CTA at <= 128 registers;
- * 9: 128 sized for 5 CTAs per SM; 10: 64 for 8; 11: 64 for 10; 12-13: the
+ * evaluates each element's traces once and each face inside a patch once:
+ * 8: 256 elements per CTA at <= 128 registers; 9: 128 sized for 5 CTAs per
+ * SM; 10: 64 for 8; 11: 192 for 3; 12-13: the
  * patch kernel with its volume contractions on the tensor cores (split-TF32
  * mma.sync, FP32 accumulation): 12: 128 at <= 128 registers, 13: 128 for 5);
  * -1 for forms with a single kernel or before the first step.  When the

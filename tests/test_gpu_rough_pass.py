@@ -22,7 +22,7 @@ def jumping_state(ne, p, seed):
     return c.ravel()
 
 
-@pytest.mark.parametrize("kernel", [2, 5, 8])  # 1 + tile shape 0, 3 + 1 (64 elements), shared-face 128
+@pytest.mark.parametrize("kernel", [2, 5, 8, 10, 12])  # tile 128 and 64, shared-face 128, patch 128 and 64
 @pytest.mark.parametrize("p,nx,ny,boundary", [
     (1, 1, 1, "transmissive"), (2, 3, 3, "periodic"), (3, 3, 3, "transmissive"),
     (1, 13, 5, "periodic"), (2, 13, 5, "transmissive"), (3, 13, 5, "periodic"),

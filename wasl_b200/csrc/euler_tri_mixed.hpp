@@ -22,10 +22,14 @@ namespace wasl_b200 {
 //   6: 128 elements, sized for 4 CTAs per SM (16 warps)
 //   7: 128 elements, sized for 3 CTAs per SM
 // and of the patch kernel:
-//   8: 128 elements, <= 128 registers (4 CTAs per SM)
+//   8: 256 elements, <= 128 registers (2 CTAs per SM)
 //   9: 128 elements, sized for 5 CTAs per SM
 //  10:  64 elements, sized for 8 CTAs per SM
-//  11:  64 elements, sized for 10 CTAs per SM
+//  11: 192 elements, sized for 3 CTAs per SM
+// (larger patches have fewer faces to outside elements, which both patches
+// evaluate: P3 at 500,000 triangles 341 us a stage in shape 8 against 371 with
+// 128 elements at the same registers, at 45,602 triangles 37 us in shape 11
+// against 45; 64 elements suit meshes that larger patches leave SMs idle on)
 // and of the patch kernel with its volume term on the tensor cores:
 //  12: 128 elements, <= 128 registers
 //  13: 128 elements, sized for 5 CTAs per SM
@@ -35,7 +39,7 @@ namespace wasl_b200 {
 //  15: 256 elements, <= 128 registers
 constexpr int kTileShapes = kTileShapeCount;
 constexpr int kTileElements[kTileShapes] = {128, 128, 256, 64, 64, 96, 128, 128,
-                                            128, 128, 64, 64, 128, 128, 128, 256};
+                                            256, 128, 64, 192, 128, 128, 128, 256};
 constexpr int kFirstPatchShape = 8, kPatchShapeEnd = 14;
 
 // R: the volume rule's order, or 0 for the symmetric rule.

@@ -60,6 +60,18 @@ template <int P, int R> struct MixedVolume {
 };
 
 template <int P, int R> __constant__ MixedVolume<P, R> c_mix;
+// The same table in device memory, for copies into shared memory (threads
+// reading constant memory at different addresses take turns).
+template <int P, int R> __device__ MixedVolume<P, R> g_mix;
+
+// How far the point loops are unrolled.  At P3 the unrolled points of a stage
+// kernel (a volume point is some 170 instructions, a face point 150) do not fit
+// the instruction cache, and warps waited for instructions more than for
+// anything but memory: two volume points and one face point per iteration take
+// the patch kernel from 345 to 310 us a stage at 500,000 triangles (four: 320),
+// the shared-face tile kernel from 396 to 376.  At P1 and P2 they fit.
+template <int P, int QV> constexpr int kVolumeUnroll = P < 3 ? QV : 2;
+template <int P> constexpr int kFaceUnroll = P < 3 ? TriShape<P>::QF : 1;
 // FP64 sum of the reference edge weights of each local edge.
 template <int P> __constant__ double c_edge_wsum[3];
 
@@ -631,7 +643,7 @@ __device__ __forceinline__ bool mean_jump(double rho_a, double rho_b, double e_a
          fabs(e_a - e_b) > kFp64Jump * fmin(e_a, e_b);
 }
 
-// One face in FP64 (the mixed form's islands): traces of both elements from
+// One point of a face in FP64 (faces across jumps): traces of both elements from
 // their FP64 coefficients (rows stride apart) and the FP64 face tables, HLLC
 // in FP64 (reference order of operations up to contraction), then the
 // high-mode perturbations dflux[q][v] = F_q - F(U_L bar).n (FP32) and the
@@ -665,30 +677,6 @@ __device__ __forceinline__ void face_point_fp64(double gamma, const double *own,
   }
   hllc_fast(gamma, ul, ur, nx, ny, f);
 }
-
-template <int P>
-__device__ __noinline__ void face_fp64(double gamma, const double *own, std::int64_t own_stride,
-                                       const double *other, std::int64_t other_stride,
-                                       bool boundary, bool self_left, const double *own_basis,
-                                       const double *other_basis, const double *weights,
-                                       double nx, double ny, const double *fln,
-                                       float (*dflux)[4], double *mode0) {
-  constexpr int M = TriShape<P>::M, QF = TriShape<P>::QF;
-#pragma unroll
-  for (int v = 0; v < 4; ++v)
-    mode0[v] = 0.0;
-  for (int q = 0; q < QF; ++q) {
-    double f[4];
-    face_point_fp64<P>(gamma, own, own_stride, other, other_stride, boundary, self_left,
-                       own_basis + q * M, other_basis + q * M, nx, ny, f);
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      dflux[q][v] = static_cast<float>(f[v] - fln[v]);
-      mode0[v] = fma(weights[q], f[v], mode0[v]);
-    }
-  }
-}
-
 
 // The end of a tile kernel's stage for element e (thread t of the tile):
 // residual scaling by 1/det J, the Shu-Osher combination in FP64
@@ -960,7 +948,9 @@ __device__ __forceinline__ void tile_element(const StageArgs &a, const FaceTable
     const float fscale = static_cast<float>(scale);
     const double sgn = self_left ? -1.0 : 1.0;
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
+    // (Rolled: the instruction cache again, 485 -> 435 us a stage at P3, 216 -> 207 at
+    // P2, 500,000 triangles.)
+#pragma unroll 1
     for (int q = 0; q < QF; ++q) {
       float to[4], tn[4], dl[4], dr[4], fl[4];
       high_trace<P>(ch, own_basis + q * M, to);
@@ -1046,351 +1036,6 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_tile_mixed(const StageAr
   if (!active)
     return;
   tile_element<P, R, TILE>(a, table, sstate, t, e, first, count, case_id);
-}
-
-// The second pass of the tile kernels: the elements the FP32 pass left (those
-// with a face across a jump of the cell means; its faces across a jump in
-// FP64, the others in FP32), 16 lanes per element.
-//
-// Near shocks the list is short (1-2% of the elements) and an element's work
-// long: its 3 (P + 1) face points with an FP64 HLLC each and its volume points,
-// one after another in one thread, were a chain of about 80 us at P3 however
-// few the elements.  Here each lane takes one face point, then one volume
-// point; then the lanes share out the 4 M coefficients, each summing its own
-// over the volume points and the faces' points in the tile kernel's order.  The
-// arithmetic is the tile kernel's, value for value, so both elements of every
-// face still get the same bits.  Bound by latency.  P3, 500,000 triangles with
-// four shocked quadrants, a stage with this pass: 494 -> 412 us.
-constexpr int kRoughLanes = 16, kRoughThreads = 128;
-
-template <int P, int R> struct RoughElement {
-  static constexpr int M = TriShape<P>::M, QF = TriShape<P>::QF, QV = MixedVolume<P, R>::QV;
-  double own[4 * M], across[3][4 * M]; // coefficients
-  double flux[3 * QF][4];              // FP64 faces: the flux
-  double fln[3][4];                    // each face's left mean's normal flux
-  double next[4 * M];                  // the new stage's coefficients
-  float dflux[3 * QF][4];              // the flux's perturbation
-  float shift[3][4];                   // to this element's mean (right element)
-  float volume[QV][8];                 // G_xi and G_eta per variable
-  float basis[3 * QF][M];              // this element's basis at its face points
-  int fp64[3];
-};
-
-template <int P, int R>
-__global__ void __launch_bounds__(kRoughThreads) euler_tri_rough(const StageArgs a) {
-  using S = TriShape<P>;
-  constexpr int M = S::M, QV = MixedVolume<P, R>::QV, QF = S::QF, H = M - 1;
-  constexpr int GROUPS = kRoughThreads / kRoughLanes;
-  constexpr double phi0 = 0.70710678118654752440;
-  static_assert(3 * QF <= kRoughLanes, "one lane per face point");
-  __shared__ FaceTable<P, float> table;
-  __shared__ MixedVolume<P, R> T;
-  extern __shared__ __align__(16) unsigned char rough_smem[];
-  RoughElement<P, R> &E =
-      reinterpret_cast<RoughElement<P, R> *>(rough_smem)[threadIdx.x / kRoughLanes];
-  const std::int64_t list = *a.rough_count;
-  if (static_cast<std::int64_t>(blockIdx.x) * GROUPS >= list)
-    return; // the whole block is past the list (uniform: no barrier reached)
-  const int t = threadIdx.x, lane = t % kRoughLanes;
-  {
-    const float *src = static_cast<const float *>(a.face_table);
-    float *dst = reinterpret_cast<float *>(&table);
-    for (int i = t; i < static_cast<int>(sizeof(table) / sizeof(float)); i += kRoughThreads)
-      dst[i] = src[i];
-    const float *mix = reinterpret_cast<const float *>(&c_mix<P, R>);
-    float *vol = reinterpret_cast<float *>(&T);
-    for (int i = t; i < static_cast<int>(sizeof(T) / sizeof(float)); i += kRoughThreads)
-      vol[i] = mix[i];
-  }
-  __syncthreads();
-  const std::int64_t ne = a.mesh.ne;
-  const double *__restrict__ in = a.in;
-  const double *__restrict__ geo = a.mesh.geo;
-  const double gamma = a.gamma;
-  const float gamma32 = static_cast<float>(gamma), g1 = static_cast<float>(gamma - 1.0);
-  // (Both groups of a warp go round together; one past the list's end idles
-  // along on its last element without writing.)
-  const std::int64_t begin = static_cast<std::int64_t>(blockIdx.x) * GROUPS + t / 32 * 2;
-  for (std::int64_t w = begin; w < list; w += static_cast<std::int64_t>(gridDim.x) * GROUPS) {
-    const std::int64_t at = w + (t / kRoughLanes) % 2;
-    const bool valid = at < list;
-    const std::int64_t e = a.rough[valid ? at : list - 1];
-    const int case_id = a.element_case ? a.element_case[e] : 0;
-    // Coefficients of the element and its neighbours.
-    for (int i = lane; i < 4 * M; i += kRoughLanes)
-      E.own[i] = in[i * ne + e];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const std::int32_t nb = a.tile.nbr[k * ne + e];
-      if (nb >= 0)
-        for (int i = lane; i < 4 * M; i += kRoughLanes)
-          E.across[k][i] = __ldg(in + i * ne + nb);
-    }
-    __syncwarp();
-    double mean[4];
-#pragma unroll
-    for (int v = 0; v < 4; ++v)
-      mean[v] = E.own[v * M] * phi0;
-    const MeanState own = mean_state(gamma, mean);
-
-    // One face point per lane.
-    if (lane < 3 * QF) {
-      const int k = lane / QF, q = lane % QF;
-      const std::int64_t slot = k * ne + e;
-      const unsigned code = a.tile.code[slot];
-      const std::int32_t nb = a.tile.nbr[slot];
-      const bool self_left = code & 1u, boundary = nb < 0;
-      const int le = (code >> 1) & 3u, re = (code >> 3) & 3u, flip = (code >> 5) & 1u;
-      const double nx = a.mesh.slot_geo[(3 * k) * ne + e];
-      const double ny = a.mesh.slot_geo[(3 * k + 1) * ne + e];
-      const float *lb = &table.lb[le][0][0];
-      const float *rb = &table.rb[(le * 3 + re) * 2 + flip][0][0];
-      const float *own_basis = self_left ? lb : rb;
-      const float *other_basis = self_left ? rb : lb;
-      if (code & 0xC0u) {
-        const float *periodic =
-            a.boundary.basis32 + static_cast<std::int64_t>(a.tile.aux[slot]) * QF * M;
-        if (code & 0x40u)
-          own_basis = periodic;
-        else
-          other_basis = periodic;
-      }
-      double nmean[4] = {0.0, 0.0, 0.0, 0.0};
-      if (!boundary) {
-#pragma unroll
-        for (int v = 0; v < 4; ++v)
-          nmean[v] = E.across[k][v * M] * phi0;
-      }
-      // The face's left state is the reference of the perturbation form.
-      MeanState ml;
-      if (self_left)
-        ml = own;
-      else
-        ml = mean_state(gamma, nmean);
-      double fln[4];
-      mean_normal_flux(ml, nx, ny, fln);
-      const bool fp64 = !boundary && mean_jump(nmean[0], mean[0], nmean[3], mean[3]);
-      if (q == 0) {
-        float shift[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        if (!boundary && !self_left) {
-          double frn[4];
-          mean_normal_flux(own, nx, ny, frn);
-#pragma unroll
-          for (int v = 0; v < 4; ++v)
-            shift[v] = static_cast<float>(fln[v] - frn[v]);
-        }
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          E.fln[k][v] = fln[v];
-          E.shift[k][v] = shift[v];
-        }
-        E.fp64[k] = fp64;
-      }
-#pragma unroll
-      for (int m = 0; m < M; ++m)
-        E.basis[lane][m] = own_basis[q * M + m];
-      if (fp64) {
-        const FaceTable<P, double> *T64 = static_cast<const FaceTable<P, double> *>(a.face_table64);
-        const double *lb64 = &T64->lb[le][0][0];
-        const double *rb64 = &T64->rb[(le * 3 + re) * 2 + flip][0][0];
-        const double *own64 = self_left ? lb64 : rb64;
-        const double *other64 = self_left ? rb64 : lb64;
-        if (code & 0xC0u) {
-          const double *periodic =
-              a.mesh.donor_basis + static_cast<std::int64_t>(a.tile.aux[slot]) * QF * M;
-          if (code & 0x40u)
-            own64 = periodic;
-          else
-            other64 = periodic;
-        }
-        double f[4];
-        face_point_fp64<P>(gamma, E.own, 1, E.across[k], 1, false, self_left, own64 + q * M,
-                           other64 + q * M, nx, ny, f);
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          E.flux[lane][v] = f[v];
-          E.dflux[lane][v] = static_cast<float>(f[v] - fln[v]);
-        }
-      } else {
-        const Ref32 ref = ref32(ml);
-        float to[4], tn[4], dl[4], dr[4], fl[4];
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          float s = 0.0f;
-#pragma unroll
-          for (int m = 0; m < H; ++m)
-            s = fmaf(static_cast<float>(E.own[v * M + m + 1]), own_basis[q * M + m + 1], s);
-          to[v] = s;
-        }
-        if (boundary) {
-#pragma unroll
-          for (int v = 0; v < 4; ++v)
-            dl[v] = dr[v] = to[v];
-        } else {
-#pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            float s = 0.0f;
-#pragma unroll
-            for (int m = 0; m < H; ++m)
-              s = fmaf(static_cast<float>(E.across[k][v * M + m + 1]), other_basis[q * M + m + 1], s);
-            tn[v] = s;
-          }
-#pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            const float jump =
-                static_cast<float>(self_left ? nmean[v] - mean[v] : mean[v] - nmean[v]);
-            dl[v] = self_left ? to[v] : tn[v];
-            dr[v] = jump + (self_left ? tn[v] : to[v]);
-          }
-        }
-        hllc_perturbed(ref, dl, dr, g1, gamma32, static_cast<float>(nx), static_cast<float>(ny), fl);
-#pragma unroll
-        for (int v = 0; v < 4; ++v)
-          E.dflux[lane][v] = fl[v];
-      }
-    }
-
-    // One volume point per lane (as the tile kernel).
-    {
-      const Ref32 bb = ref32(own);
-      const float fax = static_cast<float>(geo[e]), fay = static_cast<float>(geo[ne + e]);
-      const float fbx = static_cast<float>(geo[2 * ne + e]), fby = static_cast<float>(geo[3 * ne + e]);
-      for (int q = lane; q < QV; q += kRoughLanes) {
-        float d[4];
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          float s = 0.0f;
-#pragma unroll
-          for (int m = 0; m < H; ++m)
-            s = fmaf(static_cast<float>(E.own[v * M + m + 1]), T.phi[q][m], s);
-          d[v] = s;
-        }
-        const float inv = __frcp_rn(fmaxf(bb.rho + d[0], kVacuumFraction * bb.rho));
-        const float du = (d[1] - bb.u * d[0]) * inv;
-        const float dv = (d[2] - bb.v * d[0]) * inv;
-        const float uu = bb.u + du, vv = bb.v + dv;
-        const float dmu = bb.mx * du + d[1] * uu + bb.my * dv + d[2] * vv;
-        const float dp = g1 * (d[3] - 0.5f * dmu);
-        const float dep = d[3] + dp;
-        const float fx[4] = {d[1], bb.mx * du + d[1] * uu + dp, bb.my * du + d[2] * uu,
-                             bb.h * du + dep * uu};
-        const float fy[4] = {d[2], bb.mx * dv + d[1] * vv, bb.my * dv + d[2] * vv + dp,
-                             bb.h * dv + dep * vv};
-        const float wq = T.w[q];
-        const float wby = wq * fby, wbx = wq * fbx, wax = wq * fax, way = wq * fay;
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          E.volume[q][v] = wby * fx[v] - wbx * fy[v];
-          E.volume[q][4 + v] = wax * fy[v] - way * fx[v];
-        }
-      }
-    }
-    __syncwarp();
-
-    // One coefficient after another per lane: its residual in the tile
-    // kernel's order, and the Shu-Osher combination.
-    const double inv = geo[4 * ne + e];
-    const double dt = a.case_dt ? a.case_dt[case_id] : (a.dt ? *a.dt : a.dt_value);
-    for (int i = lane; i < 4 * M; i += kRoughLanes) {
-      const int v = i / M, m = i % M;
-      float racc = 0.0f;
-      double r0 = 0.0;
-      if (m > 0)
-        for (int q = 0; q < QV; ++q)
-          racc = fmaf(T.dxi[q][m - 1], E.volume[q][v], fmaf(T.deta[q][m - 1], E.volume[q][4 + v], racc));
-#pragma unroll 1
-      for (int k = 0; k < 3; ++k) {
-        const unsigned code = a.tile.code[k * ne + e];
-        const bool self_left = code & 1u;
-        const int le = (code >> 1) & 3u;
-        const double scale = a.mesh.slot_geo[(3 * k + 2) * ne + e];
-        const float fscale = static_cast<float>(scale);
-        if (m > 0) {
-#pragma unroll
-          for (int q = 0; q < QF; ++q) {
-            const float wq = table.ew[le][q];
-            const float wsc = (self_left ? -wq : wq) * fscale;
-            const float fl = E.dflux[k * QF + q][v];
-            const float value = wsc * (self_left ? fl : fl + E.shift[k][v]);
-            racc = fmaf(value, E.basis[k * QF + q][m], racc);
-          }
-        } else {
-          const double sgn = self_left ? -1.0 : 1.0;
-          if (E.fp64[k]) {
-            const FaceTable<P, double> *T64 =
-                static_cast<const FaceTable<P, double> *>(a.face_table64);
-            double mode0 = 0.0;
-#pragma unroll
-            for (int q = 0; q < QF; ++q)
-              mode0 = fma(T64->ew[le][q], E.flux[k * QF + q][v], mode0);
-            r0 += sgn * scale * phi0 * mode0;
-          } else {
-            float acc = 0.0f;
-#pragma unroll
-            for (int q = 0; q < QF; ++q)
-              acc = fmaf(table.ew[le][q], E.dflux[k * QF + q][v], acc);
-            const double mode0 = E.fln[k][v] * c_edge_wsum<P>[le] + static_cast<double>(acc);
-            r0 += sgn * scale * phi0 * mode0;
-          }
-        }
-      }
-      const std::int64_t idx = i * ne + e;
-      const double cur = E.own[i];
-      const double rr = (m == 0 ? r0 : static_cast<double>(racc)) * inv;
-      double o;
-      if (a.stage == 0)
-        o = cur + dt * rr;
-      else if (a.stage == 1)
-        o = 0.75 * a.u0[idx] + 0.25 * (cur + dt * rr);
-      else
-        o = (1.0 / 3.0) * a.u0[idx] + (2.0 / 3.0) * (cur + dt * rr);
-      if (valid)
-        a.out[idx] = o;
-      E.next[i] = o;
-    }
-    __syncwarp();
-    if (lane == 0 && valid) {
-      if (a.speed_max) {
-        const double scale = 1.0 / sqrt(2.0);
-        const double sa[4] = {__dmul_rn(scale, E.next[0]), __dmul_rn(scale, E.next[M]),
-                              __dmul_rn(scale, E.next[2 * M]), __dmul_rn(scale, E.next[3 * M])};
-        bool physical = true;
-        const double speed = cfl_speed(gamma, sa, 2, physical);
-        if (physical)
-          atomicMax(a.speed_max + case_id,
-                    static_cast<unsigned long long>(__double_as_longlong(speed)));
-        else
-          raise_error(a.error, kNonPhysicalAverage, e);
-      }
-      if (a.suspects) {
-        double mode0[4], reach[4];
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          mode0[v] = E.next[v * M];
-          reach[v] = 0.0;
-#pragma unroll
-          for (int m = 1; m < M; ++m)
-            reach[v] += fabs(E.next[v * M + m]) * a.floors.bound[m];
-        }
-        if (!positivity_clear(gamma, a.floors, mode0, reach))
-          a.suspects[atomicAdd(a.suspect_count, 1)] = static_cast<std::int32_t>(e);
-      }
-      if (a.sense) {
-        double total = 0.0, high = 0.0;
-#pragma unroll
-        for (int m = 0; m < M; ++m) {
-          total += E.next[m] * E.next[m];
-          if (m >= a.highest_degree_begin)
-            high += E.next[m] * E.next[m];
-        }
-        const bool troubled = !(total == 0.0 || high / total <= a.threshold);
-        a.flags[e] = troubled ? 1 : 0;
-        if (troubled)
-          a.troubled[atomicAdd(a.troubled_count, 1)] = static_cast<std::int32_t>(e);
-      }
-    }
-    __syncwarp(); // the next element's coefficients may land
-  }
 }
 
 // The FP32 pass of the tile kernel as a persistent kernel: each CTA loads the
@@ -1721,7 +1366,7 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_tile_shared(const StageA
         jump[v] = boundary ? 0.0f
                            : static_cast<float>(self_left ? nmean[v] - mean[v] : mean[v] - nmean[v]);
       const float nxf = static_cast<float>(nx), nyf = static_cast<float>(ny);
-#pragma unroll
+#pragma unroll kFaceUnroll<P>
       for (int j = 0; j < NQ; ++j) {
         const int q = q0 + j;
         float to[4], tn[4], dl[4], dr[4], fl[4];
@@ -1784,7 +1429,7 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_tile_shared(const StageA
   const double *__restrict__ geo = a.mesh.geo;
   const Ref32 bb = ref32(own);
 
-  // Volume term of the high modes (as the tile kernel, fully unrolled).
+  // Volume term of the high modes (as the tile kernel).
   float racc[4][H];
 #pragma unroll
   for (int v = 0; v < 4; ++v)
@@ -1794,7 +1439,7 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_tile_shared(const StageA
   {
     const float fax = static_cast<float>(geo[e]), fay = static_cast<float>(geo[ne + e]);
     const float fbx = static_cast<float>(geo[2 * ne + e]), fby = static_cast<float>(geo[3 * ne + e]);
-#pragma unroll
+#pragma unroll kVolumeUnroll<P, QV>
     for (int q = 0; q < QV; ++q) {
       float d[4];
 #pragma unroll
@@ -1946,6 +1591,7 @@ template <int P> struct PatchEdge {
   float w[3][QF];      // reference edge weights
 };
 template <int P> __constant__ PatchEdge<P> c_patch;
+template <int P> __device__ PatchEdge<P> g_patch; // for copies into shared memory
 
 // ---- the volume term on the tensor cores (patch kernel, MMA variant) ---------
 //
@@ -2308,7 +1954,7 @@ __device__ __forceinline__ void patch_finish(const StageArgs &a, std::int64_t e,
   }
 }
 
-template <int P, int R, int TILE, int MINB, bool MMA, bool ISLANDS>
+template <int P, int R, int TILE, int MINB, bool MMA, bool LIMITED>
 __global__ void __launch_bounds__(TILE, MINB) euler_tri_patch(const StageArgs a) {
   using S = TriShape<P>;
   using L = PatchSmem<P, R, TILE, MMA>;
@@ -2317,6 +1963,7 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_patch(const StageArgs a)
   static_assert(4 * TILE < 65536, "face items are 16-bit");
   __shared__ PatchEdge<P> table; // for the few runtime-indexed reads
   __shared__ int item_count;
+  __shared__ std::uint8_t srough[LIMITED ? TILE : 1];
   extern __shared__ __align__(16) unsigned char smem[];
   double(*smean)[TILE] = reinterpret_cast<double(*)[TILE]>(smem + L::mean);
   double(*sprim)[TILE] = reinterpret_cast<double(*)[TILE]>(smem + L::prim);
@@ -2349,11 +1996,9 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_patch(const StageArgs a)
   const double *__restrict__ in = a.in;
   const double gamma = a.gamma;
   const PatchEdges pe = a.patch;
-  // ISLANDS (with the limiter): faces across jumps of the cell means in FP64.
-  constexpr bool islands = ISLANDS;
 
   {
-    const float *src = reinterpret_cast<const float *>(&c_patch<P>);
+    const float *src = reinterpret_cast<const float *>(&g_patch<P>);
     float *dst = reinterpret_cast<float *>(&table);
     for (int i = t; i < static_cast<int>(sizeof(table) / sizeof(float)); i += TILE)
       dst[i] = src[i];
@@ -2395,6 +2040,7 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_patch(const StageArgs a)
 
   // A. State, traces, and the faces this element evaluates.
   bool evaluates[3] = {false, false, false};
+  bool rough = false; // LIMITED: a face across a jump of the cell means
   if (active) {
     std::int32_t nbrs[3];
     unsigned infos[3];
@@ -2452,7 +2098,37 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_patch(const StageArgs a)
       evaluates[j] = !inside || (infos[j] & 1u);
     }
   }
-  __syncthreads(); // item_count and the tables are set
+  __syncthreads(); // the states, item_count and the tables are set
+  if constexpr (LIMITED) {
+    // An element with a face across a jump of the means is left to the second
+    // pass; a face is evaluated where an element that stays needs it.
+    std::int32_t across[3] = {-1, -1, -1};
+    if (active) {
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        const std::int32_t raw = pe.nbr[j * ne + e];
+        if (raw < 0)
+          continue;
+        const std::int64_t nb = checked_index(raw, ne, a.error), local = nb - first;
+        double n0, n3;
+        if (local >= 0 && local < count) {
+          across[j] = static_cast<std::int32_t>(local);
+          n0 = smean[0][local];
+          n3 = smean[3][local];
+        } else {
+          n0 = __ldg(in + nb) * phi0;
+          n3 = __ldg(in + static_cast<std::int64_t>(3) * M * ne + nb) * phi0;
+        }
+        rough = rough || mean_jump(n0, smean[0][t], n3, smean[3][t]);
+      }
+    }
+    srough[t] = rough ? 1 : 0;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      if (rough && (across[j] < 0 || srough[across[j]]))
+        evaluates[j] = false;
+  }
   {
     const int lane = t & 31;
 #pragma unroll
@@ -2499,10 +2175,6 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_patch(const StageArgs a)
         for (int v = 0; v < 4; ++v)
           nmean[v] = __ldg(in + static_cast<std::int64_t>(v) * M * ne + nb) * phi0;
       }
-      // A face across a jump of the means is evaluated in FP64 by each of its
-      // elements in phase C (with the limiter): no record here.
-      if (islands && !boundary && mean_jump(nmean[0], mean[0], nmean[3], mean[3]))
-        return;
       // The face's left mean state: the reference of the perturbation form.
       MeanState ml;
       if (self_left || boundary)
@@ -2518,7 +2190,7 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_patch(const StageArgs a)
         jump[v] = boundary ? 0.0f
                            : static_cast<float>(self_left ? nmean[v] - mean[v] : mean[v] - nmean[v]);
       const float nxf = static_cast<float>(nx), nyf = static_cast<float>(ny);
-#pragma unroll
+#pragma unroll kFaceUnroll<P>
       for (int jq = 0; jq < NQ; ++jq) {
         const int q = q0 + jq;              // the face's point (left element's order)
         const int qr = rev ? QF - 1 - q : q; // the right element's point
@@ -2566,6 +2238,10 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_patch(const StageArgs a)
     patch_volume_mma<P, R, TILE>(shi, sbb, sgeo, sfrag, g1, t & ~31, t & 31);
   if (!active)
     return;
+  if (LIMITED && rough) {
+    a.rough[atomicAdd(a.rough_count, 1)] = static_cast<std::int32_t>(e);
+    return;
+  }
 
   // C. Volume term, lifting, mode 0, combination.
   const MeanState own = patch_mean<P, TILE>(smean, sprim, t);
@@ -2593,7 +2269,7 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_patch(const StageArgs a)
     const double *__restrict__ geo = a.mesh.geo;
     const float fax = static_cast<float>(geo[e]), fay = static_cast<float>(geo[ne + e]);
     const float fbx = static_cast<float>(geo[2 * ne + e]), fby = static_cast<float>(geo[3 * ne + e]);
-#pragma unroll
+#pragma unroll kVolumeUnroll<P, QV>
     for (int q = 0; q < QV; ++q) {
       float d[4];
 #pragma unroll
@@ -2645,7 +2321,6 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_patch(const StageArgs a)
     const int jl = self_left ? j : jn; // the face's left local edge (its weights)
     // The face's flux perturbations in the face's point order: from this
     // element's record, or from its left neighbour's inside the patch.
-    // (An FP64 face overwrites these with its own values below.)
     float fq[QF][4];
     if (near && !self_left) {
 #pragma unroll
@@ -2662,62 +2337,21 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_patch(const StageArgs a)
           fq[q][v] = sedge[(j * QF + qs) * 4 + v][t];
       }
     }
-    // The face's left mean state; with islands, the neighbour's mean for the
-    // jump test as well.
+    // The face's left mean state.
     MeanState ml;
-    double nmean[4] = {0.0, 0.0, 0.0, 0.0};
-    if constexpr (ISLANDS) {
-      if (near) {
-#pragma unroll
-        for (int v = 0; v < 4; ++v)
-          nmean[v] = smean[v][local];
-      } else if (!boundary) {
-#pragma unroll
-        for (int v = 0; v < 4; ++v)
-          nmean[v] = __ldg(in + static_cast<std::int64_t>(v) * M * ne + nb) * phi0;
-      }
-    }
     if (self_left || boundary) {
       ml = own;
     } else if (near) {
       ml = patch_mean<P, TILE>(smean, sprim, static_cast<int>(local));
     } else {
-      if constexpr (!ISLANDS) {
+      double nmean[4];
 #pragma unroll
-        for (int v = 0; v < 4; ++v)
-          nmean[v] = __ldg(in + static_cast<std::int64_t>(v) * M * ne + nb) * phi0;
-      }
+      for (int v = 0; v < 4; ++v)
+        nmean[v] = __ldg(in + static_cast<std::int64_t>(v) * M * ne + nb) * phi0;
       ml = mean_state(gamma, nmean);
     }
     double fln[4];
     mean_normal_flux(ml, nx, ny, fln);
-    const bool fp64 = ISLANDS && !boundary &&
-                      mean_jump(nmean[0], smean[0][t], nmean[3], smean[3][t]);
-    double m0[4] = {0.0, 0.0, 0.0, 0.0};
-    if constexpr (ISLANDS) {
-      if (fp64) {
-        // The face in FP64 from both elements' coefficients, as the tile
-        // kernels' rough pass evaluates it (the same call with the same roles
-        // on both sides, so both elements apply the same bits).
-        const FaceTable<P, double> *T64 =
-            static_cast<const FaceTable<P, double> *>(a.face_table64);
-        const int le = self_left ? j : jn, re = self_left ? jn : j;
-        // The tables' flip is the edges' relative direction along the
-        // counter-clockwise parametrization; rev compares the edges' own
-        // point orders, and edge 2's points run against it.
-        const int flip = (rev ? 1 : 0) ^ (le == 2 ? 1 : 0) ^ (re == 2 ? 1 : 0);
-        const double *lb64 = &T64->lb[le][0][0];
-        const double *rb64 = &T64->rb[(le * 3 + re) * 2 + flip][0][0];
-        float dq[QF][4];
-        face_fp64<P>(gamma, in + e, ne, in + nb, ne, false, self_left, self_left ? lb64 : rb64,
-                     self_left ? rb64 : lb64, &T64->ew[le][0], nx, ny, fln, dq, m0);
-#pragma unroll
-        for (int q = 0; q < QF; ++q)
-#pragma unroll
-          for (int v = 0; v < 4; ++v)
-            fq[q][v] = dq[q][v];
-      }
-    }
     float shift[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     if (!boundary && !self_left) {
       double frn[4];
@@ -2728,24 +2362,18 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_patch(const StageArgs a)
     }
     const float fscale = static_cast<float>(scale);
     const double sgn = self_left ? -1.0 : 1.0;
-    if (fp64) {
+    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int q = 0; q < QF; ++q) {
+      const float w = table.w[jl][q];
 #pragma unroll
       for (int v = 0; v < 4; ++v)
-        r0[v] += sgn * scale * phi0 * m0[v];
-    } else {
-      float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        acc[v] = fmaf(w, fq[q][v], acc[v]);
+    }
 #pragma unroll
-      for (int q = 0; q < QF; ++q) {
-        const float w = table.w[jl][q];
-#pragma unroll
-        for (int v = 0; v < 4; ++v)
-          acc[v] = fmaf(w, fq[q][v], acc[v]);
-      }
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        const double mode0 = fln[v] * c_edge_wsum<P>[jl] + static_cast<double>(acc[v]);
-        r0[v] += sgn * scale * phi0 * mode0;
-      }
+    for (int v = 0; v < 4; ++v) {
+      const double mode0 = fln[v] * c_edge_wsum<P>[jl] + static_cast<double>(acc[v]);
+      r0[v] += sgn * scale * phi0 * mode0;
     }
     // High modes at this element's own points qo (the face's point q).
 #pragma unroll
@@ -2763,7 +2391,422 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_patch(const StageArgs a)
       }
     }
   }
-  patch_finish<P, ISLANDS>(a, e, case_id, r0, racc);
+  patch_finish<P, LIMITED>(a, e, case_id, r0, racc);
+}
+
+// The second pass of the tile and patch kernels: the elements the FP32 pass
+// left (those with a face across a jump of the cell means; its faces across a
+// jump in FP64, the others in FP32), 16 lanes per element.
+//
+// Near shocks the list is short (1-2% of the elements) and an element's work
+// long: its 3 (P + 1) face points with an FP64 HLLC each and its volume points,
+// one after another in one thread, were a chain of about 80 us at P3 however
+// few the elements.  Here each lane takes one face point, then one volume
+// point; then the lanes share out the 4 M coefficients, each summing its own
+// over the volume points and the faces' points in the first pass's order.  The
+// arithmetic is that pass's, value for value (PATCH: the patch kernel's edges,
+// traces and reciprocals; else the tile kernels'), so both elements of every
+// face still get the same bits.  Bound by latency: 26 us at P3 for the few
+// thousand elements of 32 shocked cases, 78 us with one thread each.
+constexpr int kRoughLanes = 16, kRoughThreads = 128;
+
+template <int P, int R> struct RoughElement {
+  static constexpr int M = TriShape<P>::M, QF = TriShape<P>::QF, QV = MixedVolume<P, R>::QV;
+  double own[4 * M], across[3][4 * M]; // coefficients
+  double flux[3 * QF][4];              // FP64 faces: the flux
+  double fln[3][4];                    // each face's left mean's normal flux
+  double next[4 * M];                  // the new stage's coefficients
+  float dflux[3 * QF][4];              // the flux's perturbation
+  float shift[3][4];                   // to this element's mean (right element)
+  float volume[QV][8];                 // G_xi and G_eta per variable
+  float basis[3 * QF][M > 1 ? M - 1 : 1]; // its high modes' basis at the face points
+  double geo[5], face[9];              // the element's geometry, its faces'
+  std::int32_t nb[3];
+  int code[3], fp64[3];
+};
+
+template <int P, int R, bool PATCH>
+__global__ void __launch_bounds__(kRoughThreads) euler_tri_rough(const StageArgs a) {
+  using S = TriShape<P>;
+  constexpr int M = S::M, QV = MixedVolume<P, R>::QV, QF = S::QF, H = M - 1;
+  constexpr int GROUPS = kRoughThreads / kRoughLanes;
+  constexpr double phi0 = 0.70710678118654752440;
+  static_assert(3 * QF <= kRoughLanes, "one lane per face point");
+  using Table = std::conditional_t<PATCH, PatchEdge<P>, FaceTable<P, float>>;
+  __shared__ Table table;
+  __shared__ MixedVolume<P, R> T;
+  __shared__ FaceTable<P, double> T64;
+  extern __shared__ __align__(16) unsigned char rough_smem[];
+  RoughElement<P, R> &E =
+      reinterpret_cast<RoughElement<P, R> *>(rough_smem)[threadIdx.x / kRoughLanes];
+  const std::int64_t list = *a.rough_count;
+  if (static_cast<std::int64_t>(blockIdx.x) * GROUPS >= list)
+    return; // the whole block is past the list (uniform: no barrier reached)
+  const int t = threadIdx.x, lane = t % kRoughLanes;
+  {
+    const float *src;
+    if constexpr (PATCH)
+      src = reinterpret_cast<const float *>(&g_patch<P>);
+    else
+      src = static_cast<const float *>(a.face_table);
+    float *dst = reinterpret_cast<float *>(&table);
+    for (int i = t; i < static_cast<int>(sizeof(table) / sizeof(float)); i += kRoughThreads)
+      dst[i] = src[i];
+    const float *mix = reinterpret_cast<const float *>(&g_mix<P, R>);
+    float *vol = reinterpret_cast<float *>(&T);
+    for (int i = t; i < static_cast<int>(sizeof(T) / sizeof(float)); i += kRoughThreads)
+      vol[i] = mix[i];
+    const double *src64 = static_cast<const double *>(a.face_table64);
+    double *dst64 = reinterpret_cast<double *>(&T64);
+    for (int i = t; i < static_cast<int>(sizeof(T64) / sizeof(double)); i += kRoughThreads)
+      dst64[i] = src64[i];
+  }
+  __syncthreads();
+  const std::int64_t ne = a.mesh.ne;
+  const double *__restrict__ in = a.in;
+  const double *__restrict__ geo = a.mesh.geo;
+  const double gamma = a.gamma;
+  const float gamma32 = static_cast<float>(gamma), g1 = static_cast<float>(gamma - 1.0);
+  const std::int32_t *nbrs = PATCH ? a.patch.nbr : a.tile.nbr;
+  const std::uint8_t *codes = PATCH ? a.patch.info : a.tile.code;
+  const double *face_geo = PATCH ? a.patch.geo : a.mesh.slot_geo;
+  // (Both groups of a warp go round together; one past the list's end idles
+  // along on its last element without writing.)
+  const std::int64_t begin = static_cast<std::int64_t>(blockIdx.x) * GROUPS + t / 32 * 2;
+  for (std::int64_t w = begin; w < list; w += static_cast<std::int64_t>(gridDim.x) * GROUPS) {
+    const std::int64_t at = w + (t / kRoughLanes) % 2;
+    const bool valid = at < list;
+    const std::int64_t e = a.rough[valid ? at : list - 1];
+    const int case_id = a.element_case ? a.element_case[e] : 0;
+    // Everything that depends on the element alone, then its neighbours'
+    // coefficients: two round trips to memory.
+    constexpr int OWN = (4 * M + kRoughLanes - 1) / kRoughLanes;
+    double u0[OWN];
+#pragma unroll
+    for (int c = 0; c < OWN; ++c) {
+      const int i = c * kRoughLanes + lane;
+      u0[c] = 0.0;
+      if (i < 4 * M) {
+        E.own[i] = in[i * ne + e];
+        if (a.stage > 0)
+          u0[c] = a.u0[i * ne + e];
+      }
+    }
+    if (lane < 9)
+      E.face[lane] = face_geo[lane * ne + e];
+    if (lane < 5)
+      E.geo[lane] = geo[lane * ne + e];
+    if (lane < 3) {
+      const std::int32_t raw = nbrs[lane * ne + e];
+      E.nb[lane] = raw >= 0 ? static_cast<std::int32_t>(checked_index(raw, ne, a.error)) : raw;
+      E.code[lane] = codes[lane * ne + e];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const std::int64_t nb = E.nb[k];
+#pragma unroll
+      for (int c = 0; c < OWN; ++c) {
+        const int i = c * kRoughLanes + lane;
+        if (nb >= 0 && i < 4 * M)
+          E.across[k][i] = __ldg(in + i * ne + nb);
+      }
+    }
+    __syncwarp();
+    double mean[4];
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+      mean[v] = E.own[v * M] * phi0;
+    const MeanState own = mean_state(gamma, mean);
+
+    // One face point per lane.
+    if (lane < 3 * QF) {
+      const int k = lane / QF, q = lane % QF;
+      const std::int64_t slot = k * ne + e;
+      const unsigned code = E.code[k];
+      const bool self_left = code & 1u, boundary = E.nb[k] < 0;
+      const double nx = E.face[3 * k], ny = E.face[3 * k + 1];
+      // The face's left and right local edges, and the two bases' high modes
+      // (from 1) at the face's point q.
+      int le, re, flip;
+      const float *own_high, *other_high;
+      if constexpr (PATCH) {
+        const int jn = (code >> 1) & 3u;
+        const bool rev = code & 8u;
+        le = self_left ? k : jn;
+        re = self_left ? jn : k;
+        // The FP64 tables' flip is the edges' relative direction along the
+        // counter-clockwise parametrization; rev compares the edges' own point
+        // orders, and edge 2's points run against it.
+        flip = (rev ? 1 : 0) ^ (le == 2 ? 1 : 0) ^ (re == 2 ? 1 : 0);
+        const int qr = rev ? QF - 1 - q : q; // the right element's point
+        own_high = table.phi[k][self_left ? q : qr];
+        other_high = table.phi[jn][self_left ? qr : q];
+      } else {
+        le = (code >> 1) & 3u;
+        re = (code >> 3) & 3u;
+        flip = (code >> 5) & 1u;
+        const float *lb = &table.lb[le][0][0];
+        const float *rb = &table.rb[(le * 3 + re) * 2 + flip][0][0];
+        const float *own_basis = self_left ? lb : rb;
+        const float *other_basis = self_left ? rb : lb;
+        if (code & 0xC0u) {
+          const float *periodic =
+              a.boundary.basis32 + static_cast<std::int64_t>(a.tile.aux[slot]) * QF * M;
+          if (code & 0x40u)
+            own_basis = periodic;
+          else
+            other_basis = periodic;
+        }
+        own_high = own_basis + q * M + 1;
+        other_high = other_basis + q * M + 1;
+      }
+      double nmean[4] = {0.0, 0.0, 0.0, 0.0};
+      if (!boundary) {
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+          nmean[v] = E.across[k][v * M] * phi0;
+      }
+      // The face's left state is the reference of the perturbation form.
+      MeanState ml;
+      if (self_left || boundary)
+        ml = own;
+      else
+        ml = mean_state(gamma, nmean);
+      double fln[4];
+      mean_normal_flux(ml, nx, ny, fln);
+      const bool fp64 = !boundary && mean_jump(nmean[0], mean[0], nmean[3], mean[3]);
+      if (q == 0) {
+        float shift[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (!boundary && !self_left) {
+          double frn[4];
+          mean_normal_flux(own, nx, ny, frn);
+#pragma unroll
+          for (int v = 0; v < 4; ++v)
+            shift[v] = static_cast<float>(fln[v] - frn[v]);
+        }
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          E.fln[k][v] = fln[v];
+          E.shift[k][v] = shift[v];
+        }
+        E.fp64[k] = fp64;
+      }
+#pragma unroll
+      for (int m = 0; m < H; ++m)
+        E.basis[lane][m] = own_high[m];
+      if (fp64) {
+        const double *lb64 = &T64.lb[le][0][0];
+        const double *rb64 = &T64.rb[(le * 3 + re) * 2 + flip][0][0];
+        const double *own64 = self_left ? lb64 : rb64;
+        const double *other64 = self_left ? rb64 : lb64;
+        if (!PATCH && (code & 0xC0u)) {
+          const double *periodic =
+              a.mesh.donor_basis + static_cast<std::int64_t>(a.tile.aux[slot]) * QF * M;
+          if (code & 0x40u)
+            own64 = periodic;
+          else
+            other64 = periodic;
+        }
+        double f[4];
+        face_point_fp64<P>(gamma, E.own, 1, E.across[k], 1, false, self_left, own64 + q * M,
+                           other64 + q * M, nx, ny, f);
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          E.flux[lane][v] = f[v];
+          E.dflux[lane][v] = static_cast<float>(f[v] - fln[v]);
+        }
+      } else {
+        const Ref32 ref = ref32(ml);
+        float to[4], tn[4], dl[4], dr[4], fl[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          float s = 0.0f;
+#pragma unroll
+          for (int m = 0; m < H; ++m)
+            s = fmaf(static_cast<float>(E.own[v * M + m + 1]), own_high[m], s);
+          to[v] = s;
+        }
+        if (boundary) {
+#pragma unroll
+          for (int v = 0; v < 4; ++v)
+            dl[v] = dr[v] = to[v];
+        } else {
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            float s = 0.0f;
+#pragma unroll
+            for (int m = 0; m < H; ++m)
+              s = fmaf(static_cast<float>(E.across[k][v * M + m + 1]), other_high[m], s);
+            tn[v] = s;
+          }
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            const float jump =
+                static_cast<float>(self_left ? nmean[v] - mean[v] : mean[v] - nmean[v]);
+            dl[v] = self_left ? to[v] : tn[v];
+            dr[v] = jump + (self_left ? tn[v] : to[v]);
+          }
+        }
+        hllc_perturbed<PATCH>(ref, dl, dr, g1, gamma32, static_cast<float>(nx), static_cast<float>(ny), fl);
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+          E.dflux[lane][v] = fl[v];
+      }
+    }
+
+    // One volume point per lane (as the tile kernel).
+    {
+      const Ref32 bb = ref32(own);
+      const float fax = static_cast<float>(E.geo[0]), fay = static_cast<float>(E.geo[1]);
+      const float fbx = static_cast<float>(E.geo[2]), fby = static_cast<float>(E.geo[3]);
+      for (int q = lane; q < QV; q += kRoughLanes) {
+        float d[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          float s = 0.0f;
+#pragma unroll
+          for (int m = 0; m < H; ++m)
+            s = fmaf(static_cast<float>(E.own[v * M + m + 1]), T.phi[q][m], s);
+          d[v] = s;
+        }
+        const float inv = perturbation_rcp<PATCH>(fmaxf(bb.rho + d[0], kVacuumFraction * bb.rho));
+        const float du = (d[1] - bb.u * d[0]) * inv;
+        const float dv = (d[2] - bb.v * d[0]) * inv;
+        const float uu = bb.u + du, vv = bb.v + dv;
+        const float dmu = bb.mx * du + d[1] * uu + bb.my * dv + d[2] * vv;
+        const float dp = g1 * (d[3] - 0.5f * dmu);
+        const float dep = d[3] + dp;
+        const float fx[4] = {d[1], bb.mx * du + d[1] * uu + dp, bb.my * du + d[2] * uu,
+                             bb.h * du + dep * uu};
+        const float fy[4] = {d[2], bb.mx * dv + d[1] * vv, bb.my * dv + d[2] * vv + dp,
+                             bb.h * dv + dep * vv};
+        const float wq = T.w[q];
+        const float wby = wq * fby, wbx = wq * fbx, wax = wq * fax, way = wq * fay;
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          E.volume[q][v] = wby * fx[v] - wbx * fy[v];
+          E.volume[q][4 + v] = wax * fy[v] - way * fx[v];
+        }
+      }
+    }
+    __syncwarp();
+
+    // One coefficient after another per lane: its residual in the tile
+    // kernel's order, and the Shu-Osher combination.
+    const double inv = E.geo[4];
+    const double dt = a.case_dt ? a.case_dt[case_id] : (a.dt ? *a.dt : a.dt_value);
+#pragma unroll
+    for (int c = 0; c < OWN; ++c) {
+      const int i = c * kRoughLanes + lane;
+      if (i >= 4 * M)
+        break;
+      const int v = i / M, m = i % M;
+      float racc = 0.0f;
+      double r0 = 0.0;
+      if (m > 0)
+        for (int q = 0; q < QV; ++q)
+          racc = fmaf(T.dxi[q][m - 1], E.volume[q][v], fmaf(T.deta[q][m - 1], E.volume[q][4 + v], racc));
+#pragma unroll 1
+      for (int k = 0; k < 3; ++k) {
+        const unsigned code = E.code[k];
+        const bool self_left = code & 1u;
+        // The face's left local edge (its weights), and whether this element
+        // lifts its points in the order opposite to the face's.
+        const int le = PATCH && self_left ? k : (code >> 1) & 3u;
+        const bool reversed = PATCH && !self_left && (code & 8u);
+        const float *weights;
+        if constexpr (PATCH)
+          weights = table.w[le];
+        else
+          weights = table.ew[le];
+        const double scale = E.face[3 * k + 2];
+        const float fscale = static_cast<float>(scale);
+        if (m > 0) {
+#pragma unroll
+          for (int i = 0; i < QF; ++i) {
+            const int q = reversed ? QF - 1 - i : i;
+            const float wq = weights[q];
+            const float wsc = (self_left ? -wq : wq) * fscale;
+            const float fl = E.dflux[k * QF + q][v];
+            const float value = wsc * (self_left ? fl : fl + E.shift[k][v]);
+            racc = fmaf(value, E.basis[k * QF + q][m - 1], racc);
+          }
+        } else {
+          const double sgn = self_left ? -1.0 : 1.0;
+          if (E.fp64[k]) {
+            double mode0 = 0.0;
+#pragma unroll
+            for (int q = 0; q < QF; ++q)
+              mode0 = fma(T64.ew[le][q], E.flux[k * QF + q][v], mode0);
+            r0 += sgn * scale * phi0 * mode0;
+          } else {
+            float acc = 0.0f;
+#pragma unroll
+            for (int q = 0; q < QF; ++q)
+              acc = fmaf(weights[q], E.dflux[k * QF + q][v], acc);
+            const double mode0 = E.fln[k][v] * c_edge_wsum<P>[le] + static_cast<double>(acc);
+            r0 += sgn * scale * phi0 * mode0;
+          }
+        }
+      }
+      const std::int64_t idx = i * ne + e;
+      const double cur = E.own[i];
+      const double rr = (m == 0 ? r0 : static_cast<double>(racc)) * inv;
+      double o;
+      if (a.stage == 0)
+        o = cur + dt * rr;
+      else if (a.stage == 1)
+        o = 0.75 * u0[c] + 0.25 * (cur + dt * rr);
+      else
+        o = (1.0 / 3.0) * u0[c] + (2.0 / 3.0) * (cur + dt * rr);
+      if (valid)
+        a.out[idx] = o;
+      E.next[i] = o;
+    }
+    __syncwarp();
+    if (lane == 0 && valid) {
+      if (a.speed_max) {
+        const double scale = 1.0 / sqrt(2.0);
+        const double sa[4] = {__dmul_rn(scale, E.next[0]), __dmul_rn(scale, E.next[M]),
+                              __dmul_rn(scale, E.next[2 * M]), __dmul_rn(scale, E.next[3 * M])};
+        bool physical = true;
+        const double speed = cfl_speed(gamma, sa, 2, physical);
+        if (physical)
+          atomicMax(a.speed_max + case_id,
+                    static_cast<unsigned long long>(__double_as_longlong(speed)));
+        else
+          raise_error(a.error, kNonPhysicalAverage, e);
+      }
+      if (a.suspects) {
+        double mode0[4], reach[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          mode0[v] = E.next[v * M];
+          reach[v] = 0.0;
+#pragma unroll
+          for (int m = 1; m < M; ++m)
+            reach[v] += fabs(E.next[v * M + m]) * a.floors.bound[m];
+        }
+        if (!positivity_clear(gamma, a.floors, mode0, reach))
+          a.suspects[atomicAdd(a.suspect_count, 1)] = static_cast<std::int32_t>(e);
+      }
+      if (a.sense) {
+        double total = 0.0, high = 0.0;
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+          total += E.next[m] * E.next[m];
+          if (m >= a.highest_degree_begin)
+            high += E.next[m] * E.next[m];
+        }
+        const bool troubled = !(total == 0.0 || high / total <= a.threshold);
+        a.flags[e] = troubled ? 1 : 0;
+        if (troubled)
+          a.troubled[atomicAdd(a.troubled_count, 1)] = static_cast<std::int32_t>(e);
+      }
+    }
+    __syncwarp(); // the next element's coefficients may land
+  }
 }
 
 void check(cudaError_t rc, const char *what) {
@@ -2789,6 +2832,7 @@ template <int P, int R> void upload_mixed() {
     t.w[q] = static_cast<float>(0.5 * rule.w[q]);
   }
   check(cudaMemcpyToSymbol(c_mix<P, R>, &t, sizeof(t)), "upload mixed volume table");
+  check(cudaMemcpyToSymbol(g_mix<P, R>, &t, sizeof(t)), "upload mixed volume table");
   static FaceTable<P, double> f;
   fill_face_table<P, double>(f);
   double wsum[3];
@@ -2807,6 +2851,7 @@ template <int P, int R> void upload_mixed() {
       pt.w[le][q] = static_cast<float>(f.ew[le][q]);
     }
   check(cudaMemcpyToSymbol(c_patch<P>, &pt, sizeof(pt)), "upload patch edge table");
+  check(cudaMemcpyToSymbol(g_patch<P>, &pt, sizeof(pt)), "upload patch edge table");
 }
 
 template <int P, int R> void stage_mixed(const StageArgs &a, cudaStream_t s) {
@@ -2874,20 +2919,22 @@ template <int P, int R> constexpr std::size_t rough_smem_bytes() {
   return sizeof(RoughElement<P, R>) * (kRoughThreads / kRoughLanes);
 }
 
-template <int P, int R> void rough_opt_in() {
+template <int P, int R, bool PATCH> void rough_opt_in() {
   static bool opted_in[64] = {};
-  smem_opt_in(euler_tri_rough<P, R>, rough_smem_bytes<P, R>(),
-              sizeof(FaceTable<P, float>) + sizeof(MixedVolume<P, R>), opted_in);
+  smem_opt_in(euler_tri_rough<P, R, PATCH>, rough_smem_bytes<P, R>(),
+              sizeof(FaceTable<P, float>) + sizeof(MixedVolume<P, R>) + sizeof(FaceTable<P, double>),
+              opted_in);
 }
 
 // The second pass over the rough list, whose length only the device knows: up
 // to eight blocks (64 elements) per SM, which return at once beyond it and go
 // round where it is longer.
-template <int P, int R> void launch_rough(const StageArgs &a, cudaStream_t s) {
-  rough_opt_in<P, R>();
+template <int P, int R, bool PATCH> void launch_rough(const StageArgs &a, cudaStream_t s) {
+  rough_opt_in<P, R, PATCH>();
   constexpr int groups = kRoughThreads / kRoughLanes;
   const std::int64_t blocks = std::min<std::int64_t>((a.mesh.ne + groups - 1) / groups, 148 * 8);
-  euler_tri_rough<P, R><<<static_cast<unsigned>(blocks), kRoughThreads, rough_smem_bytes<P, R>(), s>>>(a);
+  euler_tri_rough<P, R, PATCH>
+      <<<static_cast<unsigned>(blocks), kRoughThreads, rough_smem_bytes<P, R>(), s>>>(a);
 }
 
 // The FP32 pass over all tiles, then (with a rough list) the pass over the
@@ -2909,7 +2956,7 @@ void stage_tile(const StageArgs &a, cudaStream_t s) {
     euler_tri_tile_mixed<P, R, TILE, MINB>
         <<<static_cast<unsigned>(blocks), TILE, tile_smem<P, TILE>(), s>>>(a);
   if (a.rough)
-    launch_rough<P, R>(a, s);
+    launch_rough<P, R, false>(a, s);
 }
 
 // The persistent tile kernel's attributes and its grid: every CTA resident
@@ -2947,19 +2994,20 @@ void stage_tile_persistent(const StageArgs &a, cudaStream_t s) {
   euler_tri_tile_persistent<P, R, TILE, MINB>
       <<<static_cast<unsigned>(blocks), TILE, tile_smem<P, TILE>(), s>>>(a);
   if (a.rough)
-    launch_rough<P, R>(a, s);
+    launch_rough<P, R, false>(a, s);
 }
 
 template <int P, int R, int TILE, int MINB, bool MMA> void patch_opt_in() {
-  static bool opted_in[64] = {}, opted_in_islands[64] = {};
+  static bool opted_in[64] = {}, opted_in_limited[64] = {};
   smem_opt_in(euler_tri_patch<P, R, TILE, MINB, MMA, false>, PatchSmem<P, R, TILE, MMA>::bytes,
               sizeof(PatchEdge<P>) + sizeof(int), opted_in);
   if constexpr (!MMA)
     smem_opt_in(euler_tri_patch<P, R, TILE, MINB, false, true>, PatchSmem<P, R, TILE, false>::bytes,
-                sizeof(PatchEdge<P>) + sizeof(int), opted_in_islands);
+                sizeof(PatchEdge<P>) + sizeof(int) + TILE, opted_in_limited);
 }
 
-// The patch kernel over all patches (no rough pass: runs without the limiter).
+// The patch kernel over all patches, then (with a rough list) the pass over the
+// elements it left.
 template <int P, int R, int TILE, int MINB, bool MMA = false>
 void stage_patch(const StageArgs &a, cudaStream_t s) {
   if (!a.patch.nbr)
@@ -2972,9 +3020,9 @@ void stage_patch(const StageArgs &a, cudaStream_t s) {
     launch_dependent(euler_tri_patch<P, R, TILE, MINB, MMA, false>,
                      static_cast<unsigned>(blocks), TILE, PatchSmem<P, R, TILE, MMA>::bytes, s, a);
   } else if constexpr (!MMA) {
-    // With the limiter: faces across jumps of the means in FP64, inline.
     launch_dependent(euler_tri_patch<P, R, TILE, MINB, false, true>,
                      static_cast<unsigned>(blocks), TILE, PatchSmem<P, R, TILE, false>::bytes, s, a);
+    launch_rough<P, R, true>(a, s);
   } else {
     throw std::invalid_argument("patch kernel with the tensor-core volume: runs without the"
                                 " limiter");
@@ -2992,10 +3040,10 @@ template <int P, int R> struct StageTile {
     case 5: stage_tile<P, R, 96, 5, true>(a, s); break;
     case 6: stage_tile<P, R, 128, 4, true>(a, s); break;
     case 7: stage_tile<P, R, 128, 3, true>(a, s); break;
-    case 8: stage_patch<P, R, 128, 4>(a, s); break;
+    case 8: stage_patch<P, R, 256, 2>(a, s); break;
     case 9: stage_patch<P, R, 128, 5>(a, s); break;
     case 10: stage_patch<P, R, 64, 8>(a, s); break;
-    case 11: stage_patch<P, R, 64, 10>(a, s); break;
+    case 11: stage_patch<P, R, 192, 3>(a, s); break;
     case 12: stage_patch<P, R, 128, 4, true>(a, s); break;
     case 13: stage_patch<P, R, 128, 5, true>(a, s); break;
     case 14: stage_tile_persistent<P, R, 128, 4>(a, s); break;
@@ -3015,15 +3063,15 @@ template <int P, int R> struct PrepareTile {
     shared_opt_in<P, R, 96, 5>();
     shared_opt_in<P, R, 128, 4>();
     shared_opt_in<P, R, 128, 3>();
-    patch_opt_in<P, R, 128, 4, false>();
     patch_opt_in<P, R, 128, 5, false>();
     patch_opt_in<P, R, 64, 8, false>();
-    patch_opt_in<P, R, 64, 10, false>();
+    patch_opt_in<P, R, 256, 2, false>();
+    patch_opt_in<P, R, 192, 3, false>();
     patch_opt_in<P, R, 128, 4, true>();
     patch_opt_in<P, R, 128, 5, true>();
     persistent_prepare<P, R, 128, 4>();
     persistent_prepare<P, R, 256, 2>();
-    rough_opt_in<P, R>();
+    rough_opt_in<P, R, false>();
   }
 };
 

@@ -739,9 +739,9 @@ private:
   // state into scratch (u^n is read, not written; sensing off) and keeps the
   // fastest, per polynomial order, rule order and mesh size class.
   void tune_mixed(StageArgs a) {
-    // With the limiter (flows with discontinuities) only the tile kernel,
-    // whose second pass evaluates faces at discontinuities in FP64, competes;
-    // the patch kernel's shapes only where its edge arrays were built.
+    // With the limiter (flows with discontinuities) the face-centric kernels,
+    // which have no FP64 pass, do not compete; the patch kernel's shapes only
+    // where its edge arrays were built.
     const int base = tile_ok_ && limiting_ ? 1 : 0;
     std::vector<int> kernels; // kernel_ values: 0 face-centric, 1 + shape
     if (!base)
@@ -781,6 +781,26 @@ private:
     for (std::size_t i = 0; i < kernels.size(); ++i)
       tuning_.ms[kernels[i]] = timed.ms[i] / 3.0;
     kernel_ = kernels[timed.choice];
+    if (base) {
+      // With the limiter the choice stays within one family at
+      //   P3  the tile kernels.  (The patch kernel is 14% faster a stage at
+      //       500,000 triangles, but next to strong shocks, where perturbations
+      //       are as large as the means, the families' FP32 sums differ by up to
+      //       1e-7 of the state after a few steps: P3 keeps its rounding.)
+      //   P2  the patch kernel: as fast below 65,536 elements, where a stage is
+      //       latency (30 us), 10-14% faster above.
+      //   P1  the patch kernel below 65,536 elements (equal there), both above.
+      double best = 0.0;
+      for (std::size_t i = 0; i < kernels.size(); ++i) {
+        const bool patch = euler_tri_tile_is_patch(kernels[i] - 1);
+        if (p_ == 3 ? patch : !patch && patch_ok_ && (p_ == 2 || ne_ < 65536))
+          continue;
+        if (best == 0.0 || timed.ms[i] < best) {
+          best = timed.ms[i];
+          kernel_ = kernels[i];
+        }
+      }
+    }
     tuning_.choice = kernel_;
   }
 
