@@ -53,9 +53,11 @@ def test_euler_stage_not_finite(oracle, value):
         assert np.array_equal(g.get_state(), c, equal_nan=True)
 
 
-# (order, sizes around the limit of one element per thread)
-@pytest.mark.parametrize("p,n", [(0, 1), (2, 31), (2, 32), (2, 400), (2, 1023), (2, 1024), (3, 511),
-                                 (3, 512), (6, 300)])
+# (order, sizes around the limits of one element per thread and of the clusters of
+# four and eight blocks; 19 steps: the halo is exchanged every eighth)
+@pytest.mark.parametrize("p,n", [(0, 1), (2, 31), (2, 32), (2, 95), (2, 96), (0, 97),
+                                 (2, 400), (2, 416), (2, 417), (2, 1023), (2, 1024), (1, 2345),
+                                 (3, 511), (3, 512), (3, 1952), (3, 1953), (6, 300)])
 @pytest.mark.parametrize("ends,speed", [(("periodic", "periodic"), 0.7),
                                         (("inflow", "outflow"), 0.7),
                                         (("outflow", "inflow"), -0.9),
@@ -70,7 +72,7 @@ def test_scalar_run_limits(p, n, ends, speed):
                               inflow=(0.8, -0.3)) as g:
             g.set_state(c)
             run = g.run_resident if resident else g.run
-            out.append((run(0.3, 0.0, 1.0, 7), g.get_state()))
+            out.append((run(0.3, 0.0, 1.0, 19), g.get_state()))
     assert out[0][0] == out[1][0]
     assert np.array_equal(out[0][1], out[1][1])
 

@@ -507,8 +507,7 @@ template <int V, int P> __global__ void __launch_bounds__(512) line_run_f64(Line
 }
 
 // The same run with one element per thread, for meshes of at most
-// kLineRunThreads - 1 elements (the 400-cell advection run, for one): the
-// stage's coefficients stay in registers over the whole run (and u^n too, for
+// LineRunLimit::threads - 1 elements: the stage's coefficients stay in registers over the whole run (and u^n too, for
 // scalar advection; in the thread's column of shared memory for Euler), and
 // only what a neighbour needs passes through shared memory: the one trace an
 // upwind flux reads, or Euler's right traces and face fluxes.  Bound by the
@@ -720,6 +719,150 @@ __global__ void __launch_bounds__(LineRunLimit<V, P>::threads) line_run_register
   }
 }
 
+// The advection run spread over a cluster of four blocks.  An upwind stage reads
+// one element upstream only, so a block that also holds the kRunHalo elements
+// upstream of its chunk can take kRunHalo / 3 steps on its own, the halo's
+// outermost element going stale with each stage; then the blocks exchange their
+// downstream ends through distributed shared memory, behind one cluster barrier
+// (which costs more than a stage, so every stage would not pay: measured twice
+// as slow).  Per stage a block has a quarter of the warps: at 400 cells one per
+// sub-core instead of three or four, and the stage is its chain of dependent
+// FP64 operations and a barrier of four warps instead of the pipe's 464 cycles.
+// (The block count is a template argument: read from the grid it cost 8%.)
+// The elements' arithmetic is the one-block kernel's.  400 cells at P2: 0.34 ->
+// 0.18 us per stage (0.67 us when every block exchanged every stage).
+constexpr int kRunHalo = 24;
+
+template <int P, int BLOCKS>
+__global__ void __launch_bounds__(LineRunLimit<1, P>::threads) line_run_cluster_f64(LineRunArgs r) {
+  constexpr int M = P + 1;
+  extern __shared__ double cluster_smem[]; // traces [2][T], then edges [2][M][kRunHalo]
+  const int n = static_cast<int>(r.stage.ne), t = threadIdx.x, T = blockDim.x;
+  const LineTable &table = r.stage.table;
+  const double *lb = table.lb, *rb = table.rb;
+  const double speed = r.stage.speed;
+  const bool forward = speed >= 0.0;
+  const int inflow_kind = forward ? r.stage.left_kind : r.stage.right_kind;
+  const double inflow_value = forward ? r.stage.left_value : r.stage.right_value;
+  unsigned rank;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  // Positions along the flow: element s is the s-th from the inflow end; this
+  // block's chunk is [begin, end), its threads hold [begin - kRunHalo, end).
+  const int begin = static_cast<int>(rank) * n / BLOCKS;
+  const int end = (static_cast<int>(rank) + 1) * n / BLOCKS;
+  const int s = begin - kRunHalo + t;
+  const bool wraps = inflow_kind == 0;
+  const bool holds = s < end && (s >= 0 || wraps);
+  const int along = s < 0 ? s + n : s;
+  const int e = forward ? along : n - 1 - along;
+  double *edges = cluster_smem + 2 * T;
+  double c[M], un[M];
+#pragma unroll
+  for (int m = 0; m < M; ++m)
+    c[m] = holds ? r.state[m * n + e] : 0.0;
+  const double inv = holds ? r.stage.inv_jacobian[e] : 0.0;
+  const bool at_inflow = s == 0 && !wraps;
+  // The upstream block's edges (the last block's for the first, across the period).
+  unsigned upstream_edges;
+  {
+    const unsigned local = static_cast<unsigned>(__cvta_generic_to_shared(edges));
+    const unsigned from = (rank + BLOCKS - 1) % BLOCKS;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(upstream_edges) : "r"(local), "r"(from));
+  }
+  double time = r.start_time;
+  unsigned long long steps = 0;
+  unsigned long long status = 0;
+  int buffer = 0, edge_buffer = 0, fresh = kRunHalo / 3;
+  while (time < r.end_time && steps < r.max_steps) {
+    const double remaining = r.end_time - time;
+    const double dt =
+        r.fixed_dt > 0.0 ? (remaining < r.fixed_dt ? remaining : r.fixed_dt) : remaining;
+    if (dt <= 0.0 || time + dt == time) {
+      status = 1; // every thread of the cluster finds the same dt
+      break;
+    }
+    if (fresh == 0) {
+      // The halo is stale: the downstream end of every chunk to its edges, and
+      // after the barrier the upstream block's into the halo.  Two buffers:
+      // a block rewrites one only after the next barrier, behind every read.
+      double *mine = edges + edge_buffer * M * kRunHalo;
+      const int at = s - (end - kRunHalo);
+      if (at >= 0 && s < end) {
+#pragma unroll
+        for (int m = 0; m < M; ++m)
+          mine[m * kRunHalo + at] = c[m];
+      }
+      asm volatile("barrier.cluster.arrive.release.aligned;\n"
+                   "barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+      if (t < kRunHalo && holds) {
+#pragma unroll
+        for (int m = 0; m < M; ++m)
+          asm volatile("ld.shared::cluster.f64 %0, [%1];"
+                       : "=d"(c[m])
+                       : "r"(upstream_edges +
+                             8u * static_cast<unsigned>((edge_buffer * M + m) * kRunHalo + t))
+                       : "memory");
+      }
+      edge_buffer ^= 1;
+      fresh = kRunHalo / 3;
+    }
+    --fresh;
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+      un[m] = c[m];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      double *traces = cluster_smem + buffer * T;
+      buffer ^= 1;
+      const double own = trace_of(c, forward ? rb : lb);
+      traces[t] = own;
+      double rhs[M];
+#pragma unroll
+      for (int m = 0; m < M; ++m)
+        rhs[m] = 0.0;
+      if constexpr (P > 0) {
+#pragma unroll
+        for (int q = 0; q < P; ++q) {
+          const double wf = table.w[q] * (speed * trace_of(c, table.phi[q]));
+#pragma unroll
+          for (int m = 1; m < M; ++m)
+            rhs[m] += wf * table.dphi[q][m];
+        }
+        rhs[0] = 0.0 + 0.0 * rhs[1]; // (mode 0's derivative is zero)
+      } else {
+        rhs[0] += table.w[0] * (speed * trace_of(c, table.phi[0])) * table.dphi[0][0];
+      }
+      __syncthreads();
+      double upstream = t > 0 ? traces[t - 1] : 0.0; // (t = 0 is halo: stale)
+      if (at_inflow)
+        upstream = inflow_kind == 1 ? inflow_value : trace_of(c, forward ? lb : rb);
+      const double in = speed * upstream, out = speed * own;
+      const double before = forward ? in : out, after = forward ? out : in;
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        rhs[m] += lb[m] * before;
+        rhs[m] -= rb[m] * after;
+        c[m] = combine(k, un[m], c[m], dt, rhs[m] * inv);
+      }
+    }
+    time += dt;
+    ++steps;
+  }
+  if (holds && s >= begin) {
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+      r.state[m * n + e] = c[m];
+  }
+  if (rank == 0 && t == 0) {
+    r.result[0] = steps;
+    r.result[1] = static_cast<unsigned long long>(__double_as_longlong(time));
+    r.result[2] = status;
+  }
+  // No block leaves while another may still read its edges.
+  asm volatile("barrier.cluster.arrive.release.aligned;\n"
+               "barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+
 template <int V, int P> void launch(const LineStageArgs &a, cudaStream_t s) {
   if constexpr (V == 4) {
     constexpr int E = kLineBlock - 1;
@@ -756,10 +899,46 @@ template <typename Kernel> void run_opt_in(Kernel kernel, std::size_t bytes, boo
   opted_in[device] = true;
 }
 
-// One element (and, for Euler, one face) per thread where the block has the
-// threads and the registers for it; else the elements of a thread in turn.
+// Advection from 96 cells on (four chunks of a halo's length): the cluster, of
+// four blocks while a chunk and its halo fit in four warps, of eight above.  P2,
+// us per stage, one block and the cluster: 0.220 and 0.179 at 96 cells, 0.244 and
+// 0.179 at 128, 0.285 and 0.181 at 300; at 480 cells 0.346, 0.219 with four
+// blocks and 0.181 with eight; P1 at 2000: 1.45, 0.30 and 0.22.  Else one element
+// (and, for Euler, one face) per thread where the block has the threads and the
+// registers for it; else the elements of a thread in turn.
+constexpr int kRunClusterFrom = 96, kRunCluster4To = 416;
+
+template <int P, int BLOCKS> void launch_run_cluster(const LineRunArgs &r, cudaStream_t s) {
+  const auto threads =
+      static_cast<unsigned>(((r.stage.ne + BLOCKS - 1) / BLOCKS + kRunHalo + 31) / 32 * 32);
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(BLOCKS);
+  config.blockDim = dim3(threads);
+  config.dynamicSmemBytes = sizeof(double) * (2 * threads + 2 * (P + 1) * kRunHalo);
+  config.stream = s;
+  cudaLaunchAttribute attribute[1];
+  attribute[0].id = cudaLaunchAttributeClusterDimension;
+  attribute[0].val.clusterDim.x = BLOCKS;
+  attribute[0].val.clusterDim.y = 1;
+  attribute[0].val.clusterDim.z = 1;
+  config.attrs = attribute;
+  config.numAttrs = 1;
+  if (cudaLaunchKernelEx(&config, line_run_cluster_f64<P, BLOCKS>, r) != cudaSuccess)
+    throw std::runtime_error("resident run: cluster launch failed");
+}
+
 template <int V, int P> void launch_run(const LineRunArgs &r, cudaStream_t s) {
   constexpr int limit = LineRunLimit<V, P>::threads;
+  if constexpr (V == 1) {
+    if (r.stage.ne >= kRunClusterFrom && r.stage.ne <= kRunCluster4To) {
+      launch_run_cluster<P, 4>(r, s);
+      return;
+    }
+    if (r.stage.ne > kRunCluster4To && (r.stage.ne + 7) / 8 + kRunHalo <= limit) {
+      launch_run_cluster<P, 8>(r, s);
+      return;
+    }
+  }
   if constexpr (limit > 0) {
     if (r.stage.ne < limit) {
       static bool opted_in[64] = {};
