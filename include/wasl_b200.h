@@ -82,7 +82,7 @@ typedef struct {
                                 points at P1, P2, P3) */
   int mixed_kernel;          /* mixed form: 0 autotuned; 1 face-centric kernels (face pass
                                 + element pass); 2 + s the fused tile kernel in launch
-                                shape s (0..13, see wasl_gpu_tuning) */
+                                shape s (0..15, see wasl_gpu_tuning) */
   int positivity_all;        /* with limiting: 1 applies the positivity limiter to every
                                 element, not only troubled ones (not the reference's
                                 behaviour, cpp/src/limiting/euler_modal_limiter.cpp:81-96) */

@@ -350,7 +350,7 @@ StageArgs BatchSolver::stage_args(const Group &g, int stage) const {
   a.tile.nbr = g.tile_nbr.get();
   a.tile.code = g.tile_code.get();
   a.tile.aux = g.tile_aux.get();
-  // FP64 face islands at discontinuities (the rough pass), with the limiter.
+  // The elements at discontinuities, for the rough pass (FP64), with the limiter.
   a.rough = cfg_.limiting ? g.rough.get() : nullptr;
   a.rough_count = a.rough ? g.count.get() + 1 : nullptr;
   if (g.suspects.size() > 0) {
@@ -441,7 +441,8 @@ void BatchSolver::tune() {
 // join each runs on a stream of its own, so that one group's short launches
 // (lists of troubled and rough elements: a few blocks, all latency) run beside
 // another's stage kernel.  Group 0 keeps the handle's stream.  32 cases of 1,000
-// to 16,000 triangles, 16 steps: 15.6 -> 12.1 ms with the groups side by side.
+// to 16,000 triangles, 16 steps: 17.3 -> 12.4 ms with the groups side by side
+// (and the positivity pass over listed suspects).
 void BatchSolver::fork() {
   if (groups_.size() < 2)
     return;

@@ -86,8 +86,9 @@ __device__ __forceinline__ void eval_pair(const double (&c)[2][M], const double 
 // 131,072 elements) and by what does not overlap with it (the state's loads
 // and stores, the phases' barriers).  Against one thread per element (254
 // registers, 8 warps per SM, P3 spilling, each face's flux evaluated by both
-// its elements), per stage on a B200: P1 at 131,072 elements 54 -> 47 us, P2
-// 126 -> 94 us, P3 at 51,842 elements 150 -> 92 us.
+// its elements), per stage on a B200: P1 at 131,072 elements 58 -> 45 us, P2
+// 133 -> 94 us, P3 at 51,842 elements 165 -> 89 us; at 1,152 elements, P1 20 ->
+// 12 us and P2 36 -> 21 us.
 //   * Two lanes per element (each half the variables: half the registers, twice
 //     the warps per SM) share out the points of the volume rule, so no flux is
 //     evaluated twice for it; duplicated are only the gradients' few products.

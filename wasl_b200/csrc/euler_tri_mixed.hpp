@@ -28,7 +28,7 @@ namespace wasl_b200 {
 //  11: 192 elements, sized for 3 CTAs per SM
 // (larger patches have fewer faces to outside elements, which both patches
 // evaluate: P3 at 500,000 triangles 341 us a stage in shape 8 against 371 with
-// 128 elements at the same registers, at 45,602 triangles 37 us in shape 11
+// 128 elements at the same registers (310 with the point loops rolled), at 45,602 triangles 37 us in shape 11
 // against 45; 64 elements suit meshes that larger patches leave SMs idle on)
 // and of the patch kernel with its volume term on the tensor cores:
 //  12: 128 elements, <= 128 registers

@@ -645,7 +645,7 @@ private:
     a.patch.nbr = d_patch_nbr_.get();
     a.patch.info = d_patch_info_.get();
     a.patch.geo = d_patch_geo_.get();
-    // FP64 face islands at discontinuities (the rough pass), with the limiter.
+    // The elements at discontinuities, for the rough pass (FP64), with the limiter.
     a.rough = limiting_ ? d_rough_.get() : nullptr;
     a.rough_count = a.rough ? d_count_.get() + 1 : nullptr;
     a.dt = dt_device;

@@ -330,8 +330,7 @@ void launch_batch_speed(const double *state, std::int64_t ne, int M, double gamm
 constexpr int kTileShapeCount = 16;
 int euler_tri_tile_shapes();
 int euler_tri_tile_elements(int shape);
-// Shapes of the patch kernel (StageArgs::patch; no rough pass, so runs
-// without the limiter only).
+// Shapes of the patch kernel (StageArgs::patch).
 bool euler_tri_tile_is_patch(int shape);
 // Shapes that run with the limiter (all but the patch kernel with its volume
 // term on the tensor cores).

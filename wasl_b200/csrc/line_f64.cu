@@ -507,12 +507,12 @@ template <int V, int P> __global__ void __launch_bounds__(512) line_run_f64(Line
 }
 
 // The same run with one element per thread, for meshes of at most
-// LineRunLimit::threads - 1 elements: the stage's coefficients stay in registers over the whole run (and u^n too, for
-// scalar advection; in the thread's column of shared memory for Euler), and
-// only what a neighbour needs passes through shared memory: the one trace an
-// upwind flux reads, or Euler's right traces and face fluxes.  Bound by the
-// FP64 pipe of one SM and the barriers (one per advection stage, two per Euler
-// stage).  400 cells at P2: 0.67 -> 0.34 us per stage against the kernel above,
+// LineRunLimit::threads - 1 elements: the stage's coefficients stay in registers
+// over the whole run (and u^n too, for scalar advection; in the thread's column
+// of shared memory for Euler), and only what a neighbour needs passes through
+// shared memory: the one trace an upwind flux reads, or Euler's right traces and
+// face fluxes.  Bound by the FP64 pipe of one SM and the barriers (one per
+// advection stage, two per Euler stage).  400 cells at P2: 0.67 -> 0.34 us per stage against the kernel above,
 // which keeps the three state buffers in shared memory, evaluates every trace
 // twice and reads each coefficient it needs.
 template <int V, int P> struct LineRunLimit {
