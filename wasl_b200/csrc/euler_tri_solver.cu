@@ -789,11 +789,15 @@ private:
       //       1e-7 of the state after a few steps: P3 keeps its rounding.)
       //   P2  the patch kernel: as fast below 65,536 elements, where a stage is
       //       latency (30 us), 10-14% faster above.
-      //   P1  the patch kernel below 65,536 elements (equal there), both above.
+      //   P1  the patch kernel below 65,536 elements (equal there), the tile
+      //       kernels above: 8% slower at 180,000 elements (811 against 743 us
+      //       for four steps), but there, too, the families differ by 3e-8 next
+      //       to strong shocks.
       double best = 0.0;
       for (std::size_t i = 0; i < kernels.size(); ++i) {
         const bool patch = euler_tri_tile_is_patch(kernels[i] - 1);
-        if (p_ == 3 ? patch : !patch && patch_ok_ && (p_ == 2 || ne_ < 65536))
+        const bool patches = p_ == 2 || (p_ == 1 && ne_ < 65536);
+        if (patch_ok_ && patch != patches)
           continue;
         if (best == 0.0 || timed.ms[i] < best) {
           best = timed.ms[i];
