@@ -848,6 +848,11 @@ __global__ void __launch_bounds__(LineRunLimit<1, P>::threads) line_run_cluster_
     time += dt;
     ++steps;
   }
+  // The chunks go back to r.state only when every block has loaded its halo from
+  // there (a run of up to kRunHalo / 3 steps passes no barrier above), and no
+  // block leaves while another may still read its edges.
+  asm volatile("barrier.cluster.arrive.release.aligned;\n"
+               "barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
   if (holds && s >= begin) {
 #pragma unroll
     for (int m = 0; m < M; ++m)
@@ -858,9 +863,6 @@ __global__ void __launch_bounds__(LineRunLimit<1, P>::threads) line_run_cluster_
     r.result[1] = static_cast<unsigned long long>(__double_as_longlong(time));
     r.result[2] = status;
   }
-  // No block leaves while another may still read its edges.
-  asm volatile("barrier.cluster.arrive.release.aligned;\n"
-               "barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
 
 template <int V, int P> void launch(const LineStageArgs &a, cudaStream_t s) {
