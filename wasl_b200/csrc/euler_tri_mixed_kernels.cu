@@ -788,11 +788,21 @@ __device__ __forceinline__ void tile_finish(const StageArgs &a, std::int64_t e, 
 // An element with a face across which the two cell means jump (kFp64Jump; a
 // test both elements of the face make alike) is not computed here but appended
 // to the rough list (when a.rough is set) for euler_tri_rough.
+//
+// The tile kernels' face points one at a time (rolled), where the unrolled
+// points would not fit the instruction cache: with many warps per SM at P3 485 ->
+// 435 us a stage at 500,000 triangles, at P2 216 -> 207.  At P1 they do fit (41
+// against 43 us at 180,000 triangles), and the shape without a register cap, which
+// meshes of a few warps per SM take, is bound by one warp's chain, which the
+// unrolled points shorten (P3: 30 against 35 us a stage at 7,200 triangles).
+template <int P, int MINB> constexpr bool kTileRolled = P > 1 && MINB > 1;
+
 // One element's share of the tile kernel's stage, once its tile is staged:
 // volume term, the three faces, and the finish.  An element of the FP32 pass
 // with a face across a jump of the means returns early (handed to the rough
-// pass).  Shared by the one-tile-per-CTA and the persistent kernels.
-template <int P, int R, int TILE>
+// pass).  Shared by the one-tile-per-CTA and the persistent kernels.  ROLLED: one
+// face point at a time (kTileRolled).
+template <int P, int R, int TILE, bool ROLLED>
 __device__ __forceinline__ void tile_element(const StageArgs &a, const FaceTable<P, float> &table,
                                              const double (*sstate)[TILE], int t,
                                              std::int64_t e, std::int64_t first,
@@ -800,6 +810,7 @@ __device__ __forceinline__ void tile_element(const StageArgs &a, const FaceTable
   using S = TriShape<P>;
   constexpr int M = S::M, QV = MixedVolume<P, R>::QV, QF = S::QF, H = M - 1;
   constexpr double phi0 = 0.70710678118654752440;
+  constexpr int kPoints = ROLLED ? 1 : QF;
   const std::int64_t ne = a.mesh.ne;
   const double *__restrict__ in = a.in;
   double mean[4];
@@ -948,9 +959,7 @@ __device__ __forceinline__ void tile_element(const StageArgs &a, const FaceTable
     const float fscale = static_cast<float>(scale);
     const double sgn = self_left ? -1.0 : 1.0;
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    // (Rolled: the instruction cache again, 485 -> 435 us a stage at P3, 216 -> 207 at
-    // P2, 500,000 triangles.)
-#pragma unroll 1
+#pragma unroll kPoints
     for (int q = 0; q < QF; ++q) {
       float to[4], tn[4], dl[4], dr[4], fl[4];
       high_trace<P>(ch, own_basis + q * M, to);
@@ -1035,7 +1044,7 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_tile_mixed(const StageAr
   __syncthreads();
   if (!active)
     return;
-  tile_element<P, R, TILE>(a, table, sstate, t, e, first, count, case_id);
+  tile_element<P, R, TILE, kTileRolled<P, MINB>>(a, table, sstate, t, e, first, count, case_id);
 }
 
 // The FP32 pass of the tile kernel as a persistent kernel: each CTA loads the
@@ -1086,7 +1095,7 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_tile_persistent(const St
     asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncthreads(); // the tile is staged (and, the first time, the tables)
     if (active)
-      tile_element<P, R, TILE>(a, table, sstate, t, e, first, count, case_id);
+      tile_element<P, R, TILE, kTileRolled<P, MINB>>(a, table, sstate, t, e, first, count, case_id);
     __syncthreads(); // every element is done with the tile before the next one lands
   }
 }
