@@ -136,12 +136,13 @@ __global__ void __launch_bounds__(128, kStageBlocks<P>) euler_tri_stage_f64(cons
   const double gamma = a.gamma;
   // This lane's rows: variables 2 half and 2 half + 1.
   const std::int64_t rows = static_cast<std::int64_t>(2 * half) * M * ne;
-  const double *__restrict__ in = a.in + rows;
+  const double *in = a.in + rows;
 
   // Launched as a programmatic dependent of the launch before it, the block may
   // be here while that one drains: the face table is constant, and the state is
   // not touched before that launch has completed.  (Launched plainly, both
-  // instructions are no-ops.)
+  // instructions are no-ops.)  The state is read through ordinary loads: the
+  // read-only path wants data that nothing writes while the kernel is resident.
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   {
     const double *src = static_cast<const double *>(a.face_table);
@@ -198,7 +199,7 @@ __global__ void __launch_bounds__(128, kStageBlocks<P>) euler_tri_stage_f64(cons
         double sum[QF];
 #pragma unroll
         for (int m = 0; m < M; ++m) {
-          const double x = __ldg(in + (static_cast<std::int64_t>(v) * M + m) * ne + nb);
+          const double x = in[(static_cast<std::int64_t>(v) * M + m) * ne + nb];
 #pragma unroll
           for (int q = 0; q < QF; ++q)
             sum[q] = m == 0 ? x * ob[q][0] : sum[q] + x * ob[q][m];
@@ -218,7 +219,7 @@ __global__ void __launch_bounds__(128, kStageBlocks<P>) euler_tri_stage_f64(cons
           double sum = 0.0;
 #pragma unroll
           for (int m = 0; m < M; ++m)
-            sum += __ldg(in + (static_cast<std::int64_t>(v) * M + m) * ne + d) * b[m];
+            sum += in[(static_cast<std::int64_t>(v) * M + m) * ne + d] * b[m];
           B.outside[k][q][2 * half + v][te] = sum;
         }
       }
@@ -372,8 +373,8 @@ __global__ void __launch_bounds__(128, kStageBlocks<P>) euler_tri_stage_f64(cons
   // Mass inverse and the Shu-Osher combination.
   const double inv = geo[4 * ne + e];
   const double dt = a.dt ? *a.dt : a.dt_value;
-  const double *__restrict__ u0 = a.u0 + rows;
-  double *__restrict__ out = a.out + rows;
+  const double *u0 = a.u0 + rows;
+  double *out = a.out + rows;
   double rho[M];
 #pragma unroll
   for (int v = 0; v < 2; ++v)

@@ -1864,7 +1864,7 @@ __device__ __forceinline__ MeanState patch_mean(const double (*smean)[TILE],
 // The trace of element nb's high modes (FP64 in global memory) at point q of
 // its local edge j: the instructions of phase A, so both patches agree.
 template <int P>
-__device__ __forceinline__ void patch_outside_trace(const double *__restrict__ in, std::int64_t ne,
+__device__ __forceinline__ void patch_outside_trace(const double *in, std::int64_t ne,
                                                     std::int64_t nb, const float *phi, float *out) {
   constexpr int M = TriShape<P>::M, H = M - 1;
 #pragma unroll
@@ -1872,7 +1872,7 @@ __device__ __forceinline__ void patch_outside_trace(const double *__restrict__ i
     float s = 0.0f;
 #pragma unroll
     for (int m = 0; m < H; ++m)
-      s = fmaf(static_cast<float>(__ldg(in + (static_cast<std::int64_t>(v) * M + m + 1) * ne + nb)),
+      s = fmaf(static_cast<float>(in[(static_cast<std::int64_t>(v) * M + m + 1) * ne + nb]),
                phi[m], s);
     out[v] = s;
   }
@@ -2002,7 +2002,7 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_patch(const StageArgs a)
   }
   const bool active = t < count;
   const std::int64_t e = first + t;
-  const double *__restrict__ in = a.in;
+  const double *in = a.in;
   const double gamma = a.gamma;
   const PatchEdges pe = a.patch;
 
@@ -2044,7 +2044,8 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_patch(const StageArgs a)
   // only the mesh, the tables and (as a prefetch hint) u^n.  Wait here for
   // that launch to complete and its writes to be visible before the state,
   // dt or any output is touched.  Without the launch attribute the wait
-  // returns at once.
+  // returns at once.  (The state through ordinary loads: the read-only path
+  // wants data that nothing writes while the kernel is resident.)
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
 
   // A. State, traces, and the faces this element evaluates.
@@ -2125,8 +2126,8 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_patch(const StageArgs a)
           n0 = smean[0][local];
           n3 = smean[3][local];
         } else {
-          n0 = __ldg(in + nb) * phi0;
-          n3 = __ldg(in + static_cast<std::int64_t>(3) * M * ne + nb) * phi0;
+          n0 = in[nb] * phi0;
+          n3 = in[static_cast<std::int64_t>(3) * M * ne + nb] * phi0;
         }
         rough = rough || mean_jump(n0, smean[0][t], n3, smean[3][t]);
       }
@@ -2182,7 +2183,7 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_patch(const StageArgs a)
       } else if (!boundary) {
 #pragma unroll
         for (int v = 0; v < 4; ++v)
-          nmean[v] = __ldg(in + static_cast<std::int64_t>(v) * M * ne + nb) * phi0;
+          nmean[v] = in[static_cast<std::int64_t>(v) * M * ne + nb] * phi0;
       }
       // The face's left mean state: the reference of the perturbation form.
       MeanState ml;
@@ -2356,7 +2357,7 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_patch(const StageArgs a)
       double nmean[4];
 #pragma unroll
       for (int v = 0; v < 4; ++v)
-        nmean[v] = __ldg(in + static_cast<std::int64_t>(v) * M * ne + nb) * phi0;
+        nmean[v] = in[static_cast<std::int64_t>(v) * M * ne + nb] * phi0;
       ml = mean_state(gamma, nmean);
     }
     double fln[4];
