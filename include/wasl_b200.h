@@ -322,7 +322,9 @@ int wasl_nccl_comm_create(int ranks, const uint8_t *id, int rank, int device, vo
 void wasl_nccl_comm_destroy(void *comm);
 
 /* Device pointer of the state U[variable][mode][element] and the handle's
- * CUDA stream (cudaStream_t), for callers that keep data on the device. */
+ * CUDA stream (cudaStream_t), for callers that keep data on the device.  A
+ * state written through the pointer before a call is the state that call
+ * starts from (and takes its first CFL step from). */
 int wasl_gpu_state_device(wasl_gpu *handle, double **device_pointer);
 int wasl_gpu_stream(wasl_gpu *handle, void **stream);
 

@@ -265,7 +265,10 @@ public:
   std::int64_t faces() const override { return mesh_.face_count(); }
   int modes() const override { return M_; }
   int variables() const override { return 4; }
-  double *state_device() override { return d_u_.get(); }
+  double *state_device() override {
+    state_exposed_ = true;
+    return d_u_.get();
+  }
 
   void vertices(double *out) const override {
     for (std::int64_t e = 0; e < ne_; ++e) {
@@ -444,8 +447,11 @@ public:
   // (cfl_max, then dt_from_speed, which also zeroes the speed word).  With
   // the tile kernel and no limiter, the last stage of each step also reduces
   // the next step's CFL speed, so a step after the first needs only the
-  // small dt kernel and no pass over the state.
+  // small dt kernel and no pass over the state.  The speed is kept for the next
+  // call only while nobody else holds the state's address.
   void advance(double cfl, std::int64_t steps) override {
+    if (state_exposed_)
+      speed_ready_ = false;
     for (std::int64_t n = 0; n < steps; ++n) {
       if (!speed_ready_) {
         // The speed alone: the device dt needs no arg-max (that serves the
@@ -892,6 +898,7 @@ private:
   DeviceArray<double> d_patch_geo_;
   bool fused_speed_ = false; // this step's last stage reduces the next CFL speed
   bool speed_ready_ = false; // d_speed_ holds the current state's CFL speed
+  bool state_exposed_ = false; // state_device() was called: others may write the state
   DeviceArray<unsigned long long> d_speed_;
   int kernel_ = -1; // mixed form: -1 not chosen yet, 0 face-centric, 1 + s tile shape s
   TuneResult tuning_;
