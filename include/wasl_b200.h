@@ -240,7 +240,9 @@ int wasl_gpu_sync(wasl_gpu *handle);
  * -1 for forms with a single kernel or before the first step.  When the
  * choice was autotuned (mixed_kernel 0: every variant timed on the solver's
  * own state before its first step, the fastest kept for the process per
- * polynomial order, rule order and mesh size class), `ms` receives up to
+ * polynomial order, rule order and mesh size class; with the limiter, the
+ * fastest of shapes 8-11 at order 2 and of the others at orders 1 and 3,
+ * whose results agree bit for bit), `ms` receives up to
  * `capacity` per-variant stage times and `count` their number. */
 int wasl_gpu_tuning(const wasl_gpu *handle, int *choice, double *ms, int capacity, int *count);
 

@@ -788,22 +788,24 @@ private:
       tuning_.ms[kernels[i]] = timed.ms[i] / 3.0;
     kernel_ = kernels[timed.choice];
     if (base) {
-      // With the limiter the choice stays within one family at
-      //   P3  the tile kernels.  (The patch kernel is 14% faster a stage at
-      //       500,000 triangles, but next to strong shocks, where perturbations
-      //       are as large as the means, the families' FP32 sums differ by up to
-      //       1e-7 of the state after a few steps: P3 keeps its rounding.)
-      //   P2  the patch kernel: as fast below 65,536 elements, where a stage is
-      //       latency (30 us), 10-14% faster above.
-      //   P1  the patch kernel below 65,536 elements (equal there), the tile
-      //       kernels above: 8% slower at 180,000 elements (811 against 743 us
-      //       for four steps), but there, too, the families differ by 3e-8 next
-      //       to strong shocks.
+      // With the limiter the choice stays within one family per order.  A
+      // family's shapes agree bit for bit, so the result of a run does not
+      // depend on what was timed here; the two families' FP32 sums differ.
+      // Against the plain FP64 form both are as close (four steps of 60
+      // four-quadrant runs, 1,152 to 180,000 triangles: mean errors equal to 3%
+      // at every order).  us a stage, tile and patch kernels, by triangles:
+      //        1,152    7,200   28,800   64,800  180,000  405,000
+      //   P1   23, 24   25, 24   27, 27   30, 32   56, 56  131, 123
+      //   P2   33, 38   35, 40   38, 40   50, 47  122, 111  237, 233
+      //   P3   47, 50   48, 51   54, 56   86, 71  239, 189  439, 352
+      // P1: the tile kernels (no slower to 180,000; correctly rounded
+      // reciprocals).  P2: the patch kernel.  P3: the tile kernels, although
+      // slower on large meshes: a change of family would move results next to
+      // strong shocks by up to 1.2e-7 of the state.
       double best = 0.0;
       for (std::size_t i = 0; i < kernels.size(); ++i) {
         const bool patch = euler_tri_tile_is_patch(kernels[i] - 1);
-        const bool patches = p_ == 2 || (p_ == 1 && ne_ < 65536);
-        if (patch_ok_ && patch != patches)
+        if (patch_ok_ && patch != (p_ == 2))
           continue;
         if (best == 0.0 || timed.ms[i] < best) {
           best = timed.ms[i];
