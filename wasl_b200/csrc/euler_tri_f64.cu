@@ -11,7 +11,7 @@
 //   * face terms added in ascending global face index, points in order,
 //     rhs -= value * basis (left) / += (right) (triangle_residual.hpp:59-102)
 //   * rhs *= 1/det(J), then the Shu-Osher combination (time/ssp_rk3.hpp:44-60).
-// One thread owns one element, so no atomics touch the residual.
+// Two lanes own one element, two variables each, so no atomics touch the residual.
 #include <climits>
 #include <cstdio>
 #include <stdexcept>

@@ -644,16 +644,13 @@ __device__ __forceinline__ bool mean_jump(double rho_a, double rho_b, double e_a
 }
 
 // One point of a face in FP64 (faces across jumps): traces of both elements from
-// their FP64 coefficients (rows stride apart) and the FP64 face tables, HLLC
-// in FP64 (reference order of operations up to contraction), then the
-// high-mode perturbations dflux[q][v] = F_q - F(U_L bar).n (FP32) and the
-// full mode-0 value sum_q w_q F_q.  Both elements of a face call it with the
-// same inputs in the same roles, so they get the same bits.
+// their FP64 coefficients and the FP64 face tables, then HLLC in FP64 (reference
+// order of operations up to contraction).  Both elements of a face call it with
+// the same inputs in the same roles, so they get the same bits.
 template <int P>
 __device__ __forceinline__ void face_point_fp64(double gamma, const double *own,
-                                                std::int64_t own_stride, const double *other,
-                                                std::int64_t other_stride, bool boundary,
-                                                bool self_left, const double *own_basis,
+                                                const double *other, bool self_left,
+                                                const double *own_basis,
                                                 const double *other_basis, double nx, double ny,
                                                 double *f) {
   constexpr int M = TriShape<P>::M;
@@ -663,17 +660,16 @@ __device__ __forceinline__ void face_point_fp64(double gamma, const double *own,
     double so = 0.0, sn = 0.0;
 #pragma unroll
     for (int m = 0; m < M; ++m) {
-      so = fma(own[(v * M + m) * own_stride], own_basis[m], so);
-      if (!boundary)
-        sn = fma(other[(v * M + m) * other_stride], other_basis[m], sn);
+      so = fma(own[v * M + m], own_basis[m], so);
+      sn = fma(other[v * M + m], other_basis[m], sn);
     }
     to[v] = so;
     tn[v] = sn;
   }
 #pragma unroll
   for (int v = 0; v < 4; ++v) {
-    ul[v] = boundary || self_left ? to[v] : tn[v];
-    ur[v] = boundary ? to[v] : (self_left ? tn[v] : to[v]);
+    ul[v] = self_left ? to[v] : tn[v];
+    ur[v] = self_left ? tn[v] : to[v];
   }
   hllc_fast(gamma, ul, ur, nx, ny, f);
 }
@@ -728,24 +724,16 @@ __device__ __forceinline__ void tile_finish(const StageArgs &a, std::int64_t e, 
       best = __double_as_longlong(speed);
     else
       raise_error(a.error, kNonPhysicalAverage, e);
-    // Warp max over whichever lanes are still active (past the tile's end,
-    // or handed to the rough pass, lanes have returned): the 64-bit max of
+    // Warp max over whichever lanes are still active (past the tile's end, or
+    // handed to the rough pass, lanes have returned): the 64-bit max of
     // positive FP64 bits as the max of the high words, then of the low words
-    // among the lanes holding it; one atomic per warp and case.
+    // among the lanes holding it; one atomic per warp (a tile is of one case).
     const unsigned mask = __activemask();
-    const int lane = threadIdx.x & 31;
-    // (No lane's match set is the whole mask unless all lanes share the case,
-    // so the branch is uniform across the warp.)
-    if (__match_any_sync(mask, case_id) == mask) {
-      const unsigned hi = __reduce_max_sync(mask, static_cast<unsigned>(best >> 32));
-      const unsigned lo = __reduce_max_sync(
-          mask, static_cast<unsigned>(best >> 32) == hi ? static_cast<unsigned>(best) : 0u);
-      if (lane == __ffs(mask) - 1)
-        atomicMax(a.speed_max + case_id, (static_cast<unsigned long long>(hi) << 32) | lo);
-    } else {
-      // Lanes of one warp from different cases (the rough pass of a batch).
-      atomicMax(a.speed_max + case_id, best);
-    }
+    const unsigned hi = __reduce_max_sync(mask, static_cast<unsigned>(best >> 32));
+    const unsigned lo = __reduce_max_sync(
+        mask, static_cast<unsigned>(best >> 32) == hi ? static_cast<unsigned>(best) : 0u);
+    if ((threadIdx.x & 31) == __ffs(mask) - 1)
+      atomicMax(a.speed_max + case_id, (static_cast<unsigned long long>(hi) << 32) | lo);
   }
 
   if (a.suspects)
@@ -1925,16 +1913,11 @@ __device__ __forceinline__ void patch_finish(const StageArgs &a, std::int64_t e,
     else
       raise_error(a.error, kNonPhysicalAverage, e);
     const unsigned mask = __activemask();
-    const int lane = threadIdx.x & 31;
-    if (__match_any_sync(mask, case_id) == mask) {
-      const unsigned hi = __reduce_max_sync(mask, static_cast<unsigned>(best >> 32));
-      const unsigned lo = __reduce_max_sync(
-          mask, static_cast<unsigned>(best >> 32) == hi ? static_cast<unsigned>(best) : 0u);
-      if (lane == __ffs(mask) - 1)
-        atomicMax(a.speed_max + case_id, (static_cast<unsigned long long>(hi) << 32) | lo);
-    } else {
-      atomicMax(a.speed_max + case_id, best);
-    }
+    const unsigned hi = __reduce_max_sync(mask, static_cast<unsigned>(best >> 32));
+    const unsigned lo = __reduce_max_sync(
+        mask, static_cast<unsigned>(best >> 32) == hi ? static_cast<unsigned>(best) : 0u);
+    if ((threadIdx.x & 31) == __ffs(mask) - 1)
+      atomicMax(a.speed_max + case_id, (static_cast<unsigned long long>(hi) << 32) | lo);
   }
   if (LIMITED && a.suspects)
     append_listed(!positivity_clear(a.gamma, a.floors, avg, reach), e, a.suspects, a.suspect_count);
@@ -2619,8 +2602,8 @@ __global__ void __launch_bounds__(kRoughThreads) euler_tri_rough(const StageArgs
             other64 = periodic;
         }
         double f[4];
-        face_point_fp64<P>(gamma, E.own, 1, E.across[k], 1, false, self_left, own64 + q * M,
-                           other64 + q * M, nx, ny, f);
+        face_point_fp64<P>(gamma, E.own, E.across[k], self_left, own64 + q * M, other64 + q * M, nx,
+                           ny, f);
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
           E.flux[lane][v] = f[v];
@@ -2776,18 +2759,6 @@ __global__ void __launch_bounds__(kRoughThreads) euler_tri_rough(const StageArgs
     }
     __syncwarp();
     if (lane == 0 && valid) {
-      if (a.speed_max) {
-        const double scale = 1.0 / sqrt(2.0);
-        const double sa[4] = {__dmul_rn(scale, E.next[0]), __dmul_rn(scale, E.next[M]),
-                              __dmul_rn(scale, E.next[2 * M]), __dmul_rn(scale, E.next[3 * M])};
-        bool physical = true;
-        const double speed = cfl_speed(gamma, sa, 2, physical);
-        if (physical)
-          atomicMax(a.speed_max + case_id,
-                    static_cast<unsigned long long>(__double_as_longlong(speed)));
-        else
-          raise_error(a.error, kNonPhysicalAverage, e);
-      }
       if (a.suspects) {
         double mode0[4], reach[4];
 #pragma unroll

@@ -136,12 +136,13 @@ struct StageArgs {
   const TileWork *work = nullptr;
   std::int64_t work_count = 0;
   const double *case_dt = nullptr;
-  // Tile kernel, last stage: the largest cell-average wave speed |u| + c of
-  // `out` (the CFL kernels' formula) is max-reduced into speed_max[case] as
-  // FP64 bits, and a non-physical average sets the error word.
+  // Tile and patch kernels without a rough list, last stage: the largest
+  // cell-average wave speed |u| + c of `out` (the CFL kernels' formula) is
+  // max-reduced into speed_max[case] as FP64 bits, and a non-physical average
+  // sets the error word.
   unsigned long long *speed_max = nullptr;
   unsigned long long *error = nullptr;
-  // Tile kernel: elements with a face across which the cell means jump go to
+  // Tile and patch kernels: elements with a face across which the cell means jump go to
   // the rough list [ne] (count rough_count) and are computed by the second
   // pass with FP64 faces; null: one FP32 pass.  element_case [ne] gives the
   // case (for case_dt) of a rough element; null: case 0.

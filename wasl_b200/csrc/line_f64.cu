@@ -9,8 +9,10 @@
 // Compiled with --fmad=false.  One thread owns one element; the reference's
 // face loop runs in ascending face index and element e owns faces e (left)
 // and e+1 (right), so the thread adds the volume term, then its left face,
-// then its right face.  Each face's flux is computed by both of its elements
-// from the same traces in the same order, so both use the same double.  Then
+// then its right face.  An Euler face's flux is computed once, by the thread of
+// its right element, and passed to the left one (which computes it again only
+// between two blocks); an advection flux is one product, which both elements
+// form from the same trace.  Either way both use the same double.  Then
 // rhs *= 1/J and the Shu-Osher combination (time/ssp_rk3.hpp:44-60).
 #include <algorithm>
 #include <stdexcept>
@@ -506,21 +508,25 @@ template <int V, int P> __global__ void __launch_bounds__(512) line_run_f64(Line
   }
 }
 
-// The same run with one element per thread, for meshes of at most
-// LineRunLimit::threads - 1 elements: the stage's coefficients stay in registers
-// over the whole run (and u^n too, for scalar advection; in the thread's column
-// of shared memory for Euler), and only what a neighbour needs passes through
-// shared memory: the one trace an upwind flux reads, or Euler's right traces and
-// face fluxes.  Bound by the FP64 pipe of one SM and the barriers (one per
-// advection stage, two per Euler stage).  400 cells at P2: 0.67 -> 0.34 us per stage against the kernel above,
-// which keeps the three state buffers in shared memory, evaluates every trace
-// twice and reads each coefficient it needs.
-template <int V, int P> struct LineRunLimit {
-  static constexpr int threads = V == 1 ? (P <= 2 ? 1024 : 512) : (P <= 3 ? 512 : 0);
-};
+// The same run with one element per thread, for meshes of fewer than
+// kRunThreads elements: the stage's coefficients stay in registers over the whole
+// run (and u^n too, for scalar advection; in the thread's column of shared memory
+// for Euler), and only what a neighbour needs passes through shared memory: the
+// one trace an upwind flux reads, or Euler's right traces and face fluxes.
+// Against the kernel above, which keeps the three state buffers in shared memory,
+// evaluates every trace twice and reads each coefficient it needs, 300 Euler
+// cells at P2 take 7.7 instead of 12.8 ms a run.  Bound by the FP64 pipe of one
+// SM and the barriers (one per advection stage, two per Euler stage).
+//
+// Advection from kRunClusterFrom cells on runs on a cluster (launch_run), whose
+// blocks have up to kRunClusterThreads threads; Euler from P4 on does not fit
+// the registers.
+constexpr int kRunClusterFrom = 96;
+template <int V, int P> constexpr int kRunThreads = V == 1 ? kRunClusterFrom : P <= 3 ? 512 : 0;
+template <int P> constexpr int kRunClusterThreads = P <= 2 ? 1024 : 512;
 
 template <int V, int P>
-__global__ void __launch_bounds__(LineRunLimit<V, P>::threads) line_run_registers_f64(LineRunArgs r) {
+__global__ void __launch_bounds__(kRunThreads<V, P>) line_run_registers_f64(LineRunArgs r) {
   constexpr int M = P + 1;
   extern __shared__ double run_smem[];
   const int n = static_cast<int>(r.stage.ne), e = threadIdx.x, T = blockDim.x;
@@ -657,9 +663,9 @@ __global__ void __launch_bounds__(LineRunLimit<V, P>::threads) line_run_register
           c[0][m] = combine(k, un[m], c[0][m], dt, rhs[m] * inv);
         }
       } else {
-        double(*right)[LineRunLimit<V, P>::threads] = reinterpret_cast<
-            double(*)[LineRunLimit<V, P>::threads]>(run_smem + V * M * T);
-        double(*flux)[LineRunLimit<V, P>::threads] = right + 4;
+        double(*right)[kRunThreads<V, P>] = reinterpret_cast<
+            double(*)[kRunThreads<V, P>]>(run_smem + V * M * T);
+        double(*flux)[kRunThreads<V, P>] = right + 4;
         double own[4];
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
@@ -734,7 +740,7 @@ __global__ void __launch_bounds__(LineRunLimit<V, P>::threads) line_run_register
 constexpr int kRunHalo = 24;
 
 template <int P, int BLOCKS>
-__global__ void __launch_bounds__(LineRunLimit<1, P>::threads) line_run_cluster_f64(LineRunArgs r) {
+__global__ void __launch_bounds__(kRunClusterThreads<P>) line_run_cluster_f64(LineRunArgs r) {
   constexpr int M = P + 1;
   extern __shared__ double cluster_smem[]; // traces [2][T], then edges [2][M][kRunHalo]
   const int n = static_cast<int>(r.stage.ne), t = threadIdx.x, T = blockDim.x;
@@ -908,7 +914,7 @@ template <typename Kernel> void run_opt_in(Kernel kernel, std::size_t bytes, boo
 // blocks and 0.181 with eight; P1 at 2000: 1.45, 0.30 and 0.22.  Else one element
 // (and, for Euler, one face) per thread where the block has the threads and the
 // registers for it; else the elements of a thread in turn.
-constexpr int kRunClusterFrom = 96, kRunCluster4To = 416;
+constexpr int kRunCluster4To = 416;
 
 template <int P, int BLOCKS> void launch_run_cluster(const LineRunArgs &r, cudaStream_t s) {
   const auto threads =
@@ -930,17 +936,17 @@ template <int P, int BLOCKS> void launch_run_cluster(const LineRunArgs &r, cudaS
 }
 
 template <int V, int P> void launch_run(const LineRunArgs &r, cudaStream_t s) {
-  constexpr int limit = LineRunLimit<V, P>::threads;
   if constexpr (V == 1) {
     if (r.stage.ne >= kRunClusterFrom && r.stage.ne <= kRunCluster4To) {
       launch_run_cluster<P, 4>(r, s);
       return;
     }
-    if (r.stage.ne > kRunCluster4To && (r.stage.ne + 7) / 8 + kRunHalo <= limit) {
+    if (r.stage.ne > kRunCluster4To && (r.stage.ne + 7) / 8 + kRunHalo <= kRunClusterThreads<P>) {
       launch_run_cluster<P, 8>(r, s);
       return;
     }
   }
+  constexpr int limit = kRunThreads<V, P>;
   if constexpr (limit > 0) {
     if (r.stage.ne < limit) {
       static bool opted_in[64] = {};
@@ -953,11 +959,16 @@ template <int V, int P> void launch_run(const LineRunArgs &r, cudaStream_t s) {
       return;
     }
   }
-  const std::size_t bytes = line_run_bytes(V, P, r.stage.ne);
-  static bool opted_in[64] = {};
-  run_opt_in(line_run_f64<V, P>, kLineRunMaxBytes, opted_in);
-  const std::int64_t threads = std::min<std::int64_t>(512, (r.stage.ne + 31) / 32 * 32);
-  line_run_f64<V, P><<<1, static_cast<unsigned>(threads), bytes, s>>>(r);
+  // Advection from P1 on never comes here: a state of at most kLineRunMaxBytes
+  // has no more cells than the cluster of eight takes.
+  constexpr std::int64_t most_cells = kLineRunMaxBytes / (3 * sizeof(double) * V * (P + 1));
+  if constexpr (V == 4 || (most_cells + 7) / 8 + kRunHalo > kRunClusterThreads<P>) {
+    const std::size_t bytes = line_run_bytes(V, P, r.stage.ne);
+    static bool opted_in[64] = {};
+    run_opt_in(line_run_f64<V, P>, kLineRunMaxBytes, opted_in);
+    const std::int64_t threads = std::min<std::int64_t>(512, (r.stage.ne + 31) / 32 * 32);
+    line_run_f64<V, P><<<1, static_cast<unsigned>(threads), bytes, s>>>(r);
+  }
 }
 
 template <int V> void launch_run_order(int p, const LineRunArgs &r, cudaStream_t s) {
