@@ -660,8 +660,9 @@ def advection_line(args, local_rank, cpu=True):
                     "d2h_bytes_per_step": 8 * g.state_size / steps,
                     "path": "C-ABI set_state / run_resident / get_state, host wall clock"},
             "roofline": {"bound": "latency",
-                         "note": "the state (9.6 KB) lives in one SM's shared memory for the"
-                                 " whole run; the run is a chain of 3 x steps dependent stages"},
+                         "note": "the state (9.6 KB) lives in the registers of one cluster of"
+                                 " thread blocks for the whole run; the run is a chain of"
+                                 " 3 x steps dependent stages"},
             "gpu_launches": launches, "clocks": clocks}
     if cpu:
         cpu_s, cpu_steps, kind = advection_cpu(arrays, c0)

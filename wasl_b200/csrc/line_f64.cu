@@ -301,10 +301,13 @@ __device__ __forceinline__ double combine(int stage, double u0, double c, double
 // (with one thread per element evaluating both its faces: 150 us a stage).
 constexpr int kLineBlock = 128;
 
-// Resident blocks per SM the registers are sized for.  Measured, four steps:
-// P1 (700,001 cells) 486 us (7: 510, 9: 505, no bound: 595); P2 (1,000,003)
-// 843 us (6: 883, 8: 888, no bound: 977); P3 (700,001) 868 us (5: 885, 7:
-// 1002); from P4 on a bound spills (100,001 cells: 272 us without, 312 at 6).
+// Resident blocks per SM the registers are sized for; at P0 to P3 the bound spills
+// (36, 72, 88 and 188 bytes of stores) and pays all the same.  Measured, four
+// steps: P0 (1,000,003 cells) 438 us (7: 444, 9: 431, 10: 494, no bound: 482; at
+// 300,000 cells 174, 177, 179, 197, 186); P1 (700,001) 486 us (7: 510, 9: 505, no
+// bound: 595); P2 (1,000,003) 843 us (6: 883, 8: 888, no bound: 977); P3 (700,001)
+// 868 us (5: 885, 7: 1002); from P4 on it costs (100,001 cells: 272 us without,
+// 312 at 6).
 template <int P> constexpr int kLineBlocks = P <= 1 ? 8 : P == 2 ? 7 : P == 3 ? 6 : 1;
 
 template <int P>
