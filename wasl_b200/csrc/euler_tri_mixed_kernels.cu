@@ -644,12 +644,13 @@ __device__ __forceinline__ bool mean_jump(double rho_a, double rho_b, double e_a
 }
 
 // One point of a face in FP64 (faces across jumps): traces of both elements from
-// their FP64 coefficients and the FP64 face tables, then HLLC in FP64 (reference
-// order of operations up to contraction).  Both elements of a face call it with
-// the same inputs in the same roles, so they get the same bits.
+// their FP64 coefficients (rows stride apart) and the FP64 face tables, then HLLC
+// in FP64 (reference order of operations up to contraction).  Both elements of a
+// face call it with the same inputs in the same roles, so they get the same bits.
 template <int P>
 __device__ __forceinline__ void face_point_fp64(double gamma, const double *own,
-                                                const double *other, bool self_left,
+                                                std::int64_t own_stride, const double *other,
+                                                std::int64_t other_stride, bool self_left,
                                                 const double *own_basis,
                                                 const double *other_basis, double nx, double ny,
                                                 double *f) {
@@ -660,8 +661,8 @@ __device__ __forceinline__ void face_point_fp64(double gamma, const double *own,
     double so = 0.0, sn = 0.0;
 #pragma unroll
     for (int m = 0; m < M; ++m) {
-      so = fma(own[v * M + m], own_basis[m], so);
-      sn = fma(other[v * M + m], other_basis[m], sn);
+      so = fma(own[(v * M + m) * own_stride], own_basis[m], so);
+      sn = fma(other[(v * M + m) * other_stride], other_basis[m], sn);
     }
     to[v] = so;
     tn[v] = sn;
@@ -2402,6 +2403,15 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_patch(const StageArgs a)
 // face still get the same bits.  Bound by latency: 26 us at P3 for the few
 // thousand elements of 32 shocked cases, 78 us with one thread each.
 constexpr int kRoughLanes = 16, kRoughThreads = 128;
+// The longest list that takes lanes, on meshes (or batch groups) of more than six
+// times as many elements: smaller ones always take them, which spares them the
+// second launch (1-2 us a stage).  us a stage at 180,000 triangles by the list's
+// length, lanes and threads (euler_tri_rough_long): P1 9,000 elements 82, 82, 18,000
+// 97, 85; P2 9,000 134, 136, 18,000 158, 139; P3 18,000 291, 292, 36,000 363, 287.
+template <int P> constexpr int kRoughLong = 6000 * (P + 1);
+template <int P> __host__ __device__ constexpr bool rough_long_mesh(std::int64_t ne) {
+  return ne > 6 * kRoughLong<P>;
+}
 
 template <int P, int R> struct RoughElement {
   static constexpr int M = TriShape<P>::M, QF = TriShape<P>::QF, QV = MixedVolume<P, R>::QV;
@@ -2418,6 +2428,169 @@ template <int P, int R> struct RoughElement {
   int code[3], fp64[3];
 };
 
+// A face of an element of the second pass: its sides, the two elements' high-mode
+// basis rows (modes from 1) and FP64 basis rows at its points.
+template <int P, bool PATCH> struct RoughFace {
+  static constexpr int M = TriShape<P>::M, QF = TriShape<P>::QF;
+  using Table = std::conditional_t<PATCH, PatchEdge<P>, FaceTable<P, float>>;
+  bool self_left, boundary;
+  bool reversed;   // PATCH: the right element's own points run against the face's
+  int le, re, flip; // left and right local edge, relative direction
+  unsigned code;
+  std::int64_t slot;
+  const float *own, *other;
+
+  __device__ __forceinline__ RoughFace(const StageArgs &a, const Table &table, int k,
+                                       std::int64_t slot_, std::int32_t nb, unsigned code_)
+      : self_left(code_ & 1u), boundary(nb < 0), reversed(false), code(code_), slot(slot_) {
+    if constexpr (PATCH) {
+      const int jn = (code >> 1) & 3u;
+      reversed = code & 8u;
+      le = self_left ? k : jn;
+      re = self_left ? jn : k;
+      // The FP64 tables' flip is the edges' relative direction along the
+      // counter-clockwise parametrization; the code compares the edges' own point
+      // orders, and edge 2's points run against it.
+      flip = (reversed ? 1 : 0) ^ (le == 2 ? 1 : 0) ^ (re == 2 ? 1 : 0);
+      own = &table.phi[k][0][0];
+      other = &table.phi[jn][0][0];
+    } else {
+      le = (code >> 1) & 3u;
+      re = (code >> 3) & 3u;
+      flip = (code >> 5) & 1u;
+      const float *lb = &table.lb[le][0][0];
+      const float *rb = &table.rb[(le * 3 + re) * 2 + flip][0][0];
+      own = self_left ? lb : rb;
+      other = self_left ? rb : lb;
+      if (code & 0xC0u) {
+        const float *periodic =
+            a.boundary.basis32 + static_cast<std::int64_t>(a.tile.aux[slot]) * QF * M;
+        if (code & 0x40u)
+          own = periodic;
+        else
+          other = periodic;
+      }
+    }
+  }
+  // Basis rows at the face's point q (the left element's order).
+  __device__ __forceinline__ const float *own_high(int q) const {
+    if constexpr (PATCH)
+      return own + (!self_left && reversed ? QF - 1 - q : q) * (M - 1);
+    else
+      return own + q * M + 1;
+  }
+  __device__ __forceinline__ const float *other_high(int q) const {
+    if constexpr (PATCH)
+      return other + (self_left && reversed ? QF - 1 - q : q) * (M - 1);
+    else
+      return other + q * M + 1;
+  }
+  __device__ __forceinline__ void basis64(const StageArgs &a, const FaceTable<P, double> &T64,
+                                          const double *&own64, const double *&other64) const {
+    const double *lb = &T64.lb[le][0][0];
+    const double *rb = &T64.rb[(le * 3 + re) * 2 + flip][0][0];
+    own64 = self_left ? lb : rb;
+    other64 = self_left ? rb : lb;
+    if (!PATCH && (code & 0xC0u)) {
+      const double *periodic =
+          a.mesh.donor_basis + static_cast<std::int64_t>(a.tile.aux[slot]) * QF * M;
+      if (code & 0x40u)
+        own64 = periodic;
+      else
+        other64 = periodic;
+    }
+  }
+};
+
+// The flux perturbation at a face point whose means do not jump, from both sides'
+// high-mode traces.
+template <bool PATCH>
+__device__ __forceinline__ void rough_flux32(const Ref32 &ref, bool boundary, bool self_left,
+                                             const float (&to)[4], const float (&tn)[4],
+                                             const double (&mean)[4], const double (&nmean)[4],
+                                             float g1, float gamma32, float nx, float ny,
+                                             float (&fl)[4]) {
+  float dl[4], dr[4];
+  if (boundary) {
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+      dl[v] = dr[v] = to[v];
+  } else {
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const float jump = static_cast<float>(self_left ? nmean[v] - mean[v] : mean[v] - nmean[v]);
+      dl[v] = self_left ? to[v] : tn[v];
+      dr[v] = jump + (self_left ? tn[v] : to[v]);
+    }
+  }
+  hllc_perturbed<PATCH>(ref, dl, dr, g1, gamma32, nx, ny, fl);
+}
+
+// The volume term's weighted fluxes along xi (g[0..3]) and eta (g[4..7]) at a point
+// with perturbation d (as the tile kernel).
+template <bool PATCH>
+__device__ __forceinline__ void rough_volume(const Ref32 &bb, const float (&d)[4], float g1,
+                                             float wq, float fax, float fay, float fbx, float fby,
+                                             float *g) {
+  const float inv = perturbation_rcp<PATCH>(fmaxf(bb.rho + d[0], kVacuumFraction * bb.rho));
+  const float du = (d[1] - bb.u * d[0]) * inv;
+  const float dv = (d[2] - bb.v * d[0]) * inv;
+  const float uu = bb.u + du, vv = bb.v + dv;
+  const float dmu = bb.mx * du + d[1] * uu + bb.my * dv + d[2] * vv;
+  const float dp = g1 * (d[3] - 0.5f * dmu);
+  const float dep = d[3] + dp;
+  const float fx[4] = {d[1], bb.mx * du + d[1] * uu + dp, bb.my * du + d[2] * uu,
+                       bb.h * du + dep * uu};
+  const float fy[4] = {d[2], bb.mx * dv + d[1] * vv, bb.my * dv + d[2] * vv + dp,
+                       bb.h * dv + dep * vv};
+  const float wby = wq * fby, wbx = wq * fbx, wax = wq * fax, way = wq * fay;
+#pragma unroll
+  for (int v = 0; v < 4; ++v) {
+    g[v] = wby * fx[v] - wbx * fy[v];
+    g[4 + v] = wax * fy[v] - way * fx[v];
+  }
+}
+
+// The Shu-Osher combination of one coefficient (time/ssp_rk3.hpp:44-60), and mode 0's
+// residual with a face added.  Contracted by hand, so that both kernels of the
+// second pass round alike.
+template <int P>
+__device__ __forceinline__ double rough_combine(int stage, double u0, double cur, double dt,
+                                                double rr) {
+  const double next = fma(dt, rr, cur);
+  if (stage == 0)
+    return next;
+  const double old_share = stage == 1 ? 0.75 : 1.0 / 3.0, new_share = stage == 1 ? 0.25 : 2.0 / 3.0;
+  return P == 1 ? fma(old_share, u0, __dmul_rn(new_share, next))
+                : fma(new_share, next, __dmul_rn(old_share, u0));
+}
+__device__ __forceinline__ double rough_mode0(double r0, double sgn, double scale, double mode0) {
+  constexpr double phi0 = 0.70710678118654752440;
+  return fma(__dmul_rn(__dmul_rn(sgn, scale), phi0), mode0, r0);
+}
+
+// The lists an element of the second pass goes to: suspects (its means and reach)
+// and troubled elements (its density modes).
+template <int M>
+__device__ __forceinline__ void rough_lists(const StageArgs &a, std::int64_t e,
+                                            const double (&mode0)[4], const double (&reach)[4],
+                                            const double (&rho)[M]) {
+  if (a.suspects)
+    append_listed(!positivity_clear(a.gamma, a.floors, mode0, reach), e, a.suspects, a.suspect_count);
+  if (a.sense) {
+    double total = 0.0, high = 0.0;
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      total += rho[m] * rho[m];
+      if (m >= a.highest_degree_begin)
+        high += rho[m] * rho[m];
+    }
+    const bool troubled = !(total == 0.0 || high / total <= a.threshold);
+    a.flags[e] = troubled ? 1 : 0;
+    append_listed(troubled, e, a.troubled, a.troubled_count);
+  }
+}
+
 template <int P, int R, bool PATCH>
 __global__ void __launch_bounds__(kRoughThreads) euler_tri_rough(const StageArgs a) {
   using S = TriShape<P>;
@@ -2425,16 +2598,19 @@ __global__ void __launch_bounds__(kRoughThreads) euler_tri_rough(const StageArgs
   constexpr int GROUPS = kRoughThreads / kRoughLanes;
   constexpr double phi0 = 0.70710678118654752440;
   static_assert(3 * QF <= kRoughLanes, "one lane per face point");
-  using Table = std::conditional_t<PATCH, PatchEdge<P>, FaceTable<P, float>>;
-  __shared__ Table table;
+  __shared__ typename RoughFace<P, PATCH>::Table table;
   __shared__ MixedVolume<P, R> T;
   __shared__ FaceTable<P, double> T64;
   extern __shared__ __align__(16) unsigned char rough_smem[];
   RoughElement<P, R> &E =
       reinterpret_cast<RoughElement<P, R> *>(rough_smem)[threadIdx.x / kRoughLanes];
+  // (No early start for the launch after this one: its waiting blocks would hold
+  // registers that another stream's kernels can use.)
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
   const std::int64_t list = *a.rough_count;
-  if (static_cast<std::int64_t>(blockIdx.x) * GROUPS >= list)
-    return; // the whole block is past the list (uniform: no barrier reached)
+  if ((rough_long_mesh<P>(a.mesh.ne) && list > kRoughLong<P>) ||
+      static_cast<std::int64_t>(blockIdx.x) * GROUPS >= list)
+    return; // a long list, or past its end (uniform: no barrier reached)
   const int t = threadIdx.x, lane = t % kRoughLanes;
   {
     const float *src;
@@ -2456,7 +2632,7 @@ __global__ void __launch_bounds__(kRoughThreads) euler_tri_rough(const StageArgs
   }
   __syncthreads();
   const std::int64_t ne = a.mesh.ne;
-  const double *__restrict__ in = a.in;
+  const double *in = a.in;
   const double *__restrict__ geo = a.mesh.geo;
   const double gamma = a.gamma;
   const float gamma32 = static_cast<float>(gamma), g1 = static_cast<float>(gamma - 1.0);
@@ -2502,7 +2678,7 @@ __global__ void __launch_bounds__(kRoughThreads) euler_tri_rough(const StageArgs
       for (int c = 0; c < OWN; ++c) {
         const int i = c * kRoughLanes + lane;
         if (nb >= 0 && i < 4 * M)
-          E.across[k][i] = __ldg(in + i * ne + nb);
+          E.across[k][i] = in[i * ne + nb];
       }
     }
     __syncwarp();
@@ -2515,45 +2691,10 @@ __global__ void __launch_bounds__(kRoughThreads) euler_tri_rough(const StageArgs
     // One face point per lane.
     if (lane < 3 * QF) {
       const int k = lane / QF, q = lane % QF;
-      const std::int64_t slot = k * ne + e;
-      const unsigned code = E.code[k];
-      const bool self_left = code & 1u, boundary = E.nb[k] < 0;
+      const RoughFace<P, PATCH> face(a, table, k, k * ne + e, E.nb[k], E.code[k]);
+      const bool self_left = face.self_left, boundary = face.boundary;
       const double nx = E.face[3 * k], ny = E.face[3 * k + 1];
-      // The face's left and right local edges, and the two bases' high modes
-      // (from 1) at the face's point q.
-      int le, re, flip;
-      const float *own_high, *other_high;
-      if constexpr (PATCH) {
-        const int jn = (code >> 1) & 3u;
-        const bool rev = code & 8u;
-        le = self_left ? k : jn;
-        re = self_left ? jn : k;
-        // The FP64 tables' flip is the edges' relative direction along the
-        // counter-clockwise parametrization; rev compares the edges' own point
-        // orders, and edge 2's points run against it.
-        flip = (rev ? 1 : 0) ^ (le == 2 ? 1 : 0) ^ (re == 2 ? 1 : 0);
-        const int qr = rev ? QF - 1 - q : q; // the right element's point
-        own_high = table.phi[k][self_left ? q : qr];
-        other_high = table.phi[jn][self_left ? qr : q];
-      } else {
-        le = (code >> 1) & 3u;
-        re = (code >> 3) & 3u;
-        flip = (code >> 5) & 1u;
-        const float *lb = &table.lb[le][0][0];
-        const float *rb = &table.rb[(le * 3 + re) * 2 + flip][0][0];
-        const float *own_basis = self_left ? lb : rb;
-        const float *other_basis = self_left ? rb : lb;
-        if (code & 0xC0u) {
-          const float *periodic =
-              a.boundary.basis32 + static_cast<std::int64_t>(a.tile.aux[slot]) * QF * M;
-          if (code & 0x40u)
-            own_basis = periodic;
-          else
-            other_basis = periodic;
-        }
-        own_high = own_basis + q * M + 1;
-        other_high = other_basis + q * M + 1;
-      }
+      const float *own_high = face.own_high(q), *other_high = face.other_high(q);
       double nmean[4] = {0.0, 0.0, 0.0, 0.0};
       if (!boundary) {
 #pragma unroll
@@ -2589,21 +2730,11 @@ __global__ void __launch_bounds__(kRoughThreads) euler_tri_rough(const StageArgs
       for (int m = 0; m < H; ++m)
         E.basis[lane][m] = own_high[m];
       if (fp64) {
-        const double *lb64 = &T64.lb[le][0][0];
-        const double *rb64 = &T64.rb[(le * 3 + re) * 2 + flip][0][0];
-        const double *own64 = self_left ? lb64 : rb64;
-        const double *other64 = self_left ? rb64 : lb64;
-        if (!PATCH && (code & 0xC0u)) {
-          const double *periodic =
-              a.mesh.donor_basis + static_cast<std::int64_t>(a.tile.aux[slot]) * QF * M;
-          if (code & 0x40u)
-            own64 = periodic;
-          else
-            other64 = periodic;
-        }
+        const double *own64, *other64;
+        face.basis64(a, T64, own64, other64);
         double f[4];
-        face_point_fp64<P>(gamma, E.own, E.across[k], self_left, own64 + q * M, other64 + q * M, nx,
-                           ny, f);
+        face_point_fp64<P>(gamma, E.own, 1, E.across[k], 1, self_left, own64 + q * M,
+                           other64 + q * M, nx, ny, f);
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
           E.flux[lane][v] = f[v];
@@ -2611,7 +2742,7 @@ __global__ void __launch_bounds__(kRoughThreads) euler_tri_rough(const StageArgs
         }
       } else {
         const Ref32 ref = ref32(ml);
-        float to[4], tn[4], dl[4], dr[4], fl[4];
+        float to[4], tn[4] = {0.0f, 0.0f, 0.0f, 0.0f}, fl[4];
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
           float s = 0.0f;
@@ -2620,11 +2751,7 @@ __global__ void __launch_bounds__(kRoughThreads) euler_tri_rough(const StageArgs
             s = fmaf(static_cast<float>(E.own[v * M + m + 1]), own_high[m], s);
           to[v] = s;
         }
-        if (boundary) {
-#pragma unroll
-          for (int v = 0; v < 4; ++v)
-            dl[v] = dr[v] = to[v];
-        } else {
+        if (!boundary) {
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
             float s = 0.0f;
@@ -2633,15 +2760,9 @@ __global__ void __launch_bounds__(kRoughThreads) euler_tri_rough(const StageArgs
               s = fmaf(static_cast<float>(E.across[k][v * M + m + 1]), other_high[m], s);
             tn[v] = s;
           }
-#pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            const float jump =
-                static_cast<float>(self_left ? nmean[v] - mean[v] : mean[v] - nmean[v]);
-            dl[v] = self_left ? to[v] : tn[v];
-            dr[v] = jump + (self_left ? tn[v] : to[v]);
-          }
         }
-        hllc_perturbed<PATCH>(ref, dl, dr, g1, gamma32, static_cast<float>(nx), static_cast<float>(ny), fl);
+        rough_flux32<PATCH>(ref, boundary, self_left, to, tn, mean, nmean, g1, gamma32,
+                            static_cast<float>(nx), static_cast<float>(ny), fl);
 #pragma unroll
         for (int v = 0; v < 4; ++v)
           E.dflux[lane][v] = fl[v];
@@ -2663,24 +2784,7 @@ __global__ void __launch_bounds__(kRoughThreads) euler_tri_rough(const StageArgs
             s = fmaf(static_cast<float>(E.own[v * M + m + 1]), T.phi[q][m], s);
           d[v] = s;
         }
-        const float inv = perturbation_rcp<PATCH>(fmaxf(bb.rho + d[0], kVacuumFraction * bb.rho));
-        const float du = (d[1] - bb.u * d[0]) * inv;
-        const float dv = (d[2] - bb.v * d[0]) * inv;
-        const float uu = bb.u + du, vv = bb.v + dv;
-        const float dmu = bb.mx * du + d[1] * uu + bb.my * dv + d[2] * vv;
-        const float dp = g1 * (d[3] - 0.5f * dmu);
-        const float dep = d[3] + dp;
-        const float fx[4] = {d[1], bb.mx * du + d[1] * uu + dp, bb.my * du + d[2] * uu,
-                             bb.h * du + dep * uu};
-        const float fy[4] = {d[2], bb.mx * dv + d[1] * vv, bb.my * dv + d[2] * vv + dp,
-                             bb.h * dv + dep * vv};
-        const float wq = T.w[q];
-        const float wby = wq * fby, wbx = wq * fbx, wax = wq * fax, way = wq * fay;
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          E.volume[q][v] = wby * fx[v] - wbx * fy[v];
-          E.volume[q][4 + v] = wax * fy[v] - way * fx[v];
-        }
+        rough_volume<PATCH>(bb, d, g1, T.w[q], fax, fay, fbx, fby, E.volume[q]);
       }
     }
     __syncwarp();
@@ -2732,63 +2836,284 @@ __global__ void __launch_bounds__(kRoughThreads) euler_tri_rough(const StageArgs
 #pragma unroll
             for (int q = 0; q < QF; ++q)
               mode0 = fma(T64.ew[le][q], E.flux[k * QF + q][v], mode0);
-            r0 += sgn * scale * phi0 * mode0;
+            r0 = rough_mode0(r0, sgn, scale, mode0);
           } else {
             float acc = 0.0f;
 #pragma unroll
             for (int q = 0; q < QF; ++q)
               acc = fmaf(weights[q], E.dflux[k * QF + q][v], acc);
-            const double mode0 = E.fln[k][v] * c_edge_wsum<P>[le] + static_cast<double>(acc);
-            r0 += sgn * scale * phi0 * mode0;
+            const double mode0 = fma(E.fln[k][v], c_edge_wsum<P>[le], static_cast<double>(acc));
+            r0 = rough_mode0(r0, sgn, scale, mode0);
           }
         }
       }
       const std::int64_t idx = i * ne + e;
       const double cur = E.own[i];
       const double rr = (m == 0 ? r0 : static_cast<double>(racc)) * inv;
-      double o;
-      if (a.stage == 0)
-        o = cur + dt * rr;
-      else if (a.stage == 1)
-        o = 0.75 * u0[c] + 0.25 * (cur + dt * rr);
-      else
-        o = (1.0 / 3.0) * u0[c] + (2.0 / 3.0) * (cur + dt * rr);
+      const double o = rough_combine<P>(a.stage, u0[c], cur, dt, rr);
       if (valid)
         a.out[idx] = o;
       E.next[i] = o;
     }
     __syncwarp();
     if (lane == 0 && valid) {
-      if (a.suspects) {
-        double mode0[4], reach[4];
+      double rho[M], mode0[4], reach[4];
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          mode0[v] = E.next[v * M];
-          reach[v] = 0.0;
+      for (int m = 0; m < M; ++m)
+        rho[m] = E.next[m];
 #pragma unroll
-          for (int m = 1; m < M; ++m)
-            reach[v] += fabs(E.next[v * M + m]) * a.floors.bound[m];
-        }
-        if (!positivity_clear(gamma, a.floors, mode0, reach))
-          a.suspects[atomicAdd(a.suspect_count, 1)] = static_cast<std::int32_t>(e);
+      for (int v = 0; v < 4; ++v) {
+        mode0[v] = E.next[v * M];
+        reach[v] = 0.0;
+#pragma unroll
+        for (int m = 1; m < M; ++m)
+          reach[v] += fabs(E.next[v * M + m]) * a.floors.bound[m];
       }
-      if (a.sense) {
-        double total = 0.0, high = 0.0;
-#pragma unroll
-        for (int m = 0; m < M; ++m) {
-          total += E.next[m] * E.next[m];
-          if (m >= a.highest_degree_begin)
-            high += E.next[m] * E.next[m];
-        }
-        const bool troubled = !(total == 0.0 || high / total <= a.threshold);
-        a.flags[e] = troubled ? 1 : 0;
-        if (troubled)
-          a.troubled[atomicAdd(a.troubled_count, 1)] = static_cast<std::int32_t>(e);
-      }
+      rough_lists<M>(a, e, mode0, reach, rho);
     }
     __syncwarp(); // the next element's coefficients may land
   }
 }
+
+// The same pass over a long list (more than kRoughLong elements, of which the
+// kernel above does none), one thread per element: what the lanes spend on sharing
+// an element costs more than its chain once there are enough elements to fill the
+// SMs.  The same points, sums and order: the same bits, whatever the list's length.
+// us a stage at 180,000 triangles with all of them listed, lanes and threads: P1 324
+// and 132, P2 487 and 205, P3 843 and 491.  (Both paths in one kernel: the threads'
+// registers halve the lanes' occupancy, 246 -> 269 us at P3 with 3,600 listed.)
+constexpr int kLongThreads = 64, kLongBlocks = 4; // per SM, at 255 registers
+
+// (A call, not inlined: inlined here, at P3 the compiler contracts some of its sums
+// otherwise than in the kernels whose faces meet these.)
+template <bool PATCH>
+__device__ __noinline__ void called_flux32(const Ref32 &ref, bool boundary, bool self_left,
+                                           const float (&to)[4], const float (&tn)[4],
+                                           const double (&mean)[4], const double (&nmean)[4],
+                                           float g1, float gamma32, float nx, float ny,
+                                           float (&fl)[4]) {
+  rough_flux32<PATCH>(ref, boundary, self_left, to, tn, mean, nmean, g1, gamma32, nx, ny, fl);
+}
+
+template <int P, int R, bool PATCH>
+__global__ void __launch_bounds__(kLongThreads) euler_tri_rough_long(const StageArgs a) {
+  using S = TriShape<P>;
+  constexpr int M = S::M, QV = MixedVolume<P, R>::QV, QF = S::QF, H = M - 1;
+  constexpr double phi0 = 0.70710678118654752440;
+  __shared__ typename RoughFace<P, PATCH>::Table table;
+  __shared__ double coefficient[4 * M][kLongThreads];
+  __shared__ float flux[4 * QF][kLongThreads];
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  const std::int64_t list = *a.rough_count;
+  if (list <= kRoughLong<P> || static_cast<std::int64_t>(blockIdx.x) * 32 >= list)
+    return; // (uniform)
+  const int t = threadIdx.x;
+  {
+    const float *src;
+    if constexpr (PATCH)
+      src = reinterpret_cast<const float *>(&g_patch<P>);
+    else
+      src = static_cast<const float *>(a.face_table);
+    float *dst = reinterpret_cast<float *>(&table);
+    for (int i = t; i < static_cast<int>(sizeof(table) / sizeof(float)); i += kLongThreads)
+      dst[i] = src[i];
+  }
+  __syncthreads();
+  const MixedVolume<P, R> &T = c_mix<P, R>;
+  const FaceTable<P, double> &T64 = *static_cast<const FaceTable<P, double> *>(a.face_table64);
+  const std::int64_t ne = a.mesh.ne;
+  const double *in = a.in;
+  const double *__restrict__ geo = a.mesh.geo;
+  const double gamma = a.gamma;
+  const float gamma32 = static_cast<float>(gamma), g1 = static_cast<float>(gamma - 1.0);
+  const std::int32_t *nbrs = PATCH ? a.patch.nbr : a.tile.nbr;
+  const std::uint8_t *codes = PATCH ? a.patch.info : a.tile.code;
+  const double *face_geo = PATCH ? a.patch.geo : a.mesh.slot_geo;
+  // (A warp takes 32 of the list; the first round is one warp of every block.)
+  const std::int64_t warp = static_cast<std::int64_t>(t / 32) * gridDim.x + blockIdx.x;
+  for (std::int64_t at = warp * 32 + t % 32; at < list;
+       at += static_cast<std::int64_t>(gridDim.x) * kLongThreads) {
+    const std::int64_t e = a.rough[at];
+    float ch[4][H], racc[4][H];
+    double mean[4];
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        const double x = in[(static_cast<std::int64_t>(v) * M + m) * ne + e];
+        coefficient[v * M + m][t] = x;
+        if (m == 0) {
+          mean[v] = x * phi0;
+        } else {
+          ch[v][m - 1] = static_cast<float>(x);
+          racc[v][m - 1] = 0.0f;
+        }
+      }
+    const MeanState own = mean_state(gamma, mean);
+    {
+      const Ref32 bb = ref32(own);
+      const float fax = static_cast<float>(geo[e]), fay = static_cast<float>(geo[ne + e]);
+      const float fbx = static_cast<float>(geo[2 * ne + e]), fby = static_cast<float>(geo[3 * ne + e]);
+#pragma unroll 1
+      for (int q = 0; q < QV; ++q) {
+        float d[4], g[8];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          float s = 0.0f;
+#pragma unroll
+          for (int m = 0; m < H; ++m)
+            s = fmaf(ch[v][m], T.phi[q][m], s);
+          d[v] = s;
+        }
+        rough_volume<PATCH>(bb, d, g1, T.w[q], fax, fay, fbx, fby, g);
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+#pragma unroll
+          for (int m = 0; m < H; ++m)
+            racc[v][m] = fmaf(T.dxi[q][m], g[v], fmaf(T.deta[q][m], g[4 + v], racc[v][m]));
+      }
+    }
+    double r0[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 1
+    for (int k = 0; k < 3; ++k) {
+      const std::int64_t slot = k * ne + e;
+      const std::int32_t raw = nbrs[slot];
+      const std::int32_t nb =
+          raw >= 0 ? static_cast<std::int32_t>(checked_index(raw, ne, a.error)) : raw;
+      const RoughFace<P, PATCH> face(a, table, k, slot, nb, codes[slot]);
+      const double nx = face_geo[(3 * k) * ne + e], ny = face_geo[(3 * k + 1) * ne + e];
+      const double scale = face_geo[(3 * k + 2) * ne + e];
+      double nmean[4] = {0.0, 0.0, 0.0, 0.0};
+      if (!face.boundary) {
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+          nmean[v] = in[static_cast<std::int64_t>(v) * M * ne + nb] * phi0;
+      }
+      MeanState ml;
+      if (face.self_left || face.boundary)
+        ml = own;
+      else
+        ml = mean_state(gamma, nmean);
+      double fln[4];
+      mean_normal_flux(ml, nx, ny, fln);
+      float shift[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      if (!face.boundary && !face.self_left) {
+        double frn[4];
+        mean_normal_flux(own, nx, ny, frn);
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+          shift[v] = static_cast<float>(fln[v] - frn[v]);
+      }
+      const double sgn = face.self_left ? -1.0 : 1.0;
+      const float fscale = static_cast<float>(scale);
+      const float *weights;
+      if constexpr (PATCH)
+        weights = table.w[face.le];
+      else
+        weights = table.ew[face.le];
+      if (!face.boundary && mean_jump(nmean[0], mean[0], nmean[3], mean[3])) {
+        const double *b_own, *b_other;
+        face.basis64(a, T64, b_own, b_other);
+        double mode0[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 1
+        for (int q = 0; q < QF; ++q) {
+          double f[4];
+          face_point_fp64<P>(gamma, &coefficient[0][t], kLongThreads, in + nb, ne, face.self_left,
+                             b_own + q * M, b_other + q * M, nx, ny, f);
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            flux[4 * q + v][t] = static_cast<float>(f[v] - fln[v]);
+            mode0[v] = fma(T64.ew[face.le][q], f[v], mode0[v]);
+          }
+        }
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+          r0[v] = rough_mode0(r0[v], sgn, scale, mode0[v]);
+      } else {
+        float nh[4][H];
+        if (!face.boundary) {
+#pragma unroll
+          for (int v = 0; v < 4; ++v)
+#pragma unroll
+            for (int m = 0; m < H; ++m)
+              nh[v][m] =
+                  static_cast<float>(in[(static_cast<std::int64_t>(v) * M + m + 1) * ne + nb]);
+        }
+        const Ref32 ref = ref32(ml);
+        const float nxf = static_cast<float>(nx), nyf = static_cast<float>(ny);
+        float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 1
+        for (int q = 0; q < QF; ++q) {
+          const float *own_high = face.own_high(q), *other_high = face.other_high(q);
+          float to[4], tn[4] = {0.0f, 0.0f, 0.0f, 0.0f}, fl[4];
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            float so = 0.0f, sn = 0.0f;
+#pragma unroll
+            for (int m = 0; m < H; ++m)
+              so = fmaf(ch[v][m], own_high[m], so);
+            to[v] = so;
+            if (!face.boundary) {
+#pragma unroll
+              for (int m = 0; m < H; ++m)
+                sn = fmaf(nh[v][m], other_high[m], sn);
+              tn[v] = sn;
+            }
+          }
+          called_flux32<PATCH>(ref, face.boundary, face.self_left, to, tn, mean, nmean, g1, gamma32,
+                               nxf, nyf, fl);
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            flux[4 * q + v][t] = fl[v];
+            acc[v] = fmaf(weights[q], fl[v], acc[v]);
+          }
+        }
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+          r0[v] = rough_mode0(r0[v], sgn, scale,
+                              fma(fln[v], c_edge_wsum<P>[face.le], static_cast<double>(acc[v])));
+      }
+      // The lift, in the order of this element's own points.
+#pragma unroll 1
+      for (int i = 0; i < QF; ++i) {
+        const int q = PATCH && !face.self_left && face.reversed ? QF - 1 - i : i;
+        const float wsc = (face.self_left ? -weights[q] : weights[q]) * fscale;
+        const float *basis = face.own_high(q);
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          const float fl = flux[4 * q + v][t];
+          const float value = wsc * (face.self_left ? fl : fl + shift[v]);
+#pragma unroll
+          for (int m = 0; m < H; ++m)
+            racc[v][m] = fmaf(value, basis[m], racc[v][m]);
+        }
+      }
+    }
+    const double inv = geo[4 * ne + e];
+    const double dt = a.case_dt ? a.case_dt[a.element_case ? a.element_case[e] : 0]
+                                : (a.dt ? *a.dt : a.dt_value);
+    double rho[M], mode0[4], reach[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        const std::int64_t idx = (static_cast<std::int64_t>(v) * M + m) * ne + e;
+        const double rr = (m == 0 ? r0[v] : static_cast<double>(racc[v][m > 0 ? m - 1 : 0])) * inv;
+        const double o = rough_combine<P>(a.stage, a.stage > 0 ? a.u0[idx] : 0.0,
+                                       coefficient[v * M + m][t], dt, rr);
+        a.out[idx] = o;
+        if (v == 0)
+          rho[m] = o;
+        if (m == 0)
+          mode0[v] = o;
+        else
+          reach[v] += fabs(o) * a.floors.bound[m];
+      }
+    rough_lists<M>(a, e, mode0, reach, rho);
+  }
+}
+
 
 void check(cudaError_t rc, const char *what) {
   if (rc != cudaSuccess)
@@ -2865,12 +3190,12 @@ void smem_opt_in(Kernel kernel, std::size_t dynamic, std::size_t fixed, bool (&o
     opted_in[device] = true;
 }
 
-// A stage kernel launched as a programmatic dependent of the launch before
+// A kernel of a stage launched as a programmatic dependent of the launch before
 // it on the stream: its CTAs may start while that launch drains, and wait
 // (griddepcontrol.wait) before reading what it wrote.
 template <typename Kernel>
 void launch_dependent(Kernel kernel, unsigned blocks, unsigned threads, std::size_t smem,
-                      cudaStream_t s, const StageArgs &a) {
+                      cudaStream_t s, const StageArgs &a, bool dependent = true) {
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(blocks);
   config.blockDim = dim3(threads);
@@ -2880,8 +3205,8 @@ void launch_dependent(Kernel kernel, unsigned blocks, unsigned threads, std::siz
   attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attribute[0].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attribute;
-  config.numAttrs = 1;
-  check(cudaLaunchKernelEx(&config, kernel, a), "patch kernel launch");
+  config.numAttrs = dependent ? 1 : 0;
+  check(cudaLaunchKernelEx(&config, kernel, a), "stage kernel launch");
 }
 
 template <int P, int R, int TILE, int MINB> void tile_opt_in() {
@@ -2909,13 +3234,20 @@ template <int P, int R, bool PATCH> void rough_opt_in() {
 
 // The second pass over the rough list, whose length only the device knows: up
 // to eight blocks (64 elements) per SM, which return at once beyond it and go
-// round where it is longer.
+// round where it is longer; and, on meshes large enough for a long list, the
+// kernel for that, each returning at once where it is the other's.  Both are
+// programmatic dependents (2 us a stage less than plain launches), but not in a
+// batch, whose step is a graph (a pass of 32 cases was 2-6% slower with programmatic
+// edges in it).
 template <int P, int R, bool PATCH> void launch_rough(const StageArgs &a, cudaStream_t s) {
   rough_opt_in<P, R, PATCH>();
   constexpr int groups = kRoughThreads / kRoughLanes;
   const std::int64_t blocks = std::min<std::int64_t>((a.mesh.ne + groups - 1) / groups, 148 * 8);
-  euler_tri_rough<P, R, PATCH>
-      <<<static_cast<unsigned>(blocks), kRoughThreads, rough_smem_bytes<P, R>(), s>>>(a);
+  launch_dependent(euler_tri_rough<P, R, PATCH>, static_cast<unsigned>(blocks), kRoughThreads,
+                   rough_smem_bytes<P, R>(), s, a, !a.case_dt);
+  if (rough_long_mesh<P>(a.mesh.ne))
+    launch_dependent(euler_tri_rough_long<P, R, PATCH>, 148 * kLongBlocks, kLongThreads, 0, s, a,
+                     !a.case_dt);
 }
 
 // The FP32 pass over all tiles, then (with a rough list) the pass over the
