@@ -793,10 +793,14 @@ __global__ void __launch_bounds__(128) limit_f64(const LimitArgs a) {
 
 // The limiter's finish: the limited modes back into the state, and the
 // positivity limiter on the suspects (elements the stage kernel could not
-// prove to keep the floors) that were not limited, one warp each.  Testing in
-// the stage kernel, where the new modes are at hand, saves the pass over the
-// state that positivity_rest makes: 44 us of a 515 us stage at 500,000
-// triangles, P3.
+// prove to keep the floors) that were not limited, one warp each, or, where
+// there are many, one thread each (the same bits).  Testing in the stage kernel,
+// where the new modes are at hand, saves the pass over the state that
+// positivity_rest makes: 44 us of a 515 us stage at 500,000 triangles, P3.  us a
+// stage by the list's length, warps and threads: P2 at 28,800 triangles 5,800
+// suspects 53, 56, 11,500 63, 56, at 180,000 all of them 258, 141; P3 60, 63, 71, 64
+// and 580, 291.
+constexpr int kLongSuspects = 8192;
 template <int M> __global__ void __launch_bounds__(128) finish_limited(const LimitArgs a) {
   constexpr int W = 4 * M;
   __shared__ double modes[4][W];
@@ -809,6 +813,25 @@ template <int M> __global__ void __launch_bounds__(128) finish_limited(const Lim
   if (!a.suspects)
     return;
   const int lane = threadIdx.x & 31, count = *a.suspect_count;
+  if (count > kLongSuspects) {
+    // One thread each (32 of the list per warp; the first round is one warp of
+    // every block).
+    for (std::int64_t k = ((threadIdx.x >> 5) * static_cast<std::int64_t>(gridDim.x) + blockIdx.x) * 32 + lane;
+         k < count; k += static_cast<std::int64_t>(gridDim.x) * 128) {
+      const std::int64_t e = a.suspects[k];
+      if (a.flags[e])
+        continue;
+      double lim[W];
+#pragma unroll
+      for (int i = 0; i < W; ++i)
+        lim[i] = a.state[i * ne + e];
+      positivity_limit<M>(a, lim, e);
+#pragma unroll
+      for (int i = 0; i < W; ++i)
+        a.state[i * ne + e] = lim[i];
+    }
+    return;
+  }
   double *lim = modes[threadIdx.x >> 5];
   for (int k = static_cast<int>(thread >> 5); k < count; k += static_cast<int>(gridDim.x) * 4) {
     const std::int64_t e = a.suspects[k];
