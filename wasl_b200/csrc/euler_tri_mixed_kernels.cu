@@ -679,7 +679,9 @@ __device__ __forceinline__ void face_point_fp64(double gamma, const double *own,
 // residual scaling by 1/det J, the Shu-Osher combination in FP64
 // (cpp/include/wasl/time/ssp_rk3.hpp:44-60), and, when asked for, the next
 // step's CFL speed and the modal-decay sensor on the result.
-template <int P, int TILE>
+// LISTED: with a list of positivity suspects (the sums it needs cost an unlisted
+// stage 3-4% at P2).
+template <int P, int TILE, bool LISTED>
 __device__ __forceinline__ void tile_finish(const StageArgs &a, std::int64_t e, int t, int case_id,
                                             const double (*sstate)[TILE], const double (&r0)[4],
                                             const float (&racc)[4][TriShape<P>::M - 1]) {
@@ -709,7 +711,7 @@ __device__ __forceinline__ void tile_finish(const StageArgs &a, std::int64_t e, 
         rho[m] = o;
       if (m == 0)
         avg[v] = o;
-      else if (a.suspects)
+      else if (LISTED)
         reach[v] += fabs(o) * a.floors.bound[m];
     }
 
@@ -737,7 +739,7 @@ __device__ __forceinline__ void tile_finish(const StageArgs &a, std::int64_t e, 
       atomicMax(a.speed_max + case_id, (static_cast<unsigned long long>(hi) << 32) | lo);
   }
 
-  if (a.suspects)
+  if (LISTED)
     append_listed(!positivity_clear(a.gamma, a.floors, avg, reach), e, a.suspects, a.suspect_count);
   if (a.sense) {
     double total = 0.0, high = 0.0;
@@ -791,7 +793,7 @@ template <int P, int MINB> constexpr bool kTileRolled = P > 1 && MINB > 1;
 // with a face across a jump of the means returns early (handed to the rough
 // pass).  Shared by the one-tile-per-CTA and the persistent kernels.  ROLLED: one
 // face point at a time (kTileRolled).
-template <int P, int R, int TILE, bool ROLLED>
+template <int P, int R, int TILE, bool ROLLED, bool LISTED>
 __device__ __forceinline__ void tile_element(const StageArgs &a, const FaceTable<P, float> &table,
                                              const double (*sstate)[TILE], int t,
                                              std::int64_t e, std::int64_t first,
@@ -983,10 +985,10 @@ __device__ __forceinline__ void tile_element(const StageArgs &a, const FaceTable
     }
   }
 
-  tile_finish<P, TILE>(a, e, t, case_id, sstate, r0, racc);
+  tile_finish<P, TILE, LISTED>(a, e, t, case_id, sstate, r0, racc);
 }
 
-template <int P, int R, int TILE, int MINB>
+template <int P, int R, int TILE, int MINB, bool LISTED>
 __global__ void __launch_bounds__(TILE, MINB) euler_tri_tile_mixed(const StageArgs a) {
   using S = TriShape<P>;
   constexpr int M = S::M;
@@ -1033,7 +1035,8 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_tile_mixed(const StageAr
   __syncthreads();
   if (!active)
     return;
-  tile_element<P, R, TILE, kTileRolled<P, MINB>>(a, table, sstate, t, e, first, count, case_id);
+  tile_element<P, R, TILE, kTileRolled<P, MINB>, LISTED>(a, table, sstate, t, e, first, count,
+                                                         case_id);
 }
 
 // The FP32 pass of the tile kernel as a persistent kernel: each CTA loads the
@@ -1041,7 +1044,7 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_tile_mixed(const StageAr
 // TILE-element tiles) gridDim.x apart, staging each one's state in turn; the
 // per-element arithmetic is the tile kernel's, so the results are the same
 // bit for bit.
-template <int P, int R, int TILE, int MINB>
+template <int P, int R, int TILE, int MINB, bool LISTED>
 __global__ void __launch_bounds__(TILE, MINB) euler_tri_tile_persistent(const StageArgs a) {
   using S = TriShape<P>;
   constexpr int M = S::M;
@@ -1084,7 +1087,8 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_tile_persistent(const St
     asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncthreads(); // the tile is staged (and, the first time, the tables)
     if (active)
-      tile_element<P, R, TILE, kTileRolled<P, MINB>>(a, table, sstate, t, e, first, count, case_id);
+      tile_element<P, R, TILE, kTileRolled<P, MINB>, LISTED>(a, table, sstate, t, e, first, count,
+                                                         case_id);
     __syncthreads(); // every element is done with the tile before the next one lands
   }
 }
@@ -1133,7 +1137,7 @@ template <int P, int TILE> struct SharedFaceSmem {
 // codes, then neighbours' slots; normals; geometry) do not each wait on DRAM
 // when the state and mesh are not in L2 (1.5% faster per step in the
 // vortex benchmark, which flushes L2 between steps).
-template <int P, int R, int TILE, int MINB>
+template <int P, int R, int TILE, int MINB, bool LISTED>
 __global__ void __launch_bounds__(TILE, MINB) euler_tri_tile_shared(const StageArgs a) {
   using S = TriShape<P>;
   using L = SharedFaceSmem<P, TILE>;
@@ -1551,7 +1555,7 @@ __global__ void __launch_bounds__(TILE, MINB) euler_tri_tile_shared(const StageA
     }
   }
 
-  tile_finish<P, TILE>(a, e, t, case_id, sstate, r0, racc);
+  tile_finish<P, TILE, LISTED>(a, e, t, case_id, sstate, r0, racc);
 }
 
 // ---- patch kernel ------------------------------------------------------------
@@ -3209,15 +3213,15 @@ void launch_dependent(Kernel kernel, unsigned blocks, unsigned threads, std::siz
   check(cudaLaunchKernelEx(&config, kernel, a), "stage kernel launch");
 }
 
-template <int P, int R, int TILE, int MINB> void tile_opt_in() {
+template <int P, int R, int TILE, int MINB, bool LISTED> void tile_opt_in() {
   static bool opted_in[64] = {};
-  smem_opt_in(euler_tri_tile_mixed<P, R, TILE, MINB>, tile_smem<P, TILE>(),
+  smem_opt_in(euler_tri_tile_mixed<P, R, TILE, MINB, LISTED>, tile_smem<P, TILE>(),
               sizeof(FaceTable<P, float>), opted_in);
 }
 
-template <int P, int R, int TILE, int MINB> void shared_opt_in() {
+template <int P, int R, int TILE, int MINB, bool LISTED> void shared_opt_in() {
   static bool opted_in[64] = {};
-  smem_opt_in(euler_tri_tile_shared<P, R, TILE, MINB>, SharedFaceSmem<P, TILE>::bytes,
+  smem_opt_in(euler_tri_tile_shared<P, R, TILE, MINB, LISTED>, SharedFaceSmem<P, TILE>::bytes,
               sizeof(FaceTable<P, float>) + sizeof(int), opted_in);
 }
 
@@ -3253,32 +3257,40 @@ template <int P, int R, bool PATCH> void launch_rough(const StageArgs &a, cudaSt
 // The FP32 pass over all tiles, then (with a rough list) the pass over the
 // elements it left.  SHARED picks the shared-face tile kernel for the
 // FP32 pass.
-template <int P, int R, int TILE, int MINB, bool SHARED = false>
-void stage_tile(const StageArgs &a, cudaStream_t s) {
+template <int P, int R, int TILE, int MINB, bool SHARED, bool LISTED>
+void launch_tile(const StageArgs &a, cudaStream_t s) {
   if constexpr (SHARED)
-    shared_opt_in<P, R, TILE, MINB>();
+    shared_opt_in<P, R, TILE, MINB, LISTED>();
   else
-    tile_opt_in<P, R, TILE, MINB>();
+    tile_opt_in<P, R, TILE, MINB, LISTED>();
   const std::int64_t blocks = a.work ? a.work_count : (a.mesh.ne + TILE - 1) / TILE;
   if (blocks <= 0)
     return;
   if constexpr (SHARED)
-    euler_tri_tile_shared<P, R, TILE, MINB>
+    euler_tri_tile_shared<P, R, TILE, MINB, LISTED>
         <<<static_cast<unsigned>(blocks), TILE, SharedFaceSmem<P, TILE>::bytes, s>>>(a);
   else
-    euler_tri_tile_mixed<P, R, TILE, MINB>
+    euler_tri_tile_mixed<P, R, TILE, MINB, LISTED>
         <<<static_cast<unsigned>(blocks), TILE, tile_smem<P, TILE>(), s>>>(a);
   if (a.rough)
     launch_rough<P, R, false>(a, s);
 }
 
+template <int P, int R, int TILE, int MINB, bool SHARED = false>
+void stage_tile(const StageArgs &a, cudaStream_t s) {
+  if (a.suspects)
+    launch_tile<P, R, TILE, MINB, SHARED, true>(a, s);
+  else
+    launch_tile<P, R, TILE, MINB, SHARED, false>(a, s);
+}
+
 // The persistent tile kernel's attributes and its grid: every CTA resident
 // at once (CTAs per SM at this shape's registers and shared memory, times the
 // SMs), found once per device.
-template <int P, int R, int TILE, int MINB> int persistent_prepare() {
+template <int P, int R, int TILE, int MINB, bool LISTED> int persistent_prepare() {
   static bool opted_in[64] = {};
   static int resident[64] = {};
-  smem_opt_in(euler_tri_tile_persistent<P, R, TILE, MINB>, tile_smem<P, TILE>(),
+  smem_opt_in(euler_tri_tile_persistent<P, R, TILE, MINB, LISTED>, tile_smem<P, TILE>(),
               sizeof(FaceTable<P, float>), opted_in);
   int device = 0;
   check(cudaGetDevice(&device), "cudaGetDevice");
@@ -3286,7 +3298,7 @@ template <int P, int R, int TILE, int MINB> int persistent_prepare() {
     return resident[device];
   int per_sm = 0, sms = 0;
   check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, euler_tri_tile_persistent<P, R, TILE, MINB>, TILE, tile_smem<P, TILE>()),
+            &per_sm, euler_tri_tile_persistent<P, R, TILE, MINB, LISTED>, TILE, tile_smem<P, TILE>()),
         "persistent tile occupancy");
   check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "SM count");
   const int blocks = (per_sm > 0 ? per_sm : 1) * (sms > 0 ? sms : 1);
@@ -3297,17 +3309,25 @@ template <int P, int R, int TILE, int MINB> int persistent_prepare() {
 
 // The FP32 pass as the persistent tile kernel (one wave of resident CTAs
 // looping over the tiles), then the rough pass as stage_tile runs it.
-template <int P, int R, int TILE, int MINB>
-void stage_tile_persistent(const StageArgs &a, cudaStream_t s) {
-  const int resident = persistent_prepare<P, R, TILE, MINB>();
+template <int P, int R, int TILE, int MINB, bool LISTED>
+void launch_tile_persistent(const StageArgs &a, cudaStream_t s) {
+  const int resident = persistent_prepare<P, R, TILE, MINB, LISTED>();
   const std::int64_t tiles = a.work ? a.work_count : (a.mesh.ne + TILE - 1) / TILE;
   if (tiles <= 0)
     return;
   const std::int64_t blocks = tiles < resident ? tiles : resident;
-  euler_tri_tile_persistent<P, R, TILE, MINB>
+  euler_tri_tile_persistent<P, R, TILE, MINB, LISTED>
       <<<static_cast<unsigned>(blocks), TILE, tile_smem<P, TILE>(), s>>>(a);
   if (a.rough)
     launch_rough<P, R, false>(a, s);
+}
+
+template <int P, int R, int TILE, int MINB>
+void stage_tile_persistent(const StageArgs &a, cudaStream_t s) {
+  if (a.suspects)
+    launch_tile_persistent<P, R, TILE, MINB, true>(a, s);
+  else
+    launch_tile_persistent<P, R, TILE, MINB, false>(a, s);
 }
 
 template <int P, int R, int TILE, int MINB, bool MMA> void patch_opt_in() {
@@ -3368,22 +3388,32 @@ template <int P, int R> struct StageTile {
 
 template <int P, int R> struct PrepareTile {
   static void run() {
-    tile_opt_in<P, R, 128, 4>();
-    tile_opt_in<P, R, 128, 1>();
-    tile_opt_in<P, R, 256, 2>();
-    tile_opt_in<P, R, 64, 8>();
-    shared_opt_in<P, R, 64, 7>();
-    shared_opt_in<P, R, 96, 5>();
-    shared_opt_in<P, R, 128, 4>();
-    shared_opt_in<P, R, 128, 3>();
+    tile_opt_in<P, R, 128, 4, false>();
+    tile_opt_in<P, R, 128, 4, true>();
+    tile_opt_in<P, R, 128, 1, false>();
+    tile_opt_in<P, R, 128, 1, true>();
+    tile_opt_in<P, R, 256, 2, false>();
+    tile_opt_in<P, R, 256, 2, true>();
+    tile_opt_in<P, R, 64, 8, false>();
+    tile_opt_in<P, R, 64, 8, true>();
+    shared_opt_in<P, R, 64, 7, false>();
+    shared_opt_in<P, R, 64, 7, true>();
+    shared_opt_in<P, R, 96, 5, false>();
+    shared_opt_in<P, R, 96, 5, true>();
+    shared_opt_in<P, R, 128, 4, false>();
+    shared_opt_in<P, R, 128, 4, true>();
+    shared_opt_in<P, R, 128, 3, false>();
+    shared_opt_in<P, R, 128, 3, true>();
     patch_opt_in<P, R, 128, 5, false>();
     patch_opt_in<P, R, 64, 8, false>();
     patch_opt_in<P, R, 256, 2, false>();
     patch_opt_in<P, R, 192, 3, false>();
     patch_opt_in<P, R, 128, 4, true>();
     patch_opt_in<P, R, 128, 5, true>();
-    persistent_prepare<P, R, 128, 4>();
-    persistent_prepare<P, R, 256, 2>();
+    persistent_prepare<P, R, 128, 4, false>();
+    persistent_prepare<P, R, 128, 4, true>();
+    persistent_prepare<P, R, 256, 2, false>();
+    persistent_prepare<P, R, 256, 2, true>();
     rough_opt_in<P, R, false>();
   }
 };
