@@ -114,13 +114,17 @@ template <int P> struct StageBlock {
   int count;
 };
 
-// Resident blocks per SM the registers are sized for: 5 (96 registers) at P0
-// to P2, 4 (128) at P3, where the two coefficient arrays alone take 80.
-// Measured per stage: P2 94 us (4: 99, 3: 110, 6: 102), P3 92 us (3: 93, 5: 100).
-template <int P> constexpr int kStageBlocks = P < 3 ? 5 : 4;
-
-template <int P>
-__global__ void __launch_bounds__(128, kStageBlocks<P>) euler_tri_stage_f64(const StageArgs a) {
+// Resident blocks per SM the registers are sized for (BLOCKS): 5 (96 registers) at
+// P0 to P2, 4 (128) at P3, where the two coefficient arrays alone take 80.
+// Measured per stage at 131,072 elements: P2 94 us (4: 99, 3: 110, 6: 102), P3 92
+// us (3: 93, 5: 100).  At P2 a grid that 3 or 4 blocks per SM hold at once gets the
+// registers of so few (167 or 128): more of a block's loads are in flight, which
+// counts most where the elements' numbering leaves few faces inside the blocks.  us
+// a stage with 5 and 3 blocks at 20,000 elements 35, 26, numbered at random 54, 32
+// (one thread per element: 41, 45); with 5 and 4 at 33,800 38, 32, at random 60, 41
+// (42, 48); at 39,200, more than one wave of 4, 38, 40.
+template <int P, int BLOCKS>
+__global__ void __launch_bounds__(128, BLOCKS) euler_tri_stage_f64(const StageArgs a) {
   using S = TriShape<P>;
   constexpr int M = S::M, QV = S::QV, QF = S::QF, E = StageBlock<P>::E;
   extern __shared__ __align__(16) unsigned char stage_smem[];
@@ -1059,7 +1063,7 @@ template <int P> void upload_volume(const void *symbol) {
   check(cudaMemcpyToSymbol(symbol, &table, sizeof(table)), "upload volume table");
 }
 
-template <int P> void stage(const StageArgs &a, cudaStream_t s) {
+template <int P, int BLOCKS> void launch_stage(const StageArgs &a, unsigned blocks, cudaStream_t s) {
   constexpr int bytes = sizeof(StageBlock<P>);
   // Above 48 KiB (P3) the attribute opts in, once per device.
   if constexpr (bytes > 48 * 1024) {
@@ -1067,16 +1071,26 @@ template <int P> void stage(const StageArgs &a, cudaStream_t s) {
     int device = 0;
     check(cudaGetDevice(&device), "cudaGetDevice");
     if (device >= 64 || !opted_in[device]) {
-      check(cudaFuncSetAttribute(euler_tri_stage_f64<P>,
+      check(cudaFuncSetAttribute(euler_tri_stage_f64<P, BLOCKS>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, bytes),
             "stage kernel shared memory");
       if (device < 64)
         opted_in[device] = true;
     }
   }
+  launch_kernel(true, euler_tri_stage_f64<P, BLOCKS>, blocks, 128, bytes, s, a);
+}
+
+template <int P> void stage(const StageArgs &a, cudaStream_t s) {
   constexpr int E = StageBlock<P>::E;
   const unsigned blocks = static_cast<unsigned>((a.mesh.ne + E - 1) / E);
-  launch_kernel(true, euler_tri_stage_f64<P>, blocks, 128, bytes, s, a);
+  if constexpr (P == 2) {
+    if (blocks <= 148 * 3)
+      return launch_stage<P, 3>(a, blocks, s);
+    if (blocks <= 148 * 4)
+      return launch_stage<P, 4>(a, blocks, s);
+  }
+  launch_stage<P, P < 3 ? 5 : 4>(a, blocks, s);
 }
 
 } // namespace
