@@ -41,6 +41,7 @@ MlpTrainer::~MlpTrainer() {
 void MlpTrainer::set_data(const float *features, const std::uint8_t *labels, std::int64_t n) {
   if (n <= 0)
     throw SolverError(WASL_ERR_ARGUMENT, "indicator training: no samples");
+  n_ = 0; // no data, should an allocation fail
   data_.resize(static_cast<std::size_t>(n) * shape_.features);
   labels_.resize(n);
   cuda_check(cudaMemcpyAsync(data_.get(), features, sizeof(float) * n * shape_.features,
@@ -55,10 +56,12 @@ void MlpTrainer::set_data(const float *features, const std::uint8_t *labels, std
 
 MlpWorkspace MlpTrainer::workspace(std::int64_t samples) {
   const std::size_t rows = static_cast<std::size_t>(mlp_train_rows(samples));
-  if (losses_.size() < rows) {
+  const std::size_t floats = rows * static_cast<std::size_t>(shape_.count);
+  // (Either may be gone where growing it failed before.)
+  if (rows_.size() < floats || losses_.size() < rows) {
     // (The stream may still use the old scratch.)
     cuda_check(cudaStreamSynchronize(stream_), "indicator workspace");
-    rows_.resize(rows * static_cast<std::size_t>(shape_.count));
+    rows_.resize(floats);
     losses_.resize(rows);
   }
   return {packed_.get(), rows_.get(), losses_.get()};

@@ -63,9 +63,10 @@ public:
     if (p_)
       cudaFree(p_);
     p_ = nullptr;
-    n_ = n;
+    n_ = 0; // (also when the allocation fails: size() is what there is)
     if (n)
       cuda_check(cudaMalloc(reinterpret_cast<void **>(&p_), n * sizeof(T)), "cudaMalloc");
+    n_ = n;
   }
   void upload(const std::vector<T> &h, cudaStream_t s = nullptr) {
     resize(h.size());
