@@ -67,3 +67,22 @@ def test_conserves_in_supersonic_flow(p, kernel):
             g.step(g.stable_dt(0.05))
         m1, e1 = g.mass_energy()
     assert abs(m1 - m0) <= 1e-13 * abs(m0) and abs(e1 - e0) <= 1e-13 * abs(e0)
+
+
+@pytest.mark.parametrize("p,nx,ny", [(1, 371, 100), (2, 451, 121), (3, 481, 151)])
+def test_long_lists_in_a_batch(p, nx, ny):
+    """Two cases of one order, which share a list: the single-case solver's bits."""
+    arrays = [meshgen.jittered_box(nx, jitter=0.1, seed=s, ny=ny) for s in (1, 2)]
+    states = [jumping_state(2 * nx * ny, p, p + s) for s in (1, 2)]
+    kw = dict(limiting=True, sensor_threshold=1e30, boundary="transmissive")
+    with wasl_b200.Batch([(*a, p) for a in arrays], tile_shape=1, **kw) as b:
+        for c, state in enumerate(states):
+            b.set_state(c, state)
+        b.advance(0.2, 1)
+        got = [b.get_state(c) for c in range(2)]
+    for c, a in enumerate(arrays):
+        with wasl_b200.Solver(*a, polynomial_order=p, precision="mixed", mixed_kernel=2,
+                              volume_rule_order=p, **kw) as g:
+            g.set_state(states[c])
+            g.advance(0.2, 1)
+            assert np.array_equal(got[c], g.get_state())
